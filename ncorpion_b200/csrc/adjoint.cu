@@ -14,44 +14,52 @@
 //                           + G J_k (m_k Lambda - M lambda_k)
 //   (da/dX)^T ...          = sum_k G J_k (M lambda_k - m_k Lambda)
 //   (da/dm)^T ...     |_k  = -sum_j G (lambda_j . r) / D^3 + G Lambda . s_k / |s_k|^3
-// Pair sums are FP64 with one rsqrt per pair, tiled through shared memory with
-// (target block, source chunk) work units reduced in a fixed order.  In the
+// The force and its VJP are pairsym.cuh's sums over unordered pairs (FP64, one
+// rsqrt per pair); the JVP is summed body by body, tiled through shared memory
+// with (target block, source chunk) work units reduced in a fixed order.  In the
 // MIXED gravity mode the bodies are taken in the Morton order of their initial
 // positions (a permutation done on the host at the call's boundary), every
 // evaluation computes the 128-body tiles' boxes, and only the tile pairs whose
 // boxes are near (near_theta x the larger diagonal, and each tile with itself)
-// are summed in FP64; the others in FP32 on coordinates relative to the source
-// tile's centre, the FP32 sums of every 64 sources folded into FP64 -- the
-// force kernel's scheme applied to the force, its VJP and its JVP.
+// are summed in FP64; the others in FP32 on coordinates relative to a tile's
+// centre, short FP32 sums folded into FP64 -- the force kernel's scheme applied
+// to the force, its VJP and its JVP.
+//
+// A kick and drift is three launches (tile data, pair sums, final pass with the
+// kick, the drift and the central body's), a step of the reverse sweep three
+// more.  N = 16,384, mixed: a force's pair sums take 128 us and a VJP's 269 (208
+// and 396 when each body's were made by themselves, bound by the FP32 pipe and the
+// near tiles' FP64), a forward call and a forward + adjoint call of 32 steps
+// 28.7 ms (42.9 with those and with six to nine launches a step).  N = 5,003, FP64:
+// 32 us and 62 (50 and 86), 24 steps 6.35 ms (9.46).
 #include <algorithm>
 #include <vector>
 #include "common.cuh"
+#include "pairsym.cuh"
 
 namespace ncg {
 
 namespace {
 
-constexpr int AT = 128;  // bodies per tile / threads per block
+constexpr int AT = PT;  // bodies per tile / threads per block of the JVP's pair sums
 
 struct Src {
       const double *x, *y, *z, *m, *sR, *lx, *ly, *lz;  // lx.. : adjoints (VJP) or position tangents (JVP)
       const double *dm;                                 // mass tangents (JVP)
 };
 
-// Mutual forces (OP 0: 3 outputs), their VJP (OP 1: 4 outputs) or their JVP
-// (OP 2: 3 outputs, d a_k = sum_j G [dm_j r + m_j T_kj (dx_j - dx_k)] / ...)
-// of target block blockIdx.y against source chunk blockIdx.x.
-template <int OP, bool SOFT>
-__global__ void __launch_bounds__(AT) k_pairs(Src s, int n, int tpc, double *__restrict__ part, long stride)
+// The JVP's pair sums, d a_k = sum_j G [dm_j r + m_j T_kj (dx_j - dx_k)] / ...,
+// of target block blockIdx.y against source chunk blockIdx.x, in FP64.
+template <bool SOFT>
+__global__ void __launch_bounds__(AT) k_pairs_jvp(Src s, int n, int tpc, double *__restrict__ part, long stride)
 {
       __shared__ double sx[AT], sy[AT], sz[AT], sm[AT], sr[AT], slx[AT], sly[AT], slz[AT], sdm[AT];
       const int k = blockIdx.y * AT + threadIdx.x;
       const bool act = k < n;
       const int kk = act ? k : 0;
-      const double xk = s.x[kk], yk = s.y[kk], zk = s.z[kk], mk = s.m[kk], rk = SOFT ? s.sR[kk] : 0.;
-      double lxk = 0., lyk = 0., lzk = 0.;
-      if (OP >= 1) { lxk = s.lx[kk]; lyk = s.ly[kk]; lzk = s.lz[kk]; }
-      double o0 = 0., o1 = 0., o2 = 0., o3 = 0.;
+      const double xk = s.x[kk], yk = s.y[kk], zk = s.z[kk], rk = SOFT ? s.sR[kk] : 0.;
+      const double lxk = s.lx[kk], lyk = s.ly[kk], lzk = s.lz[kk];
+      double o0 = 0., o1 = 0., o2 = 0.;
       const int ntiles = (n + AT - 1) / AT;
       const int t0 = blockIdx.x * tpc, t1 = min(ntiles, t0 + tpc);
       for (int t = t0; t < t1; ++t) {
@@ -61,8 +69,8 @@ __global__ void __launch_bounds__(AT) k_pairs(Src s, int n, int tpc, double *__r
                   sx[threadIdx.x] = s.x[j]; sy[threadIdx.x] = s.y[j]; sz[threadIdx.x] = s.z[j];
                   sm[threadIdx.x] = s.m[j];
                   if (SOFT) sr[threadIdx.x] = s.sR[j];
-                  if (OP >= 1) { slx[threadIdx.x] = s.lx[j]; sly[threadIdx.x] = s.ly[j]; slz[threadIdx.x] = s.lz[j]; }
-                  if (OP == 2) sdm[threadIdx.x] = s.dm[j];
+                  slx[threadIdx.x] = s.lx[j]; sly[threadIdx.x] = s.ly[j]; slz[threadIdx.x] = s.lz[j];
+                  sdm[threadIdx.x] = s.dm[j];
             }
             __syncthreads();
             const int cnt = min(AT, n - t * AT);
@@ -74,32 +82,18 @@ __global__ void __launch_bounds__(AT) k_pairs(Src s, int n, int tpc, double *__r
                   d2 = fma(rx, rx, fma(ry, ry, fma(rz, rz, d2)));
                   const double ri = rsqrt(d2);
                   const double i3 = ri * ri * ri;
-                  if (OP == 0) {
-                        const double w = sm[q] * i3;
-                        o0 = fma(w, rx, o0); o1 = fma(w, ry, o1); o2 = fma(w, rz, o2);
-                  } else if (OP == 2) {
-                        const double i5 = i3 * ri * ri;
-                        const double dx = slx[q] - lxk, dy = sly[q] - lyk, dz = slz[q] - lzk;
-                        const double rd = rx * dx + ry * dy + rz * dz;
-                        const double mj = sm[q], c = 3.0 * rd * i5 * mj, g = sdm[q] * i3;
-                        o0 += g * rx + mj * i3 * dx - rx * c;
-                        o1 += g * ry + mj * i3 * dy - ry * c;
-                        o2 += g * rz + mj * i3 * dz - rz * c;
-                  } else {
-                        const double i5 = i3 * ri * ri;
-                        const double mj = sm[q];
-                        const double wx = mk * slx[q] - mj * lxk, wy = mk * sly[q] - mj * lyk, wz = mk * slz[q] - mj * lzk;
-                        const double rw = rx * wx + ry * wy + rz * wz;
-                        const double c = 3.0 * rw * i5;
-                        o0 += wx * i3 - rx * c; o1 += wy * i3 - ry * c; o2 += wz * i3 - rz * c;
-                        o3 -= (slx[q] * rx + sly[q] * ry + slz[q] * rz) * i3;
-                  }
+                  const double i5 = i3 * ri * ri;
+                  const double dx = slx[q] - lxk, dy = sly[q] - lyk, dz = slz[q] - lzk;
+                  const double rd = rx * dx + ry * dy + rz * dz;
+                  const double mj = sm[q], c = 3.0 * rd * i5 * mj, g = sdm[q] * i3;
+                  o0 += g * rx + mj * i3 * dx - rx * c;
+                  o1 += g * ry + mj * i3 * dy - ry * c;
+                  o2 += g * rz + mj * i3 * dz - rz * c;
             }
       }
       if (act) {
-            double *p = part + (size_t)blockIdx.x * (OP == 1 ? 4 : 3) * stride;
+            double *p = part + (size_t)blockIdx.x * 3 * stride;
             p[k] = o0; p[stride + k] = o1; p[2 * stride + k] = o2;
-            if (OP == 1) p[3 * stride + k] = o3;
       }
 }
 
@@ -127,27 +121,22 @@ __global__ void k_adj_tilebox(const double *__restrict__ pos, int n, int ntiles,
       }
 }
 
-// k_pairs in the MIXED mode: FP64 for near tile pairs (the same pair terms),
-// FP32 relative to the source tile's centre for the others, with packed f32x2
-// arithmetic (two sources per instruction) for the force and its VJP.  (Two
-// targets a thread measured slower: 1.56 against 1.15 ms per forward+adjoint
-// step at N = 16,384, from 128 registers a thread and the serial FP64 near
-// tiles.)
-template <int OP, bool SOFT>
-__global__ void __launch_bounds__(AT) k_pairs_mx(Src s, int n, int tpc, const double *__restrict__ box, double theta,
-                                                 double *__restrict__ part, long stride)
+// k_pairs_jvp in the MIXED mode: FP64 for near tile pairs (the same pair terms),
+// FP32 relative to the source tile's centre for the others.
+template <bool SOFT>
+__global__ void __launch_bounds__(AT) k_pairs_jvp_mx(Src s, int n, int tpc, const double *__restrict__ box,
+                                                     double theta, double *__restrict__ part, long stride)
 {
       __shared__ double sx[AT], sy[AT], sz[AT], sm[AT], sr[AT], slx[AT], sly[AT], slz[AT], sdm[AT];
-      __shared__ __align__(16) float fx[AT], fy[AT], fz[AT], fm[AT], fr[AT], flx[AT], fly[AT], flz[AT], fdm[AT];
+      __shared__ float fx[AT], fy[AT], fz[AT], fm[AT], fr[AT], flx[AT], fly[AT], flz[AT], fdm[AT];
       const int ib = blockIdx.y;
       const int k = ib * AT + threadIdx.x;
       const bool act = k < n;
       const int kk = act ? k : 0;
-      const double xk = s.x[kk], yk = s.y[kk], zk = s.z[kk], mk = s.m[kk], rk = SOFT ? s.sR[kk] : 0.;
-      double lxk = 0., lyk = 0., lzk = 0.;
-      if (OP >= 1) { lxk = s.lx[kk]; lyk = s.ly[kk]; lzk = s.lz[kk]; }
-      const float mkf = (float)mk, rkf = (float)rk, lxkf = (float)lxk, lykf = (float)lyk, lzkf = (float)lzk;
-      double o0 = 0., o1 = 0., o2 = 0., o3 = 0.;
+      const double xk = s.x[kk], yk = s.y[kk], zk = s.z[kk], rk = SOFT ? s.sR[kk] : 0.;
+      const double lxk = s.lx[kk], lyk = s.ly[kk], lzk = s.lz[kk];
+      const float rkf = (float)rk, lxkf = (float)lxk, lykf = (float)lyk, lzkf = (float)lzk;
+      double o0 = 0., o1 = 0., o2 = 0.;
       const int ntiles = (n + AT - 1) / AT;
       const int t0 = blockIdx.x * tpc, t1 = min(ntiles, t0 + tpc);
       const double *bi = box + 6 * ib;
@@ -156,29 +145,22 @@ __global__ void __launch_bounds__(AT) k_pairs_mx(Src s, int n, int tpc, const do
             const double *bj = box + 6 * t;
             const bool near = t == ib || tiles_near(bi, bj, theta);
             __syncthreads();
-            if (j >= n && !near) {  // padding of the far path: far away, massless, no adjoint
-                  fx[threadIdx.x] = fy[threadIdx.x] = fz[threadIdx.x] = 1e18f;
-                  fm[threadIdx.x] = fr[threadIdx.x] = flx[threadIdx.x] = fly[threadIdx.x] = flz[threadIdx.x] = 0.f;
-                  fdm[threadIdx.x] = 0.f;
-            }
             if (j < n) {
                   if (near) {
                         sx[threadIdx.x] = s.x[j]; sy[threadIdx.x] = s.y[j]; sz[threadIdx.x] = s.z[j];
                         sm[threadIdx.x] = s.m[j];
                         if (SOFT) sr[threadIdx.x] = s.sR[j];
-                        if (OP >= 1) { slx[threadIdx.x] = s.lx[j]; sly[threadIdx.x] = s.ly[j]; slz[threadIdx.x] = s.lz[j]; }
-                        if (OP == 2) sdm[threadIdx.x] = s.dm[j];
+                        slx[threadIdx.x] = s.lx[j]; sly[threadIdx.x] = s.ly[j]; slz[threadIdx.x] = s.lz[j];
+                        sdm[threadIdx.x] = s.dm[j];
                   } else {
                         fx[threadIdx.x] = (float)(s.x[j] - bj[0]);
                         fy[threadIdx.x] = (float)(s.y[j] - bj[1]);
                         fz[threadIdx.x] = (float)(s.z[j] - bj[2]);
                         fm[threadIdx.x] = (float)s.m[j];
                         if (SOFT) fr[threadIdx.x] = (float)s.sR[j];
-                        if (OP >= 1) {
-                              flx[threadIdx.x] = (float)s.lx[j]; fly[threadIdx.x] = (float)s.ly[j];
-                              flz[threadIdx.x] = (float)s.lz[j];
-                        }
-                        if (OP == 2) fdm[threadIdx.x] = (float)s.dm[j];
+                        flx[threadIdx.x] = (float)s.lx[j]; fly[threadIdx.x] = (float)s.ly[j];
+                        flz[threadIdx.x] = (float)s.lz[j];
+                        fdm[threadIdx.x] = (float)s.dm[j];
                   }
             }
             __syncthreads();
@@ -192,114 +174,15 @@ __global__ void __launch_bounds__(AT) k_pairs_mx(Src s, int n, int tpc, const do
                         d2 = fma(rx, rx, fma(ry, ry, fma(rz, rz, d2)));
                         const double ri = rsqrt(d2);
                         const double i3 = ri * ri * ri;
-                        if (OP == 0) {
-                              const double w = sm[q] * i3;
-                              o0 = fma(w, rx, o0); o1 = fma(w, ry, o1); o2 = fma(w, rz, o2);
-                        } else if (OP == 2) {
-                              const double i5 = i3 * ri * ri;
-                              const double dx = slx[q] - lxk, dy = sly[q] - lyk, dz = slz[q] - lzk;
-                              const double rd = rx * dx + ry * dy + rz * dz;
-                              const double mj = sm[q], c = 3.0 * rd * i5 * mj, g = sdm[q] * i3;
-                              o0 += g * rx + mj * i3 * dx - rx * c;
-                              o1 += g * ry + mj * i3 * dy - ry * c;
-                              o2 += g * rz + mj * i3 * dz - rz * c;
-                        } else {
-                              const double i5 = i3 * ri * ri;
-                              const double mj = sm[q];
-                              const double wx = mk * slx[q] - mj * lxk, wy = mk * sly[q] - mj * lyk, wz = mk * slz[q] - mj * lzk;
-                              const double rw = rx * wx + ry * wy + rz * wz;
-                              const double c = 3.0 * rw * i5;
-                              o0 += wx * i3 - rx * c; o1 += wy * i3 - ry * c; o2 += wz * i3 - rz * c;
-                              o3 -= (slx[q] * rx + sly[q] * ry + slz[q] * rz) * i3;
-                        }
+                        const double i5 = i3 * ri * ri;
+                        const double dx = slx[q] - lxk, dy = sly[q] - lyk, dz = slz[q] - lzk;
+                        const double rd = rx * dx + ry * dy + rz * dz;
+                        const double mj = sm[q], c = 3.0 * rd * i5 * mj, g = sdm[q] * i3;
+                        o0 += g * rx + mj * i3 * dx - rx * c;
+                        o1 += g * ry + mj * i3 * dy - ry * c;
+                        o2 += g * rz + mj * i3 * dz - rz * c;
                   }
-            } else if (OP == 0) {
-                  // packed f32x2: two sources per instruction; FP32 runs of 64 sources
-                  const float xr = (float)(xk - bj[0]), yr = (float)(yk - bj[1]), zr = (float)(zk - bj[2]);
-                  const f2 XT = f2_pack(xr, xr), YT = f2_pack(yr, yr), ZT = f2_pack(zr, zr), RT = f2_pack(rkf, rkf);
-                  const int ce = (cnt + 1) & ~1;
-                  for (int q0 = 0; q0 < ce; q0 += 64) {
-                        f2 P0 = 0ull, P1 = 0ull, P2 = 0ull;
-                        const int qe = min(ce, q0 + 64);
-#pragma unroll 4
-                        for (int q = q0; q < qe; q += 2) {
-                              const f2 dx = f2_sub(*(const f2 *)&fx[q], XT), dy = f2_sub(*(const f2 *)&fy[q], YT);
-                              const f2 dz = f2_sub(*(const f2 *)&fz[q], ZT);
-                              f2 d2;
-                              if (SOFT) {
-                                    const f2 e = f2_add(*(const f2 *)&fr[q], RT);
-                                    d2 = f2_fma(dx, dx, f2_mul(e, e));
-                              } else {
-                                    d2 = f2_mul(dx, dx);
-                              }
-                              d2 = f2_fma(dy, dy, d2);
-                              d2 = f2_fma(dz, dz, d2);
-                              const f2 i = f2_rsqrt(d2);
-                              const f2 w = f2_mul(f2_mul(*(const f2 *)&fm[q], i), f2_mul(i, i));
-                              P0 = f2_fma(w, dx, P0);
-                              P1 = f2_fma(w, dy, P1);
-                              P2 = f2_fma(w, dz, P2);
-                        }
-                        float lo, hi;
-                        f2_unpack(P0, lo, hi); o0 += (double)lo + (double)hi;
-                        f2_unpack(P1, lo, hi); o1 += (double)lo + (double)hi;
-                        f2_unpack(P2, lo, hi); o2 += (double)lo + (double)hi;
-                  }
-            } else if (OP == 1) {
-                  // the VJP's pair terms, packed as OP 0
-                  const float xr = (float)(xk - bj[0]), yr = (float)(yk - bj[1]), zr = (float)(zk - bj[2]);
-                  const f2 XT = f2_pack(xr, xr), YT = f2_pack(yr, yr), ZT = f2_pack(zr, zr), RT = f2_pack(rkf, rkf);
-                  const f2 MK = f2_pack(mkf, mkf), NLX = f2_pack(-lxkf, -lxkf), NLY = f2_pack(-lykf, -lykf),
-                           NLZ = f2_pack(-lzkf, -lzkf), NEG3 = f2_pack(-3.f, -3.f);
-                  // sources q, q + 1 packed, four per 128-bit shared load (a far tile is
-                  // padded with far, massless sources up to a multiple of four)
-                  const int ce = (cnt + 3) & ~3;
-                  for (int q0 = 0; q0 < ce; q0 += 64) {
-                        f2 P0 = 0ull, P1 = 0ull, P2 = 0ull, P3 = 0ull;
-                        const int qe = min(ce, q0 + 64);
-                        auto term = [&](f2 XS, f2 YS, f2 ZS, f2 RS, f2 mj, f2 LX, f2 LY, f2 LZ) {
-                              const f2 rx = f2_sub(XS, XT), ry = f2_sub(YS, YT), rz = f2_sub(ZS, ZT);
-                              f2 d2;
-                              if (SOFT) {
-                                    const f2 e = f2_add(RS, RT);
-                                    d2 = f2_fma(rx, rx, f2_mul(e, e));
-                              } else {
-                                    d2 = f2_mul(rx, rx);
-                              }
-                              d2 = f2_fma(ry, ry, d2);
-                              d2 = f2_fma(rz, rz, d2);
-                              const f2 ri = f2_rsqrt(d2);
-                              const f2 r2i = f2_mul(ri, ri);
-                              const f2 i3 = f2_mul(r2i, ri), i5 = f2_mul(i3, r2i);
-                              // w = m_k lambda_j - m_j lambda_k
-                              const f2 wx = f2_fma(mj, NLX, f2_mul(MK, LX)), wy = f2_fma(mj, NLY, f2_mul(MK, LY));
-                              const f2 wz = f2_fma(mj, NLZ, f2_mul(MK, LZ));
-                              const f2 rw = f2_fma(rz, wz, f2_fma(ry, wy, f2_mul(rx, wx)));
-                              const f2 nc = f2_mul(f2_mul(NEG3, rw), i5);  // -3 (r . w) / D^5
-                              P0 = f2_fma(wx, i3, f2_fma(rx, nc, P0));
-                              P1 = f2_fma(wy, i3, f2_fma(ry, nc, P1));
-                              P2 = f2_fma(wz, i3, f2_fma(rz, nc, P2));
-                              const f2 lr = f2_fma(LZ, rz, f2_fma(LY, ry, f2_mul(LX, rx)));
-                              P3 = f2_sub(P3, f2_mul(lr, i3));
-                        };
-#pragma unroll 1
-                        for (int q = q0; q < qe; q += 4) {
-                              const ulonglong2 X = *(const ulonglong2 *)&fx[q], Y = *(const ulonglong2 *)&fy[q];
-                              const ulonglong2 Z = *(const ulonglong2 *)&fz[q], M = *(const ulonglong2 *)&fm[q];
-                              const ulonglong2 LX = *(const ulonglong2 *)&flx[q], LY = *(const ulonglong2 *)&fly[q];
-                              const ulonglong2 LZ = *(const ulonglong2 *)&flz[q];
-                              ulonglong2 R = make_ulonglong2(0ull, 0ull);
-                              if (SOFT) R = *(const ulonglong2 *)&fr[q];
-                              term(X.x, Y.x, Z.x, R.x, M.x, LX.x, LY.x, LZ.x);
-                              term(X.y, Y.y, Z.y, R.y, M.y, LX.y, LY.y, LZ.y);
-                        }
-                        float lo, hi;
-                        f2_unpack(P0, lo, hi); o0 += (double)lo + (double)hi;
-                        f2_unpack(P1, lo, hi); o1 += (double)lo + (double)hi;
-                        f2_unpack(P2, lo, hi); o2 += (double)lo + (double)hi;
-                        f2_unpack(P3, lo, hi); o3 += (double)lo + (double)hi;
-                  }
-            } else {  // OP 2 (the JVP), scalar FP32
+            } else {
                   const float xr = (float)(xk - bj[0]), yr = (float)(yk - bj[1]), zr = (float)(zk - bj[2]);
                   for (int q0 = 0; q0 < cnt; q0 += 64) {  // FP32 runs of 64 sources
                         float p0 = 0.f, p1 = 0.f, p2 = 0.f;
@@ -323,9 +206,77 @@ __global__ void __launch_bounds__(AT) k_pairs_mx(Src s, int n, int tpc, const do
             }
       }
       if (act) {
-            double *p = part + (size_t)blockIdx.x * (OP == 1 ? 4 : 3) * stride;
+            double *p = part + (size_t)blockIdx.x * 3 * stride;
             p[k] = o0; p[stride + k] = o1; p[2 * stride + k] = o2;
-            if (OP == 1) p[3 * stride + k] = o3;
+      }
+}
+
+// The pair sums' tile data of positions pos (3 blocks of n), one warp per tile:
+// FP64 records and, with `mixed`, the tile's box and its FP32 copy.  pos_out
+// (may be null): a copy of pos and, behind it, of the central body's position.
+// lv (may be null): the reverse sweep's adjoint velocities, first advanced by the
+// adjoint of the drift, lv += dt lx (and LV += dt LX), then copied to l32.
+__global__ void k_lf_tiles(const double *__restrict__ pos, const double *__restrict__ m, int n, int ntiles, int mixed,
+                           D4 *__restrict__ s64, float *__restrict__ s32, double *__restrict__ box,
+                           double *__restrict__ pos_out, const double *__restrict__ cm, double dt,
+                           const double *__restrict__ lx, double *__restrict__ lv, float *__restrict__ l32,
+                           const double *__restrict__ LX, double *__restrict__ LV)
+{
+      const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+      if (warp >= ntiles) return;
+      if (warp == 0 && lane < 3) {
+            if (pos_out) pos_out[3 * (size_t)n + lane] = cm[lane];
+            if (lv) LV[lane] += dt * LX[lane];
+      }
+      const int base = warp * PT;
+      D4 b[PU];
+      double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+#pragma unroll
+      for (int u = 0; u < PU; u++) {
+            const int k = base + lane + 32 * u;
+            if (k < n) {
+                  b[u] = D4{pos[k], pos[(size_t)n + k], pos[2 * (size_t)n + k], m[k]};
+                  s64[k] = b[u];
+                  if (pos_out) {
+                        pos_out[k] = b[u].x;
+                        pos_out[(size_t)n + k] = b[u].y;
+                        pos_out[2 * (size_t)n + k] = b[u].z;
+                  }
+                  lo[0] = fmin(lo[0], b[u].x); hi[0] = fmax(hi[0], b[u].x);
+                  lo[1] = fmin(lo[1], b[u].y); hi[1] = fmax(hi[1], b[u].y);
+                  lo[2] = fmin(lo[2], b[u].z); hi[2] = fmax(hi[2], b[u].z);
+            }
+            if (lv)
+                  for (int d = 0; d < 3; d++) {
+                        double v = 0.;
+                        if (k < n) {
+                              const size_t q = (size_t)d * n + k;
+                              v = lv[q] + dt * lx[q];
+                              lv[q] = v;
+                        }
+                        if (mixed) l32[((size_t)warp * 3 + d) * PT + lane + 32 * u] = (float)v;
+                  }
+      }
+      if (!mixed) return;
+      for (int o = 16; o > 0; o >>= 1)
+            for (int d = 0; d < 3; d++) {
+                  lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                  hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+            }
+      const double c[3] = {0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2])};
+      if (lane < 3) {
+            box[warp * 6 + lane] = c[lane];
+            box[warp * 6 + 3 + lane] = 0.5 * (hi[lane] - lo[lane]);
+      }
+      float *tile = s32 + (size_t)warp * 4 * PT;
+#pragma unroll
+      for (int u = 0; u < PU; u++) {
+            const int j = lane + 32 * u;
+            const bool in = base + j < n;
+            tile[j] = in ? (float)(b[u].x - c[0]) : 1e18f;
+            tile[PT + j] = in ? (float)(b[u].y - c[1]) : 1e18f;
+            tile[2 * PT + j] = in ? (float)(b[u].z - c[2]) : 1e18f;
+            tile[3 * PT + j] = in ? (float)b[u].w : 0.f;
       }
 }
 
@@ -352,68 +303,135 @@ __device__ __forceinline__ void block_sum3(double v0, double v1, double v2, doub
 }
 
 
-// acc = G * sum of chunk partials + central term; per-body CM_acc terms.
-__global__ void __launch_bounds__(SB) k_force_final(const double *__restrict__ part, int nch, long stride, Src s,
-                                                    int n, const double *__restrict__ cm, double G, double M,
-                                                    int central, double *ax, double *ay, double *az,
-                                                    double *__restrict__ red)
+// The sum over the grid of one value per lane of each block's warp 0 (three
+// components), by the last block to arrive: every block leaves its warp's sums in
+// red, the last one adds them in block order (deterministic).  True for the
+// threads of the last block, with the sums in tot[3] (shared).  count returns to 0.
+__device__ __forceinline__ bool grid_sum3(double v0, double v1, double v2, double *__restrict__ red,
+                                          unsigned *__restrict__ count, double *tot)
 {
-      const int k = blockIdx.x * blockDim.x + threadIdx.x;
-      double c[3] = {0., 0., 0.};
-      if (k < n) {
-            double a[3] = {0., 0., 0.};
-#pragma unroll 8  // the chunks' loads in flight together (sums still in chunk order)
-            for (int ch = 0; ch < nch; ch++)
-                  for (int d = 0; d < 3; d++) a[d] += part[(size_t)ch * 3 * stride + d * stride + k];
-            for (int d = 0; d < 3; d++) a[d] *= G;
-            if (central) {
-                  double sx = s.x[k] - cm[0], sy = s.y[k] - cm[1], sz = s.z[k] - cm[2];
-                  double r2 = sx * sx + sy * sy + sz * sz;
-                  double ri = rsqrt(r2), i3 = ri * ri * ri;
-                  a[0] -= G * M * sx * i3; a[1] -= G * M * sy * i3; a[2] -= G * M * sz * i3;
-                  double g = G * s.m[k] * i3;
-                  c[0] = g * sx; c[1] = g * sy; c[2] = g * sz;
+      __shared__ double sh[3][SB];
+      __shared__ int last;
+      if (threadIdx.x < 32) {
+            for (int o = 16; o > 0; o >>= 1) {
+                  v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+                  v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+                  v2 += __shfl_xor_sync(0xffffffffu, v2, o);
             }
-            ax[k] = a[0]; ay[k] = a[1]; az[k] = a[2];
+            if (threadIdx.x == 0) {
+                  red[3 * blockIdx.x] = v0;
+                  red[3 * blockIdx.x + 1] = v1;
+                  red[3 * blockIdx.x + 2] = v2;
+                  __threadfence();
+                  last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+            }
       }
-      if (central) block_sum3(c[0], c[1], c[2], red);  // the CM_acc terms (central is uniform)
+      __syncthreads();
+      if (!last) return false;
+      __threadfence();
+      double s[3] = {0., 0., 0.};
+      for (int b = threadIdx.x; b < (int)gridDim.x; b += SB)
+            for (int d = 0; d < 3; d++) s[d] += __ldcg(red + 3 * b + d);
+      for (int d = 0; d < 3; d++) sh[d][threadIdx.x] = s[d];
+      __syncthreads();
+      for (int o = SB / 2; o > 0; o >>= 1) {
+            if (threadIdx.x < o)
+                  for (int d = 0; d < 3; d++) sh[d][threadIdx.x] += sh[d][threadIdx.x + o];
+            __syncthreads();
+      }
+      if (threadIdx.x < 3) tot[threadIdx.x] = sh[threadIdx.x][0];
+      __syncthreads();
+      return true;
 }
 
-// VJP outputs: mu (3), nu (1) per body; per-body terms of the CM-position VJP.
-__global__ void __launch_bounds__(SB) k_vjp_final(const double *__restrict__ part, int nch, long stride, Src s,
-                                                  int n, const double *__restrict__ cm,
-                                                  const double *__restrict__ Lam, double G, double M, int central,
-                                                  double *mux, double *muy, double *muz, double *nu,
-                                                  double *__restrict__ red)
+// The force's final pass, 32 bodies a block: a = G * (the pair sums) + central
+// term, then the kick v += dt a and the drift x += dt v; the last block kicks and
+// drifts the central body with the sum of its terms.
+__global__ void __launch_bounds__(SB) k_lf_force(PairRun pr, int n, double *__restrict__ X, double *__restrict__ V,
+                                                 const double *__restrict__ m, double *__restrict__ cm, double G,
+                                                 double M, int central, double dt, double *__restrict__ red,
+                                                 unsigned *__restrict__ count)
 {
-      const int k = blockIdx.x * blockDim.x + threadIdx.x;
-      double xt[3] = {0., 0., 0.};
-      if (k < n) {
-      double o[4] = {0., 0., 0., 0.};
-#pragma unroll 8  // the chunks' loads in flight together (sums still in chunk order)
-      for (int c = 0; c < nch; c++)
-            for (int d = 0; d < 4; d++) o[d] += part[(size_t)c * 4 * stride + d * stride + k];
-      for (int d = 0; d < 4; d++) o[d] *= G;
-      if (central) {
-            double sv[3] = {s.x[k] - cm[0], s.y[k] - cm[1], s.z[k] - cm[2]};
-            double r2 = sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2];
-            double ri = rsqrt(r2), i3 = ri * ri * ri, i5 = i3 * ri * ri;
-            double mk = s.m[k];
-            double lam[3] = {s.lx[k], s.ly[k], s.lz[k]};
-            // w = m_k Lambda - M lambda_k ;  J w = w/|s|^3 - 3 s (s.w)/|s|^5
-            double w[3], sw = 0.;
-            for (int d = 0; d < 3; d++) { w[d] = mk * Lam[d] - M * lam[d]; sw += sv[d] * w[d]; }
-            double Jw[3];
-            for (int d = 0; d < 3; d++) Jw[d] = w[d] * i3 - 3.0 * sv[d] * sw * i5;
+      __shared__ double sh[3][8][32];
+      __shared__ double tot[3];
+      const long k = (long)blockIdx.x * 32 + (threadIdx.x & 31);
+      double a[3], c[3] = {0., 0., 0.};
+      pair_rows_sum<3>(pr.part, pr.npad, pr.nb, (int)(k / pr.bsize), pr.k0, pr.nk, k, k < n, sh, a);
+      if (threadIdx.x < 32 && k < n) {
+            double x[3];
             for (int d = 0; d < 3; d++) {
-                  o[d] += G * Jw[d];
-                  xt[d] = -G * Jw[d];  // G J (M lambda - m Lambda)
+                  if (pr.base) a[d] = pr.base[d * pr.npad + k] + a[d];
+                  a[d] *= G;
+                  x[d] = X[(size_t)d * n + k];
             }
-            o[3] += G * (Lam[0] * sv[0] + Lam[1] * sv[1] + Lam[2] * sv[2]) * i3;
+            if (central) {
+                  double s[3] = {x[0] - cm[0], x[1] - cm[1], x[2] - cm[2]};
+                  double r2 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+                  double ri = rsqrt(r2), i3 = ri * ri * ri;
+                  const double g = G * m[k] * i3;
+                  for (int d = 0; d < 3; d++) {
+                        a[d] -= G * M * s[d] * i3;
+                        c[d] = g * s[d];
+                  }
+            }
+            for (int d = 0; d < 3; d++) {
+                  const size_t q = (size_t)d * n + k;
+                  const double v = V[q] + dt * a[d];
+                  V[q] = v;
+                  X[q] = x[d] + dt * v;
+            }
       }
-      mux[k] = o[0]; muy[k] = o[1]; muz[k] = o[2]; nu[k] = o[3];
+      if (!central) return;
+      if (grid_sum3(c[0], c[1], c[2], red, count, tot) && threadIdx.x < 3) {
+            const double v = cm[3 + threadIdx.x] + dt * tot[threadIdx.x];
+            cm[3 + threadIdx.x] = v;
+            cm[threadIdx.x] += dt * v;
       }
-      if (central) block_sum3(xt[0], xt[1], xt[2], red);  // the CM-position VJP's terms
+}
+
+// The VJP's final pass: lx += dt (its position part), gm += dt (its mass part);
+// the last block advances the central body's LX.
+__global__ void __launch_bounds__(SB) k_lf_vjp(PairRun pr, int n, const double *__restrict__ pos,
+                                               const double *__restrict__ m, const double *__restrict__ lv,
+                                               const double *__restrict__ cm, const double *__restrict__ Lam, double G,
+                                               double M, int central, double dt, double *__restrict__ lx,
+                                               double *__restrict__ gm, double *__restrict__ LX,
+                                               double *__restrict__ red, unsigned *__restrict__ count)
+{
+      __shared__ double sh[4][8][32];
+      __shared__ double tot[3];
+      const long k = (long)blockIdx.x * 32 + (threadIdx.x & 31);
+      double o[4], xt[3] = {0., 0., 0.};
+      pair_rows_sum<4>(pr.part, pr.npad, pr.nb, (int)(k / pr.bsize), pr.k0, pr.nk, k, k < n, sh, o);
+      if (threadIdx.x < 32 && k < n) {
+            for (int d = 0; d < 4; d++) {
+                  if (pr.base) o[d] = pr.base[d * pr.npad + k] + o[d];
+                  o[d] *= G;
+            }
+            if (central) {
+                  double sv[3], lam[3];
+                  for (int d = 0; d < 3; d++) {
+                        sv[d] = pos[(size_t)d * n + k] - cm[d];
+                        lam[d] = lv[(size_t)d * n + k];
+                  }
+                  double r2 = sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2];
+                  double ri = rsqrt(r2), i3 = ri * ri * ri, i5 = i3 * ri * ri;
+                  const double mk = m[k];
+                  // w = m_k Lambda - M lambda_k ;  J w = w/|s|^3 - 3 s (s.w)/|s|^5
+                  double w[3], sw = 0.;
+                  for (int d = 0; d < 3; d++) { w[d] = mk * Lam[d] - M * lam[d]; sw += sv[d] * w[d]; }
+                  for (int d = 0; d < 3; d++) {
+                        const double Jw = w[d] * i3 - 3.0 * sv[d] * sw * i5;
+                        o[d] += G * Jw;
+                        xt[d] = -G * Jw;  // G J (M lambda - m Lambda)
+                  }
+                  o[3] += G * (Lam[0] * sv[0] + Lam[1] * sv[1] + Lam[2] * sv[2]) * i3;
+            }
+            for (int d = 0; d < 3; d++) lx[(size_t)d * n + k] += dt * o[d];
+            gm[k] += dt * o[3];
+      }
+      if (!central) return;
+      if (grid_sum3(xt[0], xt[1], xt[2], red, count, tot) && threadIdx.x < 3) LX[threadIdx.x] += dt * tot[threadIdx.x];
 }
 
 // JVP: d a = G * sum of chunk partials - G M J_k (dx_k - dX); per-body terms
@@ -471,97 +489,63 @@ __global__ void k_axpy3(double a, const double *__restrict__ x, double *__restri
       if (k < 3 && cmy) cmy[k] += a * cmx[k];
 }
 
-__global__ void k_axpy1(double a, const double *__restrict__ x, double *__restrict__ y, int n)
-{
-      int k = blockIdx.x * blockDim.x + threadIdx.x;
-      if (k < n) y[k] += a * x[k];
-}
-
 }  // namespace
 
 namespace {
 
 struct LF {
-      int n, ntiles, tpc, nch, np;
-      bool soft, central;
-      double G, M;
-      double *X, *V, *m, *sR, *cm, *acc, *part, *red, *acm;
-      double *lx, *lv, *LX, *LV, *mu, *nu, *gm, *muX;
+      int n, ntiles, tpc, nch;
+      int soft;                    // 0: none, 1: uniform (eps2), 2: general
+      bool central;
+      double G, M, eps2;
+      double *X, *V, *m, *sR, *cm, *out, *part, *red;
+      double *lx, *lv, *LX, *LV, *gm;
       double *ckpt, *seg;
       double *tx, *tv, *tm, *tX, *da, *dA;  // tangents (JVP)
+      double *jpart;               // the JVP's chunk partials
+      D4 *s64;
+      float *s32, *sR32, *l32;
+      unsigned *count;
+      PairPlan pf, pv;             // the force's and the VJP's pair sums
       int C, ncp;
-      bool mixed;                  // MIXED gravity mode: k_pairs_mx with tile boxes
+      bool mixed;                  // MIXED gravity mode
       double theta, *box;
-      double *boxseg;              // mixed mode: the tile boxes of a segment's recomputed steps
       cudaStream_t st;
 };
 
-// the pair sums of OP over positions pos; the mixed mode's tile boxes in box
-// (null: L.box), computed from pos first unless `have_box`
+// the pair sums of OP over positions pos; VJP: after lv += dt lx.  pos_out: see k_lf_tiles.
 template <int OP>
-int lf_pairs(LF &L, const Src &s, const double *pos, double *box = nullptr, bool have_box = false)
+int lf_pairs(LF &L, const double *pos, const double *cmpos, double *pos_out, double dt, PairRun &run)
 {
       const int n = L.n;
-      dim3 grid(L.nch, L.ntiles);
-      if (L.mixed) {
-            if (!box) box = L.box;
-            if (!have_box) {
-                  k_adj_tilebox<<<(L.ntiles * 32 + 255) / 256, 256, 0, L.st>>>(pos, n, L.ntiles, box);
-                  NCG_LAUNCHED();
-            }
-            if (L.soft) k_pairs_mx<OP, true><<<grid, AT, 0, L.st>>>(s, n, L.tpc, box, L.theta, L.part, n);
-            else k_pairs_mx<OP, false><<<grid, AT, 0, L.st>>>(s, n, L.tpc, box, L.theta, L.part, n);
-      } else {
-            if (L.soft) k_pairs<OP, true><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.part, n);
-            else k_pairs<OP, false><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.part, n);
-      }
+      k_lf_tiles<<<(L.ntiles * 32 + 127) / 128, 128, 0, L.st>>>(pos, L.m, n, L.ntiles, L.mixed, L.s64, L.s32, L.box,
+                                                                pos_out, cmpos, dt, L.lx, OP == 1 ? L.lv : nullptr,
+                                                                L.l32, L.LX, L.LV);
+      NCG_LAUNCHED();
+      PairData pd{L.s64, L.sR, L.s32, L.sR32, L.box, n, L.ntiles, 0, L.lv, L.l32};
+      return pair_sums<OP>(pd, OP == 0 ? L.pf : L.pv, L.mixed ? 0 : 1, L.soft, L.theta, L.eps2, L.part, run, L.st);
+}
+
+// kick (v += dt a, CM too) then drift (x += dt v, CM too); pos_out (may be null):
+// the positions that the kick sees
+int lf_step(LF &L, double dt, double *pos_out = nullptr)
+{
+      PairRun run;
+      NCG_TRY(lf_pairs<0>(L, L.X, L.cm, pos_out, dt, run));
+      k_lf_force<<<(L.n + 31) / 32, SB, 0, L.st>>>(run, L.n, L.X, L.V, L.m, L.cm, L.G, L.M, L.central, dt, L.red,
+                                                   L.count);
       NCG_LAUNCHED();
       return NCGPU_OK;
 }
 
-int lf_force(LF &L, const double *pos, const double *cmpos, double *box = nullptr)
+// The adjoint of one kick and drift: lv += dt lx, then lx and gm by the kick's VJP.
+int lf_vjp(LF &L, const double *pos, const double *cmpos, double dt)
 {
-      const int n = L.n;
-      Src s{pos, pos + n, pos + 2 * n, L.m, L.sR, nullptr, nullptr, nullptr};
-      NCG_TRY(lf_pairs<0>(L, s, pos, box));
-      const int nb = (n + SB - 1) / SB;
-      k_force_final<<<nb, SB, 0, L.st>>>(L.part, L.nch, n, s, n, cmpos, L.G, L.M, L.central, L.acc, L.acc + n,
-                                         L.acc + 2 * n, L.red);
+      PairRun run;
+      NCG_TRY(lf_pairs<1>(L, pos, cmpos, nullptr, dt, run));
+      k_lf_vjp<<<(L.n + 31) / 32, SB, 0, L.st>>>(run, L.n, pos, L.m, L.lv, cmpos, L.LV, L.G, L.M, L.central, dt, L.lx,
+                                                 L.gm, L.LX, L.red, L.count);
       NCG_LAUNCHED();
-      if (L.central) {
-            k_sum3f<<<1, 32, 0, L.st>>>(L.red, nb, L.acm);
-            NCG_LAUNCHED();
-      }
-      return NCGPU_OK;
-}
-
-// kick (v += dt a, CM too) then drift (x += dt v, CM too); box: where the
-// force's tile boxes go (null: L.box)
-int lf_step(LF &L, double dt, double *box = nullptr)
-{
-      NCG_TRY(lf_force(L, L.X, L.cm, box));
-      const int n = L.n, nb = (n + 255) / 256;
-      k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.acc, L.V, n, n, L.acm, L.central ? L.cm + 3 : nullptr);
-      NCG_LAUNCHED();
-      k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.V, L.X, n, n, L.cm + 3, L.central ? L.cm : nullptr);
-      NCG_LAUNCHED();
-      return NCGPU_OK;
-}
-
-// box: the tile boxes of pos when known (null: computed)
-int lf_vjp(LF &L, const double *pos, const double *cmpos, double *box = nullptr)
-{
-      const int n = L.n;
-      Src s{pos, pos + n, pos + 2 * n, L.m, L.sR, L.lv, L.lv + n, L.lv + 2 * n};
-      NCG_TRY(lf_pairs<1>(L, s, pos, box, box != nullptr));
-      const int nb = (n + SB - 1) / SB;
-      k_vjp_final<<<nb, SB, 0, L.st>>>(L.part, L.nch, n, s, n, cmpos, L.LV, L.G, L.M, L.central, L.mu, L.mu + n,
-                                       L.mu + 2 * n, L.nu, L.red);
-      NCG_LAUNCHED();
-      if (L.central) {
-            k_sum3f<<<1, 32, 0, L.st>>>(L.red, nb, L.muX);
-            NCG_LAUNCHED();
-      }
       return NCGPU_OK;
 }
 
@@ -569,22 +553,28 @@ int lf_vjp(LF &L, const double *pos, const double *cmpos, double *box = nullptr)
 int lf_step_jvp(LF &L, double dt)
 {
       const int n = L.n, nb = (n + 255) / 256;
-      NCG_TRY(lf_force(L, L.X, L.cm));
       Src s{L.X, L.X + n, L.X + 2 * n, L.m, L.sR, L.tx, L.tx + n, L.tx + 2 * n, L.tm};
-      NCG_TRY(lf_pairs<2>(L, s, L.X));
+      dim3 grid(L.nch, L.ntiles);
+      if (L.mixed) {
+            k_adj_tilebox<<<(L.ntiles * 32 + 255) / 256, 256, 0, L.st>>>(L.X, n, L.ntiles, L.box);
+            NCG_LAUNCHED();
+            if (L.soft) k_pairs_jvp_mx<true><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.box, L.theta, L.jpart, n);
+            else k_pairs_jvp_mx<false><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.box, L.theta, L.jpart, n);
+      } else {
+            if (L.soft) k_pairs_jvp<true><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.jpart, n);
+            else k_pairs_jvp<false><<<grid, AT, 0, L.st>>>(s, n, L.tpc, L.jpart, n);
+      }
+      NCG_LAUNCHED();
       const int nbs = (n + SB - 1) / SB;
-      k_jvp_final<<<nbs, SB, 0, L.st>>>(L.part, L.nch, n, s, n, L.cm, L.tX, L.G, L.M, L.central, L.da, L.da + n,
+      k_jvp_final<<<nbs, SB, 0, L.st>>>(L.jpart, L.nch, n, s, n, L.cm, L.tX, L.G, L.M, L.central, L.da, L.da + n,
                                         L.da + 2 * n, L.red);
       NCG_LAUNCHED();
       if (L.central) {
             k_sum3f<<<1, 32, 0, L.st>>>(L.red, nbs, L.dA);
             NCG_LAUNCHED();
       }
-      k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.acc, L.V, n, n, L.acm, L.central ? L.cm + 3 : nullptr);
-      NCG_LAUNCHED();
+      NCG_TRY(lf_step(L, dt));
       k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.da, L.tv, n, n, L.dA, L.central ? L.tX + 3 : nullptr);
-      NCG_LAUNCHED();
-      k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.V, L.X, n, n, L.cm + 3, L.central ? L.cm : nullptr);
       NCG_LAUNCHED();
       k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.tv, L.tx, n, n, L.tX + 3, L.central ? L.tX : nullptr);
       NCG_LAUNCHED();
@@ -605,11 +595,15 @@ void join3(double *dst, const double *src, int n, cudaStream_t st, cudaError_t *
                                    cudaMemcpyDeviceToHost, st);
 }
 
-// sR = sp * R, element by element (in place when sR == R)
-__global__ void k_scale_R(const double *R, double sp, double *sR, int n)
+// sR = sp * R, element by element (in place when sR == R), and its FP32 copy with
+// zero padding up to npad
+__global__ void k_scale_R(const double *R, double sp, double *sR, int n, float *__restrict__ sR32, int npad)
 {
       int k = blockIdx.x * blockDim.x + threadIdx.x;
-      if (k < n) sR[k] = sp * R[k];
+      if (k >= npad) return;
+      const double r = k < n ? sp * R[k] : 0.;
+      if (k < n) sR[k] = r;
+      sR32[k] = (float)r;
 }
 
 __global__ void k_xf(const double *__restrict__ X, const double *__restrict__ V, double h, double *__restrict__ out,
@@ -635,32 +629,46 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
       L.G = c.P.par_G;
       L.M = a->cm[6];
       L.central = c.P.par_central_mass_bool != 0;
-      L.soft = c.P.par_softening_parameter != 0.;
-      L.ntiles = (n + AT - 1) / AT;
-      if (mixed) {
-            // (target tile, source chunk) work units: about 8 per resident CTA
-            // slot, so that the last wave is short
-            int occ = 1;
-            NCG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pairs_mx<1, true>, AT, 0));
-            const long want = 8L * std::max(occ, 1) * c.sm_count;
-            L.nch = (int)std::max(1L, std::min((long)L.ntiles, (want + L.ntiles - 1) / L.ntiles));
-      } else {
-            L.nch = std::max(1, std::min(L.ntiles, (2048 + L.ntiles - 1) / L.ntiles));
+      const double sp = c.P.par_softening_parameter;
+      L.soft = 0;
+      L.eps2 = 0.;
+      if (sp != 0.) {  // all radii equal: one softening length
+            const auto mm = std::minmax_element(a->R, a->R + n);
+            L.soft = *mm.first == *mm.second ? 1 : 2;
+            const double eu = 2.0 * sp * a->R[0];
+            L.eps2 = eu * eu;
       }
-      L.tpc = (L.ntiles + L.nch - 1) / L.nch;
-      L.nch = (L.ntiles + L.tpc - 1) / L.tpc;
-      L.np = (n + SB - 1) / SB;  // blocks of the fold kernels: their CM sums in red
+      L.ntiles = (n + AT - 1) / AT;
+      L.nch = 0;
+      if (jvp) {
+            if (mixed) {
+                  // (target tile, source chunk) work units: about 8 per resident CTA
+                  // slot, so that the last wave is short
+                  int occ = 1;
+                  NCG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pairs_jvp_mx<true>, AT, 0));
+                  const long want = 8L * std::max(occ, 1) * c.sm_count;
+                  L.nch = (int)std::max(1L, std::min((long)L.ntiles, (want + L.ntiles - 1) / L.ntiles));
+            } else {
+                  L.nch = std::max(1, std::min(L.ntiles, (2048 + L.ntiles - 1) / L.ntiles));
+            }
+            L.tpc = (L.ntiles + L.nch - 1) / L.nch;
+            L.nch = (L.ntiles + L.tpc - 1) / L.tpc;
+      }
+      L.pf = pair_plan<0>(n);
+      L.pv = pair_plan<1>(n);
       L.mixed = mixed;
       L.theta = c.P.par_near_theta > 0. ? c.P.par_near_theta : 0.15;
       L.C = a->checkpoint > 0 ? a->checkpoint : 32;
       L.ncp = (a->nsteps + L.C - 1) / L.C + 1;
-      const size_t N = (size_t)n, st = 6 * N + 6;
-      size_t total = 3 * N * 2 + 2 * N + 6 + 3 * N + 4 * N * L.nch + 3 * (size_t)L.np + 3  // X V m sR cm acc part red acm
-                     + 3 * N * 2 + 6 + 3 * N + N + N + 3                              // lx lv LX LV mu nu gm muX
-                     + st * L.ncp + (size_t)L.C * (3 * N + 3)                         // checkpoints, segment
-                     + 3 * N * 3 + N + 6 + 3                                          // tx tv tm tX da dA
-                     + 6 * (size_t)L.ntiles                                           // tile boxes
-                     + (mixed && vjp ? 6 * (size_t)L.ntiles * L.C : 0);               // a segment's boxes
+      const size_t N = (size_t)n, st = 6 * N + 6, NP = (size_t)L.ntiles * AT;
+      const size_t nred = (N + 31) / 32;  // blocks of the final passes
+      const size_t npart = vjp ? std::max(L.pf.doubles, L.pv.doubles) : L.pf.doubles;
+      size_t total = 4 * NP + 2 * NP + NP / 2 + 3 * NP / 2 + 2                   // s64 s32 sR32 l32 count
+                     + 3 * N * 2 + 2 * N + 6 + 3 * N + npart + 3 * nred          // X V m sR cm out part red
+                     + 3 * N * 2 + 6 + N                                         // lx lv LX LV gm
+                     + (vjp ? st * L.ncp + (size_t)L.C * (3 * N + 3) : 0)        // checkpoints, segment
+                     + (jvp ? 3 * N * 3 + N + 6 + 3 + 3 * N * L.nch : 0)         // tx tv tm tX da dA, partials
+                     + 6 * (size_t)L.ntiles;                                     // tile boxes
       if (total > c.lf_cap) {  // grown when needed, kept for the next call
             if (c.lf_buf) cudaFree(c.lf_buf);
             c.lf_buf = nullptr;
@@ -670,15 +678,23 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
       }
       double *p = c.lf_buf;
       auto take = [&](size_t k) { double *q = p; p += k; return q; };
+      L.s64 = (D4 *)take(4 * NP);  // (the widest alignment first)
+      L.s32 = (float *)take(2 * NP);
+      L.sR32 = (float *)take(NP / 2);
+      L.l32 = (float *)take(3 * NP / 2);
+      L.count = (unsigned *)take(2);
       L.X = take(3 * N); L.V = take(3 * N); L.m = take(N); L.sR = take(N); L.cm = take(6);
-      L.acc = take(3 * N); L.part = take(4 * N * L.nch); L.red = take(3 * (size_t)L.np);
-      L.acm = take(3);
-      L.lx = take(3 * N); L.lv = take(3 * N); L.LX = take(3); L.LV = take(3); L.mu = take(3 * N); L.nu = take(N);
-      L.gm = take(N); L.muX = take(3);
-      L.ckpt = take(st * L.ncp); L.seg = take((size_t)L.C * (3 * N + 3));
-      L.tx = take(3 * N); L.tv = take(3 * N); L.tm = take(N); L.tX = take(6); L.da = take(3 * N); L.dA = take(3);
+      L.out = take(3 * N); L.part = take(npart); L.red = take(3 * nred);
+      L.lx = take(3 * N); L.lv = take(3 * N); L.LX = take(3); L.LV = take(3); L.gm = take(N);
+      if (vjp) {
+            L.ckpt = take(st * L.ncp);
+            L.seg = take((size_t)L.C * (3 * N + 3));
+      }
+      if (jvp) {
+            L.tx = take(3 * N); L.tv = take(3 * N); L.tm = take(N); L.tX = take(6); L.da = take(3 * N); L.dA = take(3);
+            L.jpart = take(3 * N * L.nch);
+      }
       L.box = take(6 * (size_t)L.ntiles);
-      L.boxseg = take(mixed && vjp ? 6 * (size_t)L.ntiles * L.C : 0);
       int status = NCGPU_OK;
       cudaError_t e = cudaSuccess;
       const double h = a->dt / 2.0, dt = a->dt;
@@ -688,7 +704,7 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
       if (e == cudaSuccess) e = cudaMemcpyAsync(L.m, a->m, sizeof(double) * N, cudaMemcpyHostToDevice, L.st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(L.sR, a->R, sizeof(double) * N, cudaMemcpyHostToDevice, L.st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(L.cm, a->cm, 6 * sizeof(double), cudaMemcpyHostToDevice, L.st);
-      if (e == cudaSuccess) e = cudaMemsetAsync(L.acm, 0, 3 * sizeof(double), L.st);
+      if (e == cudaSuccess) e = cudaMemsetAsync(L.count, 0, sizeof(unsigned), L.st);
       if (e != cudaSuccess) return cuda_fail(e, "leapfrog upload", __FILE__, __LINE__);
 #define LF_TRY(call)                         \
       do {                                   \
@@ -700,7 +716,7 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
             cudaError_t e_ = cudaGetLastError();                                      \
             if (e_ != cudaSuccess) { status = cuda_fail(e_, "launch", __FILE__, __LINE__); goto done; } \
       } while (0)
-      k_scale_R<<<nb, 256, 0, L.st>>>(L.sR, c.P.par_softening_parameter, L.sR, n);
+      k_scale_R<<<(int)((NP + 255) / 256), 256, 0, L.st>>>(L.sR, sp, L.sR, n, L.sR32, (int)NP);
       LF_LAUNCHED();
       if (jvp) {
             split3(L.tx, a->tan_x0, n, L.st, &e);
@@ -732,9 +748,9 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
             if (e != cudaSuccess) { status = cuda_fail(e, "tangent download", __FILE__, __LINE__); goto done; }
       }
       if (a->x_final || a->v_final) {
-            k_xf<<<nb, 256, 0, L.st>>>(L.X, L.V, h, L.acc, n);  // half back-drift of the output (src/rk4.c:929-936)
+            k_xf<<<nb, 256, 0, L.st>>>(L.X, L.V, h, L.out, n);  // half back-drift of the output (src/rk4.c:929-936)
             LF_LAUNCHED();
-            if (a->x_final) join3(a->x_final, L.acc, n, L.st, &e);
+            if (a->x_final) join3(a->x_final, L.out, n, L.st, &e);
             if (a->v_final) join3(a->v_final, L.V, n, L.st, &e);
             if (e == cudaSuccess) e = cudaStreamSynchronize(L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "leapfrog download", __FILE__, __LINE__); goto done; }
@@ -755,24 +771,12 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
                   if (e == cudaSuccess) e = cudaMemcpyAsync(L.cm, ck + 6 * N, 6 * sizeof(double), cudaMemcpyDeviceToDevice, L.st);
                   if (e != cudaSuccess) { status = cuda_fail(e, "restore", __FILE__, __LINE__); goto done; }
                   for (int s = s0; s < s1; s++) {  // recompute, keeping the positions each kick saw
-                        double *sg = L.seg + (size_t)(s - s0) * (3 * N + 3);
-                        e = cudaMemcpyAsync(sg, L.X, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, L.st);
-                        if (e == cudaSuccess) e = cudaMemcpyAsync(sg + 3 * N, L.cm, 3 * sizeof(double), cudaMemcpyDeviceToDevice, L.st);
-                        if (e != cudaSuccess) { status = cuda_fail(e, "segment", __FILE__, __LINE__); goto done; }
-                        LF_TRY(lf_step(L, dt, L.mixed ? L.boxseg + (size_t)(s - s0) * 6 * L.ntiles : nullptr));
+                        LF_TRY(lf_step(L, dt, L.seg + (size_t)(s - s0) * (3 * N + 3)));
                   }
                   for (int s = s1 - 1; s >= s0; s--) {
+                        // drift x_{s+1} = x_s + dt v_{s+1}, then kick v_{s+1} = v_s + dt a(x_s)
                         const double *sg = L.seg + (size_t)(s - s0) * (3 * N + 3);
-                        // drift x_{s+1} = x_s + dt v_{s+1}
-                        k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.lx, L.lv, n, n, L.LX, L.LV);
-                        LF_LAUNCHED();
-                        // kick v_{s+1} = v_s + dt a(x_s)
-                        // (the recomputation's boxes of these positions)
-                        LF_TRY(lf_vjp(L, sg, sg + 3 * N, L.mixed ? L.boxseg + (size_t)(s - s0) * 6 * L.ntiles : nullptr));
-                        k_axpy3<<<nb, 256, 0, L.st>>>(dt, L.mu, L.lx, n, n, L.muX, L.central ? L.LX : nullptr);
-                        LF_LAUNCHED();
-                        k_axpy1<<<nb, 256, 0, L.st>>>(dt, L.nu, L.gm, n);
-                        LF_LAUNCHED();
+                        LF_TRY(lf_vjp(L, sg, sg + 3 * N, dt));
                   }
             }
             // initial half drift x = x0 + h v0

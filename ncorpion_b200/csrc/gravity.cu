@@ -719,20 +719,6 @@ __global__ void __launch_bounds__(MXB, 12) k_grav_tiled(const D4 *__restrict__ s
       }
 }
 
-// Adds the partial rows of offsets k0 .. k0 + nk - 1 to the sums in base (3
-// blocks of npad; set instead of added to when `first`): for body counts whose
-// rows do not fit the partial buffer at once.
-__global__ void __launch_bounds__(256) k_pair_accum(const double *__restrict__ part, long npad, int nb, int k0, int nk,
-                                                    int bsize, int n, int first, double *__restrict__ base)
-{
-      __shared__ double sh[3][8][32];
-      const long q = (long)blockIdx.x * 32 + (threadIdx.x & 31);
-      double v[3];
-      pair_rows_sum(part, npad, nb, (int)(q / bsize), k0, nk, q, q < n, sh, v);
-      if (threadIdx.x < 32 && q < n)
-            for (int d = 0; d < 3; d++) base[d * npad + q] = first ? v[d] : base[d * npad + q] + v[d];
-}
-
 // Sum the chunk partials in chunk order, multiply by G, add the FP64 central
 // term and scatter back to slot order; per-body CM_acc terms for the reduction.
 __device__ __forceinline__ void grav_finish(int q, bool own, const double (&m)[3], const D4 *__restrict__ s64,
@@ -780,23 +766,21 @@ __global__ void k_grav_final(const double *__restrict__ partial, int nchunks, lo
       grav_finish(q, own, m, s64, slots, n, cmx, cmy, cmz, mu, G, central, j2, ax, ay, az, cterm);
 }
 
-// The same from the rows of k_pair_sym (offsets k0 .. k0 + nk - 1) and, when
-// not null, the sums of the earlier offsets in base.
-__global__ void __launch_bounds__(256) k_pair_final(const double *__restrict__ part, long npad, int nb, int k0, int nk,
-                                                    int bsize, const double *__restrict__ base,
-                                                    const D4 *__restrict__ s64, const int *__restrict__ slots, int n,
-                                                    double cmx, double cmy, double cmz, double mu, double G,
-                                                    int central, J2Arg j2, double *__restrict__ ax,
-                                                    double *__restrict__ ay, double *__restrict__ az,
-                                                    double *__restrict__ cterm)
+// The same from the rows of k_pair_sym and, when not null, the sums of the
+// earlier offsets in base.
+__global__ void __launch_bounds__(256) k_pair_final(PairRun pr, const D4 *__restrict__ s64,
+                                                    const int *__restrict__ slots, int n, double cmx, double cmy,
+                                                    double cmz, double mu, double G, int central, J2Arg j2,
+                                                    double *__restrict__ ax, double *__restrict__ ay,
+                                                    double *__restrict__ az, double *__restrict__ cterm)
 {
       __shared__ double sh[3][8][32];
       const long q = (long)blockIdx.x * 32 + (threadIdx.x & 31);
       double v[3];
-      pair_rows_sum(part, npad, nb, (int)(q / bsize), k0, nk, q, q < n, sh, v);
+      pair_rows_sum<3>(pr.part, pr.npad, pr.nb, (int)(q / pr.bsize), pr.k0, pr.nk, q, q < n, sh, v);
       if (threadIdx.x >= 32 || q >= n) return;
-      if (base)
-            for (int d = 0; d < 3; d++) v[d] = base[d * npad + q] + v[d];
+      if (pr.base)
+            for (int d = 0; d < 3; d++) v[d] = pr.base[d * pr.npad + q] + v[d];
       grav_finish((int)q, true, v, s64, slots, n, cmx, cmy, cmz, mu, G, central, j2, ax, ay, az, cterm);
 }
 
@@ -875,77 +859,6 @@ int finish_cm(int central, int n, double *d_cm_acc, cudaStream_t st)
       if (central) return par_sum3(c.cmterm, n, nullptr, d_cm_acc, st);
       k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
       NCG_LAUNCHED();
-      return NCGPU_OK;
-}
-
-// What pair_sums left in ctx().partial for the final pass: the rows of offsets
-// k0 .. k0 + nk - 1, and the sums of the earlier ones in base (or null).
-struct PairRun {
-      int nb, bsize, k0, nk;
-      long npad;
-      const double *base;
-};
-
-template <int MODE, int SOFT, int B, int W>
-int pair_launch(const PairData &pd, int k0, int nk, double theta, double eps2, long npad, cudaStream_t st)
-{
-      constexpr size_t smem = pair_smem<MODE, SOFT, B, W>();
-      if (smem > 48 * 1024)
-            NCG_CK(cudaFuncSetAttribute(k_pair_sym<MODE, SOFT, B, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-      k_pair_sym<MODE, SOFT, B, W><<<dim3(pd.nb, nk), 32 * W, smem, st>>>(pd, k0, theta, eps2, ctx().partial, npad);
-      NCG_LAUNCHED();
-      return NCGPU_OK;
-}
-
-template <int MODE, int SOFT>
-int pair_launch_b(int B, const PairData &pd, int k0, int nk, double theta, double eps2, long npad, cudaStream_t st)
-{
-      if (B == 4) return pair_launch<MODE, SOFT, 4, 4>(pd, k0, nk, theta, eps2, npad, st);
-      if (B == 2) return pair_launch<MODE, SOFT, 2, 4>(pd, k0, nk, theta, eps2, npad, st);
-      return pair_launch<MODE, SOFT, 1, 2>(pd, k0, nk, theta, eps2, npad, st);
-}
-
-constexpr size_t PAIR_ROWS_MAX = (size_t)1 << 27;  // doubles of partial rows at once (1 GB)
-
-// Every unordered pair of pd's bodies once, into partial rows of ctx().partial.
-int pair_sums(PairData pd, int MODE, int soft, double theta, double eps2, PairRun &run, cudaStream_t st)
-{
-      Ctx &c = ctx();
-      // Tiles a block: larger blocks write fewer partial rows, smaller ones give more
-      // and shorter units.  Whole mixed calls, equal radii, B = 1 / 2 / 4 (8 is slower
-      // everywhere): 204 / 213 / 331 us at 12,345 bodies, 316 / 308 / 398 at 20,011,
-      // 520 / 498 / 576 at 30,011, 1,730 / 1,669 / 1,657 at 65,536; FP64 276 / 297 / 352
-      // at 12,345, 972 / 958 / 966 at 30,011, 3,935 / 3,882 / 3,808 at 65,536.
-      const int B = pd.ntiles <= 128 ? 1 : pd.ntiles < 384 ? 2 : 4;
-      pd.nb = (pd.ntiles + B - 1) / B;
-      const long npad = (long)pd.nb * B * PT;
-      const int nk = pair_offsets(pd.nb);
-      const size_t row = 6 * (size_t)npad;  // both sides of an offset
-      int per = (int)std::max<size_t>(1, std::min<size_t>(nk, PAIR_ROWS_MAX / row));
-      per = (nk + (nk + per - 1) / per - 1) / ((nk + per - 1) / per);  // equal shares
-      const bool whole = per >= nk;
-      NCG_TRY(ensure_partial(row * per + (whole ? 0 : 3 * (size_t)npad)));
-      double *base = whole ? nullptr : c.partial + row * per;
-      for (int k0 = 0; k0 < nk; k0 += per) {
-            const int m = std::min(per, nk - k0);
-            int s;
-            if (MODE == 0)
-                  s = soft == 0   ? pair_launch_b<0, 0>(B, pd, k0, m, theta, eps2, npad, st)
-                      : soft == 1 ? pair_launch_b<0, 1>(B, pd, k0, m, theta, eps2, npad, st)
-                                  : pair_launch_b<0, 2>(B, pd, k0, m, theta, eps2, npad, st);
-            else
-                  s = soft == 0   ? pair_launch_b<1, 0>(B, pd, k0, m, theta, eps2, npad, st)
-                      : soft == 1 ? pair_launch_b<1, 1>(B, pd, k0, m, theta, eps2, npad, st)
-                                  : pair_launch_b<1, 2>(B, pd, k0, m, theta, eps2, npad, st);
-            NCG_TRY(s);
-            if (k0 + m < nk) {
-                  k_pair_accum<<<(pd.n + 31) / 32, 256, 0, st>>>(c.partial, npad, pd.nb, k0, m, B * PT, pd.n, k0 == 0,
-                                                                 base);
-                  NCG_LAUNCHED();
-            }
-            run = PairRun{pd.nb, B * PT, k0, m, npad, base};
-      }
       return NCGPU_OK;
 }
 
@@ -1093,15 +1006,16 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       const double theta = P.par_near_theta > 0. ? P.par_near_theta : 0.15;
       if (nparts == 1) {
             // the whole field: every pair once
-            PairData pd{s64, c.srcR, (const float *)c.src32, c.srcR32, c.tilebox, n, ntiles, 0};
-            NCG_CK(cudaEventRecord(c.kev0, st));
+            PairData pd{s64, c.srcR, (const float *)c.src32, c.srcR32, c.tilebox, n, ntiles, 0, nullptr, nullptr};
+            const PairPlan pl = pair_plan<0>(n);
+            NCG_TRY(ensure_partial(pl.doubles));
             PairRun pr;
-            NCG_TRY(pair_sums(pd, mode == NCGPU_GRAVITY_MIXED ? 0 : 1, soft_kind, theta, eps2, pr, st));
+            NCG_CK(cudaEventRecord(c.kev0, st));
+            NCG_TRY(pair_sums<0>(pd, pl, mode == NCGPU_GRAVITY_MIXED ? 0 : 1, soft_kind, theta, eps2, c.partial, pr, st));
             NCG_CK(cudaEventRecord(c.kev1, st));
             c.kev_valid = 1;
-            k_pair_final<<<(n + 31) / 32, 256, 0, st>>>(c.partial, pr.npad, pr.nb, pr.k0, pr.nk, pr.bsize, pr.base, s64,
-                                                        c.vals, n, cmh[0], cmh[1], cmh[2], mu, G, central, j2, ax, ay,
-                                                        az, c.cmterm);
+            k_pair_final<<<(n + 31) / 32, 256, 0, st>>>(pr, s64, c.vals, n, cmh[0], cmh[1], cmh[2], mu, G, central, j2,
+                                                        ax, ay, az, c.cmterm);
             NCG_LAUNCHED();
             return finish_cm(central, n, d_cm_acc, st);
       }
