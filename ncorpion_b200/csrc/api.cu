@@ -217,12 +217,11 @@ int kick_state()
       c.com_reduced = 0;
       const int nslots = c.largest_id + 1;
       const bool mesh_grav = c.P.par_mesh_bool && !c.force_naive && !c.P.par_mesh_brute_gravity;
-      // the central mass's state on the host: for the brute-force gravity's
-      // arguments and the J2 term; mesh gravity, and the exact brute force on a
-      // few thousand bodies, read it from device memory
-      const bool exact_small = c.P.par_gravity_mode == NCGPU_GRAVITY_EXACT && nslots <= EXACT_SMALL_N;
+      // the central mass's state on the host: for the tiled gravity's arguments and
+      // the J2 term; mesh gravity and the exact brute force read it from device memory
+      const bool exact = c.P.par_gravity_mode == NCGPU_GRAVITY_EXACT;
       double cm9[9] = {0.};
-      if ((!mesh_grav && !exact_small) || c.P.par_J2_bool) NCG_TRY(state_cm_host(cm9));
+      if ((!mesh_grav && !exact) || c.P.par_J2_bool) NCG_TRY(state_cm_host(cm9));
       const J2Arg j2 = j2_arg(c.P, cm9[6], c.j2);
       if (mesh_grav)
             NCG_TRY(mesh_gravity_state(j2));

@@ -694,8 +694,8 @@ int sync_scalars_h(int *h);  // device scalars into c.* and h[S_COUNT], error wo
 // Morton-ordered target blocks in the tiled modes); every other row gets -0.0
 // (+0.0 for empty slots from part 0), so that the sum over the parts is the
 // full field, bit for bit.  CM_acc is the full one in every part.
-// cm_dev (may be null): the central body in device memory; the exact mode up to
-// EXACT_SMALL_N body slots then runs without reading anything back.
+// cm_dev (may be null): the central body in device memory, which the exact mode
+// then reads there.  An unknown mode is the exact one up to EXACT_SMALL_N slots.
 constexpr int EXACT_SMALL_N = 8192;
 int gravity_eval(const BodyView &bv, int largest_id, const double *cm_host8, const J2Arg &j2, double *d_acc,
                  long acc_stride_block, double *d_cm_acc, int mode, cudaStream_t st, int part = 0, int nparts = 1,
@@ -733,14 +733,13 @@ int compact_existing(const int *ex, int largest_id, int *n_host, cudaStream_t st
 // ctx().n_dev[0].
 int compact_existing_dev(const int *ex, int largest_id, cudaStream_t st);
 
-// Compaction of flagged slots with caller-provided scratch (no library context).
-int compact_flags_into(const int *flags, int n_slots, int *blockcnt, int *n_dev, int *out_idx, int *n_host,
-                       cudaStream_t st);
+// Compaction of flagged slots with caller-provided scratch (no library context):
+// blockcnt ceil(n_slots/1024) + 1 ints, n_dev the count.
+int compact_flags_dev(const int *flags, int n_slots, int *blockcnt, int *n_dev, int *out_idx, cudaStream_t st);
 
 // The exact gravity on caller-provided scratch (no library context).
 int gravity_exact_into(const BodyView &bv, int largest_id, const double *cmh, double G, double sp, int central,
-                       const J2Arg &j2, int *cidx, double *src, double *srcR, double *cterm, int *blockcnt,
-                       int *n_dev, unsigned *err, double *ax, double *ay, double *az, double *d_cm_acc,
-                       cudaStream_t st);
+                       const J2Arg &j2, int *cidx, double *src, double *srcR, int *blockcnt, int *n_dev, double *ax,
+                       double *ay, double *az, double *d_cm_acc, cudaStream_t st);
 
 }  // namespace ncg

@@ -4,11 +4,11 @@
 //
 // Three arithmetic modes share the same driver:
 //
-// EXACT  one thread per target body, sources streamed in ascending slot order
-//        through shared memory with 1-D bulk copies (cp.async.bulk) on a
-//        double-buffered mbarrier pipeline.  Every operation is the reference's,
-//        in the reference's order and rounding (explicit _rn intrinsics, no FMA
-//        contraction), so accelerations are bit-identical to vector_field:
+// EXACT  pair terms computed by whole CTAs, a few targets each, and added in
+//        ascending slot order by a warp of their own.  Every operation is the
+//        reference's, in the reference's order and rounding (explicit _rn
+//        intrinsics, no FMA contraction), so accelerations are bit-identical to
+//        vector_field:
 //          a_i = central_i ; for j ascending, j != i:
 //          a_i += ((G*m_j) * (x_j - x_i)) / (D*D*D),   (the three quotients by
 //          D^3 correctly rounded from one correctly rounded reciprocal)
@@ -16,13 +16,14 @@
 //        (the reference subtracts ((G*m_j)*(x_i-x_j))/D^3 for j < i, which is
 //        the same IEEE value).  CM_acc is summed sequentially in slot order.
 // FP64   bodies ordered along a Morton curve, 128-body tiles, one FP64 rsqrt per
-//        pair; (target block, source chunk) work units, partial sums reduced
-//        in a fixed order (deterministic).
-// MIXED  same tiling; pair terms in FP32 on coordinates relative to the source
-//        tile's centre (one MUFU rsqrt per pair), FP32 partial sums over runs of
-//        64 sources accumulated in FP64; tile pairs
-//        whose bounding boxes are closer than near_theta x the larger box
-//        diagonal (always including the target's own tile) are summed in FP64.
+//        pair.  The whole field takes every unordered pair once (pairsym.cuh); a
+//        part of it (one of several GPUs) sums its target blocks by themselves,
+//        (target block, source chunk) work units.  Partial sums reduced in a
+//        fixed order (deterministic).
+// MIXED  same tiling; pair terms in FP32 on coordinates relative to a tile's
+//        centre (one MUFU rsqrt per pair), short FP32 sums accumulated in FP64;
+//        tile pairs whose bounding boxes are closer than near_theta x the larger
+//        box diagonal (always including the target's own tile) are summed in FP64.
 //        The central-mass term and G are applied in FP64.
 #include <algorithm>
 #include "common.cuh"
@@ -34,274 +35,329 @@ namespace ncg {
 namespace {
 
 constexpr int T = 128;        // bodies per tile
-constexpr int EXB = 128;      // threads per block, exact kernel
 constexpr int MXB = 64;       // threads per block, tiled kernels (2 targets each)
 
 // ---------------------------------------------------------------- packing --
 
-__global__ void k_pack_exact(BodyView bv, const int *__restrict__ cidx, int n, int npad, double G,
-                             D4 *__restrict__ src, double *__restrict__ srcR, const int *__restrict__ n_dev = nullptr)
+__global__ void k_pack_exact(BodyView bv, const int *__restrict__ cidx, const int *__restrict__ n_dev, double G,
+                             D4 *__restrict__ src, double *__restrict__ srcR)
 {
       int p = blockIdx.x * blockDim.x + threadIdx.x;
-      if (n_dev) n = *n_dev;  // the count on the device (npad bounds it)
-      if (p >= npad) return;
-      if (p < n) {
-            long s = (long)cidx[p] * bv.stride;
-            D4 d;
-            d.x = bv.x[s];
-            d.y = bv.y[s];
-            d.z = bv.z[s];
-            d.w = __dmul_rn(G, bv.m[s]);  // G*mp, evaluated first in G*mp*DX/D3
-            src[p] = d;
-            srcR[p] = bv.R[s];
-      } else {
-            src[p] = D4{0., 0., 0., 0.};
-            srcR[p] = 0.;
-      }
+      if (p >= *n_dev) return;  // (the grid covers every slot)
+      long s = (long)cidx[p] * bv.stride;
+      D4 d;
+      d.x = bv.x[s];
+      d.y = bv.y[s];
+      d.z = bv.z[s];
+      d.w = __dmul_rn(G, bv.m[s]);  // G*mp, evaluated first in G*mp*DX/D3
+      src[p] = d;
+      srcR[p] = bv.R[s];
 }
 
 // ------------------------------------------------------------ exact kernel --
 
-template <bool SOFT>
-__global__ void __launch_bounds__(EXB) k_grav_exact(const D4 *__restrict__ src, const double *__restrict__ srcR,
-                                                    const int *__restrict__ cidx, int n, int ntiles,
-                                                    double cmx, double cmy, double cmz, double mu, double sp,
-                                                    int central, J2Arg j2, BodyView bv, int p_lo, int p_hi,
-                                                    double *__restrict__ ax, double *__restrict__ ay,
-                                                    double *__restrict__ az, double *__restrict__ cterm,
-                                                    unsigned *__restrict__ err)
+// The central body: in device memory, or by value.
+struct CmArg {
+      const double *dev;
+      double x, y, z, m;
+};
+
+// The central mass's acceleration of a body (with J2, src/physics.c:123-160) and
+// CM_acc's terms from it: c[0..2] the central ones, c[3..5] J2's share.
+__device__ __forceinline__ void central_terms(const D4 &me, double cmx, double cmy, double cmz, double mu,
+                                              const J2Arg &j2, double mk, double (&a)[3], double (&c)[6])
 {
-      __shared__ D4 tile[2][T];
-      __shared__ alignas(16) double tR[2][T];
-      __shared__ uint64_t bar[2];
-
-      const int tid = threadIdx.x;
-      const int p = blockIdx.x * EXB + tid;
-      const bool active = p < n;
-      const D4 me = src[active ? p : 0];
-      const double Ri = srcR[active ? p : 0];
-
-      double a_x = 0., a_y = 0., a_z = 0.;
-      if (central && active) {
-            // src/physics.c:123-139: DX = X - XX, rk = sqrt(DX*DX + DY*DY + DZ*DZ)
-            double DX = __dsub_rn(me.x, cmx), DY = __dsub_rn(me.y, cmy), DZ = __dsub_rn(me.z, cmz);
-            double rk = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(DX, DX), __dmul_rn(DY, DY)), __dmul_rn(DZ, DZ)));
-            double r3 = __dmul_rn(__dmul_rn(rk, rk), rk);
-            const double y3 = __drcp_rn(r3);  // the six quotients by r3 share RN(1/r3)
-            a_x = div_by_recip(__dmul_rn(-mu, DX), r3, y3);
-            a_y = div_by_recip(__dmul_rn(-mu, DY), r3, y3);
-            a_z = div_by_recip(__dmul_rn(-mu, DZ), r3, y3);
-            // CM_acc terms: G*mk*DX/r3, then (with J2) the J2 share, so that
-            // cterm's sequential sum adds them in the reference's order
-            const int f = j2.on ? 2 : 1;
-            const size_t nf = (size_t)f * n;
-            cterm[f * p] = div_by_recip(__dmul_rn(me.w, DX), r3, y3);
-            cterm[nf + f * p] = div_by_recip(__dmul_rn(me.w, DY), r3, y3);
-            cterm[2 * nf + f * p] = div_by_recip(__dmul_rn(me.w, DZ), r3, y3);
-            if (j2.on) {  // src/physics.c:149-160
-                  double cj[3];
-                  d_j2(j2, mu, DX, DY, DZ, rk, r3, bv.m[(long)cidx[p] * bv.stride], a_x, a_y, a_z, cj);
-                  cterm[2 * p + 1] = cj[0];
-                  cterm[nf + 2 * p + 1] = cj[1];
-                  cterm[2 * nf + 2 * p + 1] = cj[2];
-            }
-      }
-      // targets of this part: [p_lo, p_hi) of the compacted order; the others
-      // get -0.0, the identity of the sum that combines the parts
-      const bool own = active && p >= p_lo && p < p_hi;
-      if (!__syncthreads_or(own)) {
-            if (active) {
-                  const int slot = cidx[p];
-                  ax[slot] = -0.0;
-                  ay[slot] = -0.0;
-                  az[slot] = -0.0;
-            }
-            return;
-      }
-
-      if (tid == 0) {
-            mbar_init(&bar[0], 1);
-            mbar_init(&bar[1], 1);
-            mbar_fence_init();
-      }
-      __syncthreads();
-      const unsigned bytes = T * sizeof(D4) + (SOFT ? T * sizeof(double) : 0);
-      if (tid == 0 && ntiles > 0) {
-            mbar_arrive_expect(&bar[0], bytes);
-            bulk_g2s(tile[0], src, T * sizeof(D4), &bar[0]);
-            if (SOFT) bulk_g2s(tR[0], srcR, T * sizeof(double), &bar[0]);
-      }
-      for (int t = 0; t < ntiles; ++t) {
-            const int b = t & 1;
-            if (tid == 0 && t + 1 < ntiles) {
-                  fence_proxy_async_smem();
-                  mbar_arrive_expect(&bar[b ^ 1], bytes);
-                  bulk_g2s(tile[b ^ 1], src + (size_t)(t + 1) * T, T * sizeof(D4), &bar[b ^ 1]);
-                  if (SOFT) bulk_g2s(tR[b ^ 1], srcR + (size_t)(t + 1) * T, T * sizeof(double), &bar[b ^ 1]);
-            }
-            bool ok = mbar_wait_bounded(&bar[b], (t >> 1) & 1);
-            if (__syncthreads_or(!ok)) {
-                  if (tid == 0) {
-                        atomicOr(err, ERR_TIMEOUT);
-                        // let the copies already issued land before leaving
-                        mbar_wait_bounded(&bar[b], (t >> 1) & 1);
-                        if (t + 1 < ntiles) mbar_wait_bounded(&bar[b ^ 1], ((t + 1) >> 1) & 1);
-                  }
-                  return;
-            }
-            if (own) {
-                  const int jbase = t * T;
-                  const int cnt = min(T, n - jbase);
-                  for (int jj = 0; jj < cnt; ++jj) {
-                        if (jbase + jj == p) continue;
-                        const D4 s = tile[b][jj];
-                        double dx = __dsub_rn(s.x, me.x);
-                        double dy = __dsub_rn(s.y, me.y);
-                        double dz = __dsub_rn(s.z, me.z);
-                        double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                        if (SOFT) {
-                              double sf = __dmul_rn(sp, __dadd_rn(Ri, tR[b][jj]));
-                              r2 = __dadd_rn(r2, __dmul_rn(sf, sf));
-                        }
-                        double D = __dsqrt_rn(r2);
-                        double D3 = __dmul_rn(__dmul_rn(D, D), D);
-                        const double y = __drcp_rn(D3);  // the three quotients by D3 share RN(1/D3)
-                        a_x = __dadd_rn(a_x, div_by_recip(__dmul_rn(s.w, dx), D3, y));
-                        a_y = __dadd_rn(a_y, div_by_recip(__dmul_rn(s.w, dy), D3, y));
-                        a_z = __dadd_rn(a_z, div_by_recip(__dmul_rn(s.w, dz), D3, y));
-                  }
-            }
-            __syncthreads();
-      }
-      if (active) {
-            int slot = cidx[p];
-            ax[slot] = own ? a_x : -0.0;
-            ay[slot] = own ? a_y : -0.0;
-            az[slot] = own ? a_z : -0.0;
-      }
+      // src/physics.c:123-139: DX = X - XX, rk = sqrt(DX*DX + DY*DY + DZ*DZ)
+      const double DX = __dsub_rn(me.x, cmx), DY = __dsub_rn(me.y, cmy), DZ = __dsub_rn(me.z, cmz);
+      const double rk = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(DX, DX), __dmul_rn(DY, DY)), __dmul_rn(DZ, DZ)));
+      const double r3 = __dmul_rn(__dmul_rn(rk, rk), rk);
+      const double y3 = __drcp_rn(r3);  // the six quotients by r3 share RN(1/r3)
+      a[0] = div_by_recip(__dmul_rn(-mu, DX), r3, y3);
+      a[1] = div_by_recip(__dmul_rn(-mu, DY), r3, y3);
+      a[2] = div_by_recip(__dmul_rn(-mu, DZ), r3, y3);
+      c[0] = div_by_recip(__dmul_rn(me.w, DX), r3, y3);
+      c[1] = div_by_recip(__dmul_rn(me.w, DY), r3, y3);
+      c[2] = div_by_recip(__dmul_rn(me.w, DZ), r3, y3);
+      c[3] = c[4] = c[5] = 0.;
+      if (j2.on) d_j2(j2, mu, DX, DY, DZ, rk, r3, mk, a[0], a[1], a[2], c + 3);  // src/physics.c:149-160
 }
 
-// k_grav_exact for few bodies.  One thread a target leaves most of the SMs
-// idle below ~19,000 bodies (128 targets a CTA), so here a CTA holds XT
-// targets and computes their pair terms with all its threads, XS sources a
-// round, into shared memory; then one thread per target and component adds the
-// round's terms in source order.  The terms (k_grav_exact's operation
-// sequence) and the order of the additions are k_grav_exact's, so the sums
-// are bit-identical.
-constexpr int XT = 8;     // targets a CTA
-constexpr int XS = 64;    // sources a round
-constexpr int XTH = 128;  // threads a CTA: XTH / XT source lanes a target
-
-template <bool SOFT>
-__global__ void __launch_bounds__(XTH) k_grav_exact_small(const D4 *__restrict__ src, const double *__restrict__ srcR,
-                                                          const int *__restrict__ cidx, const int *__restrict__ n_dev,
-                                                          const double *__restrict__ cmd, double G, double sp,
-                                                          int central, J2Arg j2, BodyView bv, int part, int nparts,
-                                                          double *__restrict__ ax, double *__restrict__ ay,
-                                                          double *__restrict__ az, double *__restrict__ cterm)
+// div_by_recip for x != 0.
+__device__ __forceinline__ double div_by_recip_nz(double x, double b, double y)
 {
-      // the count and the central body from device memory (the grid covers every
-      // slot; the part's slice as the host would cut it)
-      const int n = *n_dev;
-      const int p_lo = (int)((long)n * part / nparts), p_hi = (int)((long)n * (part + 1) / nparts);
-      const double cmx = cmd[0], cmy = cmd[1], cmz = cmd[2];
-      const double mu = G * cmd[6];
-      __shared__ double tm[3][XS][XT + 1];  // the round's terms (padded rows)
-      __shared__ D4 ss[XS];
-      __shared__ double sR[XS];
-      __shared__ double a0[3][XT];           // the targets' starting sums (central terms)
-      const int tid = threadIdx.x;
-      const int pbase = blockIdx.x * XT;
-      if (tid < XT) {
-            const int p = pbase + tid;
-            double a[3] = {0., 0., 0.};
-            if (central && p < n) {  // as k_grav_exact (src/physics.c:123-160)
-                  const D4 me = src[p];
-                  double DX = __dsub_rn(me.x, cmx), DY = __dsub_rn(me.y, cmy), DZ = __dsub_rn(me.z, cmz);
-                  double rk = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(DX, DX), __dmul_rn(DY, DY)), __dmul_rn(DZ, DZ)));
-                  double r3 = __dmul_rn(__dmul_rn(rk, rk), rk);
-                  const double y3 = __drcp_rn(r3);
-                  a[0] = div_by_recip(__dmul_rn(-mu, DX), r3, y3);
-                  a[1] = div_by_recip(__dmul_rn(-mu, DY), r3, y3);
-                  a[2] = div_by_recip(__dmul_rn(-mu, DZ), r3, y3);
-                  const int f = j2.on ? 2 : 1;
-                  const size_t nf = (size_t)f * n;
-                  cterm[f * p] = div_by_recip(__dmul_rn(me.w, DX), r3, y3);
-                  cterm[nf + f * p] = div_by_recip(__dmul_rn(me.w, DY), r3, y3);
-                  cterm[2 * nf + f * p] = div_by_recip(__dmul_rn(me.w, DZ), r3, y3);
-                  if (j2.on) {
-                        double cj[3];
-                        d_j2(j2, mu, DX, DY, DZ, rk, r3, bv.m[(long)cidx[p] * bv.stride], a[0], a[1], a[2], cj);
-                        cterm[2 * p + 1] = cj[0];
-                        cterm[nf + 2 * p + 1] = cj[1];
-                        cterm[2 * nf + 2 * p + 1] = cj[2];
+      double q = __dmul_rn(x, y);
+      double r = __fma_rn(-q, b, x);
+      q = __fma_rn(r, y, q);
+      r = __fma_rn(-q, b, x);
+      return __fma_rn(r, y, q);
+}
+
+// Whether x may be a zero: its high word is (on the integer pipe; true as well for
+// the smallest subnormals, which either division handles).
+__device__ __forceinline__ bool maybe_zero(double x)
+{
+      return (__double2hiint(x) & 0x7fffffff) == 0;
+}
+
+// Named barriers: `threads` threads in all arrive at or wait on barrier id.
+__device__ __forceinline__ void bar_sync(int id, int threads)
+{
+      asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads)
+{
+      asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// The exact field of XT targets a CTA.  What has an order is the additions: a
+// target's terms in ascending source order, 8 cycles each.  So XP / 32 warps compute
+// the pair terms, XS sources a round, into one of two buffers in shared memory, and
+// one more warp adds the round before: a lane per target and component, one
+// dependent addition a source.  Block 0 (with a central mass) makes CM_acc's three
+// sequential sums the same way, its warps computing the bodies' terms.
+// Bound by the additions' latency below ~2,000 bodies (and by the FP64 pipe they
+// share with the terms: about 1,100 cycles a round with one CTA an SM), by the FP64
+// pipe and issue above (49 FP64 instructions a pair of 102: pipe and issue slots 60 %
+// busy).  One thread a target, computing and adding its own terms, had 128 targets a
+// CTA: 4.44 ms at 20,011 bodies (157 CTAs, one an SM; now 1.85) and 20.9 ms at 65,536
+// (19.2); computing and adding a round in turn 35 us at 1,000 (16.4), 65 at 2,000
+// (34.8) and 412 at 8,192 (334), with CM_acc's sums in a kernel of their own behind.
+constexpr int XT = 8;            // targets a CTA
+constexpr int XS = 64;           // sources a round
+constexpr int XROW = XS * XT + 8;  // a component's terms of a round (the pad keeps the adders off each other's banks)
+constexpr int XCM = 256;         // bodies a round of block 0
+constexpr int XV = 8;            // terms an adding lane loads ahead
+
+template <bool SOFT, int XP, int OCC>
+__global__ void __launch_bounds__(XP + 32, OCC) k_grav_exact(const D4 *__restrict__ src, const double *__restrict__ srcR,
+                                                       const int *__restrict__ cidx, const int *__restrict__ n_dev,
+                                                       CmArg cm, double G, double sp, int central, J2Arg j2,
+                                                       BodyView bv, int part, int nparts,
+                                                       double *__restrict__ ax, double *__restrict__ ay,
+                                                       double *__restrict__ az, double *__restrict__ cm_acc)
+{
+      constexpr int FULL = 1, EMPTY = 3;  // barriers FULL + buffer, EMPTY + buffer
+      constexpr int XTH = XP + 32;        // the threads that compute and the adding warp
+      constexpr int SL = XP / XT, NS = XS / SL;  // source lanes a target, sources a thread
+      __shared__ double tm[2][3 * XROW];
+      const int tid = threadIdx.x, n = *n_dev;
+      const double cmx = cm.dev ? cm.dev[0] : cm.x, cmy = cm.dev ? cm.dev[1] : cm.y, cmz = cm.dev ? cm.dev[2] : cm.z;
+      const double mu = G * (cm.dev ? cm.dev[6] : cm.m);
+      const bool adder = tid >= XP;
+      const int lane = tid & 31;
+      if (central && blockIdx.x == 0) {
+            const int f = j2.on ? 2 : 1, rounds = (n + XCM - 1) / XCM;
+            double acc = 0.;
+            for (int k = 0; k < rounds; k++) {
+                  double *t = tm[k & 1];
+                  if (!adder) {
+                        const int p = k * XCM + tid;
+                        double a[3], c[6] = {0., 0., 0., 0., 0., 0.};
+                        if (tid < XCM && p < n)
+                              central_terms(src[p], cmx, cmy, cmz, mu, j2,
+                                            j2.on ? bv.m[(long)cidx[p] * bv.stride] : 0., a, c);
+                        if (k >= 2) bar_sync(EMPTY + (k & 1), XTH);
+                        for (int d = 0; d < 3 && tid < XCM; d++) {
+                              t[d * f * XCM + f * tid] = c[d];
+                              if (j2.on) t[d * f * XCM + f * tid + 1] = c[3 + d];
+                        }
+                        bar_arrive(FULL + (k & 1), XTH);
+                  } else {
+                        bar_sync(FULL + (k & 1), XTH);
+                        if (lane < 3) {
+                              const int m = f * min(XCM, n - k * XCM);
+                              const volatile double *u = t + lane * f * XCM;
+                              double v[XV], w[XV];
+#pragma unroll
+                              for (int e = 0; e < XV; e++) v[e] = u[e];
+                              int q = 0;
+                              for (; q + XV <= m; q += XV) {
+#pragma unroll
+                                    for (int e = 0; e < XV; e++) w[e] = u[min(q + XV, f * XCM - XV) + e];
+#pragma unroll
+                                    for (int e = 0; e < XV; e++) {
+                                          acc = __dadd_rn(acc, v[e]);
+                                          v[e] = w[e];
+                                    }
+                              }
+                              for (; q < m; q++) acc = __dadd_rn(acc, u[q]);
+                        }
+                        __syncwarp();
+                        if (k + 2 < rounds) bar_arrive(EMPTY + (k & 1), XTH);
                   }
             }
-            for (int c = 0; c < 3; c++) a0[c][tid] = a[c];
+            if (adder && lane < 3) cm_acc[lane] = acc;
+            return;
       }
-      // the part's targets; a CTA without any writes -0.0 (the identity of the
-      // sum that combines the parts) and leaves
-      const bool any_own = pbase < n && pbase + XT > p_lo && pbase < p_hi;
-      if (!any_own) {
-            __syncthreads();
+      const int pbase = (blockIdx.x - (central ? 1 : 0)) * XT;
+      if (pbase >= n) return;
+      // the part's slice of the existing bodies; the others get -0.0, the identity
+      // of the sum that combines the parts
+      const int p_lo = (int)((long)n * part / nparts), p_hi = (int)((long)n * (part + 1) / nparts);
+      if (pbase + XT <= p_lo || pbase >= p_hi) {
             if (tid < XT && pbase + tid < n) {
                   const int slot = cidx[pbase + tid];
                   ax[slot] = -0.0; ay[slot] = -0.0; az[slot] = -0.0;
             }
             return;
       }
-      // this thread's target for the terms, and (threads < 3 XT) its sum
-      const int tt = tid % XT, lane = tid / XT;
-      const int pt = pbase + tt;
-      const D4 me = src[pt < n ? pt : 0];
-      const double Ri = SOFT ? srcR[pt < n ? pt : 0] : 0.;
-      const bool summer = tid < 3 * XT;
-      const int sc = tid / XT, st = tid % XT, ps = pbase + st;
-      __syncthreads();
-      double acc = summer ? a0[sc][st] : 0.;
-      for (int j0 = 0; j0 < n; j0 += XS) {
-            if (tid < XS && j0 + tid < n) {
-                  ss[tid] = src[j0 + tid];
-                  if (SOFT) sR[tid] = srcR[j0 + tid];
-            }
-            __syncthreads();
-            for (int j = lane; j < XS; j += XTH / XT) {
-                  const int q = j0 + j;
-                  double tx = 0., ty = 0., tz = 0.;
-                  if (q < n && q != pt && pt < n) {
-                        const D4 sj = ss[j];
-                        double dx = __dsub_rn(sj.x, me.x);
-                        double dy = __dsub_rn(sj.y, me.y);
-                        double dz = __dsub_rn(sj.z, me.z);
+      const int rounds = (n + XS - 1) / XS;
+      if (!adder) {
+            const int tt = tid % XT, sl = tid / XT;  // target; sources sl, sl + XP / XT of a round
+            const int pt = pbase + tt;
+            const D4 me = src[pt < n ? pt : 0];
+            const double Ri = SOFT ? srcR[pt < n ? pt : 0] : 0.;
+            const int kself = pbase / XS;  // the round of the targets themselves
+            D4 s[NS];
+            double sR[NS];
+            auto fetch = [&](int k) {
+#pragma unroll
+                  for (int u = 0; u < NS; u++) {
+                        const int j = min(k * XS + sl + SL * u, n - 1);
+                        s[u] = src[j];
+                        sR[u] = SOFT ? srcR[j] : 0.;
+                  }
+            };
+            if (NS == 1) fetch(0);
+            for (int k = 0; k < rounds; k++) {
+                  double t[NS][3];
+                  if (NS > 1) fetch(k);
+#pragma unroll
+                  for (int u = 0; u < NS; u++) {
+                        const double dx = __dsub_rn(s[u].x, me.x);
+                        const double dy = __dsub_rn(s[u].y, me.y);
+                        const double dz = __dsub_rn(s[u].z, me.z);
                         double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
                         if (SOFT) {
-                              double sf = __dmul_rn(sp, __dadd_rn(Ri, sR[j]));
+                              const double sf = __dmul_rn(sp, __dadd_rn(Ri, sR[u]));
                               r2 = __dadd_rn(r2, __dmul_rn(sf, sf));
                         }
-                        double D = __dsqrt_rn(r2);
-                        double D3 = __dmul_rn(__dmul_rn(D, D), D);
-                        const double y = __drcp_rn(D3);
-                        tx = div_by_recip(__dmul_rn(sj.w, dx), D3, y);
-                        ty = div_by_recip(__dmul_rn(sj.w, dy), D3, y);
-                        tz = div_by_recip(__dmul_rn(sj.w, dz), D3, y);
+                        const double D = __dsqrt_rn(r2);
+                        const double D3 = __dmul_rn(__dmul_rn(D, D), D);
+                        const double y = __drcp_rn(D3);  // the three quotients by D3 share RN(1/D3)
+                        const double gx = __dmul_rn(s[u].w, dx), gy = __dmul_rn(s[u].w, dy), gz = __dmul_rn(s[u].w, dz);
+                        if (maybe_zero(gx) || maybe_zero(gy) || maybe_zero(gz)) {
+                              t[u][0] = div_by_recip(gx, D3, y);
+                              t[u][1] = div_by_recip(gy, D3, y);
+                              t[u][2] = div_by_recip(gz, D3, y);
+                        } else {
+                              t[u][0] = div_by_recip_nz(gx, D3, y);
+                              t[u][1] = div_by_recip_nz(gy, D3, y);
+                              t[u][2] = div_by_recip_nz(gz, D3, y);
+                        }
                   }
-                  tm[0][j][tt] = tx;
-                  tm[1][j][tt] = ty;
-                  tm[2][j][tt] = tz;
+                  if (k == kself || k == rounds - 1) {  // -0.0 leaves every sum as it is
+#pragma unroll
+                        for (int u = 0; u < NS; u++) {
+                              const int j = k * XS + sl + SL * u;
+                              if (j >= n || j == pt) t[u][0] = t[u][1] = t[u][2] = -0.0;
+                        }
+                  }
+                  if (NS == 1 && k + 1 < rounds) fetch(k + 1);  // (few CTAs an SM: the load's latency shows)
+                  const int b = k & 1;
+                  if (k >= 2) bar_sync(EMPTY + b, XTH);
+#pragma unroll
+                  for (int u = 0; u < NS; u++)
+#pragma unroll
+                        for (int d = 0; d < 3; d++) tm[b][d * XROW + (sl + SL * u) * XT + tt] = t[u][d];
+                  bar_arrive(FULL + b, XTH);
             }
-            __syncthreads();
-            if (summer && ps < n) {
-                  const int je = min(XS, n - j0);
-                  for (int j = 0; j < je; ++j)
-                        if (j0 + j != ps) acc = __dadd_rn(acc, tm[sc][j][st]);
-            }
-            __syncthreads();
+            return;
       }
-      if (summer && ps < n) {
-            const bool own = ps >= p_lo && ps < p_hi;
+      const int d = min(lane / XT, 2), ps = pbase + lane % XT;
+      const bool live = lane < 3 * XT && ps < n;
+      double acc = 0.;
+      if (central && live) {
+            double a[3], c[6];
+            central_terms(src[ps], cmx, cmy, cmz, mu, j2, j2.on ? bv.m[(long)cidx[ps] * bv.stride] : 0., a, c);
+            acc = d == 0 ? a[0] : d == 1 ? a[1] : a[2];
+      }
+      for (int k = 0; k < rounds; k++) {
+            const int b = k & 1;
+            bar_sync(FULL + b, XTH);
+            const volatile double *u = tm[b] + d * XROW + lane % XT;
+            double v[XV], w[XV];  // XV loads in flight while XV terms are added
+#pragma unroll
+            for (int e = 0; e < XV; e++) v[e] = u[e * XT];
+#pragma unroll
+            for (int q = 0; q < XS; q += XV) {
+                  if (q + XV < XS)
+#pragma unroll
+                        for (int e = 0; e < XV; e++) w[e] = u[(q + XV + e) * XT];
+#pragma unroll
+                  for (int e = 0; e < XV; e++) {
+                        acc = __dadd_rn(acc, v[e]);
+                        v[e] = w[e];
+                  }
+            }
+            if (k + 2 < rounds) bar_arrive(EMPTY + b, XTH);
+      }
+      if (live) {
             const int slot = cidx[ps];
-            double *out = sc == 0 ? ax : sc == 1 ? ay : az;
-            out[slot] = own ? acc : -0.0;
+            double *out = d == 0 ? ax : d == 1 ? ay : az;
+            out[slot] = ps >= p_lo && ps < p_hi ? acc : -0.0;
+      }
+}
+
+// Up to PREP_N slots in one CTA: the compaction of the existing ones, their packed
+// copies (k_pack_exact) and `fill` in the empty slots' rows, instead of five
+// launches of about 2 us each.
+constexpr int PREP_U = 8, PREP_N = 1024 * PREP_U;
+
+__global__ void __launch_bounds__(1024) k_prep_exact(BodyView bv, int nslots, double G, double fill,
+                                                     int *__restrict__ cidx, int *__restrict__ n_dev,
+                                                     D4 *__restrict__ src, double *__restrict__ srcR,
+                                                     double *__restrict__ ax, double *__restrict__ ay,
+                                                     double *__restrict__ az)
+{
+      __shared__ int cnt[PREP_U * 32];
+      const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+      bool in[PREP_U];
+      unsigned below[PREP_U];
+#pragma unroll
+      for (int u = 0; u < PREP_U; u++) {
+            const int i = u * 1024 + tid;
+            in[u] = i < nslots && bv.ex[i] != 0;
+            const unsigned m = __ballot_sync(0xffffffffu, in[u]);
+            below[u] = __popc(m & ((1u << lane) - 1u));
+            if (lane == 0) cnt[u * 32 + w] = __popc(m);
+            if (i < nslots && !in[u]) {
+                  ax[i] = fill;
+                  ay[i] = fill;
+                  az[i] = fill;
+            }
+      }
+      __syncthreads();
+      if (w == 0) {  // exclusive prefix of the 256 warp counts, eight a lane
+            int c[PREP_U], s = 0;
+#pragma unroll
+            for (int u = 0; u < PREP_U; u++) {
+                  c[u] = cnt[lane * PREP_U + u];
+                  s += c[u];
+            }
+            int incl = s;
+            for (int o = 1; o < 32; o <<= 1) {
+                  const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                  if (lane >= o) incl += v;
+            }
+            int run = incl - s;
+#pragma unroll
+            for (int u = 0; u < PREP_U; u++) {
+                  cnt[lane * PREP_U + u] = run;
+                  run += c[u];
+            }
+            if (lane == 31) *n_dev = incl;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < PREP_U; u++) {
+            const int i = u * 1024 + tid;
+            if (!in[u]) continue;
+            const int p = cnt[u * 32 + w] + (int)below[u];
+            const long s = (long)i * bv.stride;
+            cidx[p] = i;
+            src[p] = D4{bv.x[s], bv.y[s], bv.z[s], __dmul_rn(G, bv.m[s])};
+            srcR[p] = bv.R[s];
       }
 }
 
@@ -310,9 +366,8 @@ __global__ void __launch_bounds__(XTH) k_grav_exact_small(const D4 *__restrict__
 // without init), one CTA (one warp) per component, so the result matches the
 // reference bit for bit.  out may alias init.
 __global__ void __launch_bounds__(32) k_seq_sum3(const double *__restrict__ cterm, int n, const double *init,
-                                                 double *out, const int *__restrict__ n_dev = nullptr, int f = 1)
+                                                 double *out)
 {
-      if (n_dev) n = f * *n_dev;  // (f terms a body)
       __shared__ __align__(16) double stage[CHN];
       const int w = blockIdx.x;
       const double s = warp_chain_sum(cterm + (size_t)w * n, n, init ? init[w] : 0., stage);
@@ -852,6 +907,48 @@ int seq_sum3(const double *terms, int n, const double *init, double *out, cudaSt
 
 namespace {
 
+// The exact field of the existing bodies of slots 0 .. nslots - 1 into ax, ay, az
+// (`fill` in the empty slots' rows) and cm_acc, on the scratch it is given.  started
+// (may be null): recorded before the field kernel.
+int exact_field(const BodyView &bv, int nslots, const CmArg &cm, double G, double sp, int central, const J2Arg &j2,
+                int part, int nparts, double fill, int *cidx, D4 *src, double *srcR, int *blockcnt, int *n_dev,
+                double *ax, double *ay, double *az, double *cm_acc, cudaStream_t st, cudaEvent_t started)
+{
+      if (nslots == 0 || !central) {
+            k_set3<<<1, 1, 0, st>>>(cm_acc, 0., 0., 0.);
+            NCG_LAUNCHED();
+            if (nslots == 0) return NCGPU_OK;
+      }
+      if (nslots <= PREP_N) {
+            k_prep_exact<<<1, 1024, 0, st>>>(bv, nslots, G, fill, cidx, n_dev, src, srcR, ax, ay, az);
+            NCG_LAUNCHED();
+      } else {
+            k_fill3<<<(nslots + 255) / 256, 256, 0, st>>>(ax, ay, az, nslots, fill);
+            NCG_LAUNCHED();
+            NCG_TRY(compact_flags_dev(bv.ex, nslots, blockcnt, n_dev, cidx, st));
+            k_pack_exact<<<(nslots + 255) / 256, 256, 0, st>>>(bv, cidx, n_dev, G, src, srcR);
+            NCG_LAUNCHED();
+      }
+      if (started) NCG_CK(cudaEventRecord(started, st));
+      const int nb = (nslots + XT - 1) / XT + (central ? 1 : 0);
+#define NCG_EXACT(XP_, OCC_)                                                                                          \
+      do {                                                                                                           \
+            if (sp != 0.)                                                                                            \
+                  k_grav_exact<true, XP_, OCC_><<<nb, XP_ + 32, 0, st>>>(src, srcR, cidx, n_dev, cm, G, sp, central, \
+                                                                         j2, bv, part, nparts, ax, ay, az, cm_acc);  \
+            else                                                                                                     \
+                  k_grav_exact<false, XP_, OCC_><<<nb, XP_ + 32, 0, st>>>(src, srcR, cidx, n_dev, cm, G, sp, central,\
+                                                                          j2, bv, part, nparts, ax, ay, az, cm_acc); \
+      } while (0)
+      // (512 threads a CTA while there are fewer than two CTAs an SM: 16.4 against 20.5 us
+      // at 1,000 bodies, both 34.8 at 2,000, 113 against 102 at 4,001)
+      if (nslots <= 2048) NCG_EXACT(512, 2);
+      else NCG_EXACT(256, 4);
+#undef NCG_EXACT
+      NCG_LAUNCHED();
+      return NCGPU_OK;
+}
+
 // CM_acc of the tiled modes: the two-level sum of its terms, or zero.
 int finish_cm(int central, int n, double *d_cm_acc, cudaStream_t st)
 {
@@ -873,57 +970,27 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       if (nparts < 1 || part < 0 || part >= nparts) return NCGPU_E_ARG;
       const int nslots = largest_id + 1;
       double *ax = d_acc, *ay = d_acc + bs, *az = d_acc + 2 * bs;
+      // empty slots: +0.0 from part 0, -0.0 (the identity of the parts' sum) from the others
+      const double fill = part == 0 ? 0. : -0.;
+      const bool tiled = mode == NCGPU_GRAVITY_FP64 || mode == NCGPU_GRAVITY_MIXED;
+      const int central = P.par_central_mass_bool;
+      if (!tiled) {
+            // (nothing comes back to the host: the kernels read the count of existing
+            // bodies from device memory)
+            if (mode != NCGPU_GRAVITY_EXACT && nslots > EXACT_SMALL_N) return NCGPU_E_ARG;
+            NCG_TRY(exact_field(bv, nslots, CmArg{cm_dev, cmh[0], cmh[1], cmh[2], cmh[6]}, P.par_G, P.par_softening_parameter, central, j2, part, nparts, fill,
+                                c.cidx, (D4 *)c.src64, c.srcR, c.cnt, c.n_dev, ax, ay, az, d_cm_acc, st, c.kev0));
+            NCG_CK(cudaEventRecord(c.kev1, st));
+            c.kev_valid = 1;
+            return NCGPU_OK;
+      }
       if (nslots > 0) {
-            // empty slots: +0.0 from part 0, -0.0 (the identity of the parts' sum) from the others
-            k_fill3<<<(nslots + 255) / 256, 256, 0, st>>>(ax, ay, az, nslots, part == 0 ? 0. : -0.);
+            k_fill3<<<(nslots + 255) / 256, 256, 0, st>>>(ax, ay, az, nslots, fill);
             NCG_LAUNCHED();
       }
       int n = 0;
-      const bool tiled = mode == NCGPU_GRAVITY_FP64 || mode == NCGPU_GRAVITY_MIXED;
-      double rr[2] = {0., 0.};  // radius range of the existing bodies (tiled modes)
-      if (!tiled && nslots <= EXACT_SMALL_N) {
-            // few bodies, exact: the count stays on the device, the kernels read it
-            // (grids sized for every slot) and the central body from device memory
-            if (nslots == 0) {
-                  k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
-                  NCG_LAUNCHED();
-                  return NCGPU_OK;
-            }
-            NCG_TRY(compact_existing_dev(bv.ex, largest_id, st));
-            const double *cmd = cm_dev;
-            if (!cmd) {
-                  NCG_CK(cudaMemcpyAsync(c.red + 4064, cmh, 8 * sizeof(double), cudaMemcpyHostToDevice, st));
-                  cmd = c.red + 4064;
-            }
-            const int npad_max = (nslots + T - 1) / T * T;
-            D4 *src = (D4 *)c.src64;
-            k_pack_exact<<<(npad_max + 255) / 256, 256, 0, st>>>(bv, c.cidx, 0, npad_max, P.par_G, src, c.srcR,
-                                                                 c.n_dev);
-            NCG_LAUNCHED();
-            const double sp = P.par_softening_parameter;
-            const int central = P.par_central_mass_bool;
-            const int nbs = (nslots + XT - 1) / XT;
-            NCG_CK(cudaEventRecord(c.kev0, st));
-            if (sp != 0.)
-                  k_grav_exact_small<true><<<nbs, XTH, 0, st>>>(src, c.srcR, c.cidx, c.n_dev, cmd, P.par_G, sp, central,
-                                                               j2, bv, part, nparts, ax, ay, az, c.cmterm);
-            else
-                  k_grav_exact_small<false><<<nbs, XTH, 0, st>>>(src, c.srcR, c.cidx, c.n_dev, cmd, P.par_G, sp,
-                                                                central, j2, bv, part, nparts, ax, ay, az, c.cmterm);
-            NCG_LAUNCHED();
-            NCG_CK(cudaEventRecord(c.kev1, st));
-            c.kev_valid = 1;
-            if (central) {
-                  k_seq_sum3<<<3, 32, 0, st>>>(c.cmterm, 0, nullptr, d_cm_acc, c.n_dev, j2.on ? 2 : 1);
-            } else {
-                  k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
-            }
-            NCG_LAUNCHED();
-            return NCGPU_OK;
-      }
-      if (!tiled) {
-            NCG_TRY(compact_existing(bv.ex, largest_id, &n, st));
-      } else if (nslots > 0) {
+      double rr[2] = {0., 0.};  // radius range of the existing bodies
+      if (nslots > 0) {
             // compaction, bounding box, Morton order and the tile data sized for
             // every slot, the count of existing bodies read in the kernels; the
             // count and the radius range come back to the host (for the pair
@@ -951,7 +1018,6 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
             rr[1] = h3[1];
             n = (int)h3[2];
       }
-      const int central = P.par_central_mass_bool;
       const double G = P.par_G;
       const double mu = G * cmh[6];
       if (n == 0) {
@@ -963,35 +1029,6 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       const int npad = ntiles * T;
       const double sp = P.par_softening_parameter;
       const bool soft = sp != 0.;
-      BodyView cv = bv;
-      if (mode == NCGPU_GRAVITY_EXACT) {
-            D4 *src = (D4 *)c.src64;
-            k_pack_exact<<<(npad + 255) / 256, 256, 0, st>>>(cv, c.cidx, n, npad, G, src, c.srcR);
-            NCG_LAUNCHED();
-            int nb = (n + EXB - 1) / EXB;
-            const int p_lo = (int)((long)n * part / nparts), p_hi = (int)((long)n * (part + 1) / nparts);
-            NCG_CK(cudaEventRecord(c.kev0, st));
-            if (soft)
-                  k_grav_exact<true><<<nb, EXB, 0, st>>>(src, c.srcR, c.cidx, n, ntiles, cmh[0], cmh[1], cmh[2], mu,
-                                                         sp, central, j2, cv, p_lo, p_hi, ax, ay, az, c.cmterm,
-                                                         c.err);
-            else
-                  k_grav_exact<false><<<nb, EXB, 0, st>>>(src, c.srcR, c.cidx, n, ntiles, cmh[0], cmh[1], cmh[2],
-                                                          mu, sp, central, j2, cv, p_lo, p_hi, ax, ay, az, c.cmterm,
-                                                          c.err);
-            NCG_LAUNCHED();
-            NCG_CK(cudaEventRecord(c.kev1, st));
-            c.kev_valid = 1;
-            if (central) {
-                  k_seq_sum3<<<3, 32, 0, st>>>(c.cmterm, j2.on ? 2 * n : n, nullptr, d_cm_acc);
-            } else {
-                  k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
-            }
-            NCG_LAUNCHED();
-            return NCGPU_OK;
-      }
-      if (mode != NCGPU_GRAVITY_FP64 && mode != NCGPU_GRAVITY_MIXED) return NCGPU_E_ARG;
-
       // (the Morton order and the tile data were made above, before the count came back)
       D4 *s64 = (D4 *)c.src64;
       double eps2 = 0.;
@@ -1070,45 +1107,15 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
 namespace ncg {
 
 // The EXACT gravity of gravity_eval on caller-provided scratch, without the
-// library context: cidx (n), src (npad double4 = 4*npad doubles), srcR (npad),
-// cterm (3n, 6n with J2), blockcnt/n_dev for the compaction, err (1 word).  Writes ax, ay,
-// az (slots 0..largest_id, zero for empty slots) and d_cm_acc.
+// library context: cidx (n), src (n double4), srcR (n), blockcnt/n_dev for the
+// compaction.  Writes ax, ay, az (slots 0..largest_id, zero for empty slots) and
+// d_cm_acc.
 int gravity_exact_into(const BodyView &bv, int largest_id, const double *cmh, double G, double sp, int central,
-                       const J2Arg &j2, int *cidx, double *src, double *srcR, double *cterm, int *blockcnt,
-                       int *n_dev, unsigned *err, double *ax, double *ay, double *az, double *d_cm_acc,
-                       cudaStream_t st)
+                       const J2Arg &j2, int *cidx, double *src, double *srcR, int *blockcnt, int *n_dev, double *ax,
+                       double *ay, double *az, double *d_cm_acc, cudaStream_t st)
 {
-      const int nslots = largest_id + 1;
-      if (nslots > 0) {
-            k_fill3<<<(nslots + 255) / 256, 256, 0, st>>>(ax, ay, az, nslots, 0.);
-            NCG_LAUNCHED();
-      }
-      int n = 0;
-      NCG_TRY(compact_flags_into(bv.ex, nslots, blockcnt, n_dev, cidx, &n, st));
-      if (n == 0 || !central) {
-            k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
-            NCG_LAUNCHED();
-            if (n == 0) return NCGPU_OK;
-      }
-      const int ntiles = (n + T - 1) / T;
-      const int npad = ntiles * T;
-      const double mu = G * cmh[6];
-      D4 *s4 = (D4 *)src;
-      k_pack_exact<<<(npad + 255) / 256, 256, 0, st>>>(bv, cidx, n, npad, G, s4, srcR);
-      NCG_LAUNCHED();
-      const int nb = (n + EXB - 1) / EXB;
-      if (sp != 0.)
-            k_grav_exact<true><<<nb, EXB, 0, st>>>(s4, srcR, cidx, n, ntiles, cmh[0], cmh[1], cmh[2], mu, sp, central,
-                                                   j2, bv, 0, n, ax, ay, az, cterm, err);
-      else
-            k_grav_exact<false><<<nb, EXB, 0, st>>>(s4, srcR, cidx, n, ntiles, cmh[0], cmh[1], cmh[2], mu, sp,
-                                                    central, j2, bv, 0, n, ax, ay, az, cterm, err);
-      NCG_LAUNCHED();
-      if (central) {
-            k_seq_sum3<<<3, 32, 0, st>>>(cterm, j2.on ? 2 * n : n, nullptr, d_cm_acc);
-            NCG_LAUNCHED();
-      }
-      return NCGPU_OK;
+      return exact_field(bv, largest_id + 1, CmArg{nullptr, cmh[0], cmh[1], cmh[2], cmh[6]}, G, sp, central, j2, 0, 1, 0., cidx, (D4 *)src, srcR, blockcnt, n_dev,
+                         ax, ay, az, d_cm_acc, st, nullptr);
 }
 
 }  // namespace ncg

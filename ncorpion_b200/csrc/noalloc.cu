@@ -41,7 +41,7 @@ constexpr size_t OFF_CTERM = OFF_SRCR + NPAD * 8;               // 6 * NPAD doub
 constexpr size_t OFF_ACC = OFF_CTERM + 6 * NPAD * 8;            // 3 * NPAD doubles
 constexpr size_t OFF_CIDX = OFF_ACC + 3 * NPAD * 8;             // NPAD ints
 constexpr size_t OFF_BLK = OFF_CIDX + NPAD * 4;                 // NBLK ints
-constexpr size_t OFF_MISC = (OFF_BLK + NBLK * 4 + 255) / 256 * 256;  // n_dev, err
+constexpr size_t OFF_MISC = (OFF_BLK + NBLK * 4 + 255) / 256 * 256;  // n_dev
 constexpr size_t NOALLOC_SCRATCH_BYTES = OFF_MISC + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
@@ -86,28 +86,23 @@ extern "C" int ncgpu_vector_field_static(const double *d_bodies, const int *d_ex
       NCG_TRY(scratch_address(&base));
       cudaStream_t st = (cudaStream_t)stream;
       double *src = (double *)(base + OFF_SRC), *srcR = (double *)(base + OFF_SRCR);
-      double *cterm = (double *)(base + OFF_CTERM), *acc = (double *)(base + OFF_ACC);
+      double *acc = (double *)(base + OFF_ACC);
       int *cidx = (int *)(base + OFF_CIDX), *blk = (int *)(base + OFF_BLK);
       int *n_dev = (int *)(base + OFF_MISC);
-      unsigned *err = (unsigned *)(base + OFF_MISC + 64);
-      NCG_CK(cudaMemsetAsync(base + OFF_BLK, 0, OFF_MISC + 256 - OFF_BLK, st));  // counts, n, error word
+      NCG_CK(cudaMemsetAsync(base + OFF_BLK, 0, OFF_MISC + 256 - OFF_BLK, st));  // counts, n
       BodyView bv{d_bodies, d_bodies + 1, d_bodies + 2, d_bodies + 3, d_bodies + 4, d_bodies + 5,
                   d_bodies + 6, d_bodies + 7, 8, d_exists};
       const long bs = largest_id + 1;
       if (params->par_J2_bool && !params->par_central_mass_bool) return NCGPU_E_ARG;
       NCG_TRY(gravity_exact_into(bv, largest_id, (const double *)cm, params->par_G, params->par_softening_parameter,
-                                 params->par_central_mass_bool, j2_arg(*params, cm->mass, j2_value(*params, cm->mass, params->par_sideral_omega)), cidx, src, srcR, cterm,
-                                 blk, n_dev, err, acc,
-                                 acc + NPAD, acc + 2 * NPAD, d_cm_acc, st));
+                                 params->par_central_mass_bool,
+                                 j2_arg(*params, cm->mass, j2_value(*params, cm->mass, params->par_sideral_omega)), cidx,
+                                 src, srcR, blk, n_dev, acc, acc + NPAD, acc + 2 * NPAD, d_cm_acc, st));
       if (bs > 0) {
             for (int d = 0; d < 3; d++)
                   NCG_CK(cudaMemcpy2DAsync(d_acc + d, 3 * sizeof(double), acc + d * NPAD, sizeof(double),
                                            sizeof(double), bs, cudaMemcpyDeviceToDevice, st));
       }
-      unsigned h = 0;
-      NCG_CK(cudaMemcpyAsync(&h, err, sizeof h, cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
-      if (h & ERR_TIMEOUT) return NCGPU_E_TIMEOUT;
-      if (h) return NCGPU_E_CUDA;
       return NCGPU_OK;
 }

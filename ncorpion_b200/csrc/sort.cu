@@ -277,39 +277,38 @@ int scan_exclusive(const int *in, int *out, int n, int *sums, cudaStream_t st)
       return NCGPU_OK;
 }
 
+// Order-preserving compaction of the flagged slots 0..n_slots-1 into out_idx
+// with caller-provided scratch; the count in *n_dev.
+int compact_flags_dev(const int *flags, int n_slots, int *blockcnt, int *n_dev, int *out_idx, cudaStream_t st)
+{
+      if (n_slots <= 0) {
+            NCG_CK(cudaMemsetAsync(n_dev, 0, sizeof(int), st));
+            return NCGPU_OK;
+      }
+      int nb = (n_slots + CB - 1) / CB;
+      k_count_flags<<<nb, CB, 0, st>>>(flags, n_slots, blockcnt);
+      NCG_LAUNCHED();
+      k_scan_single<<<1, 1024, 0, st>>>(blockcnt, nb, n_dev);
+      NCG_LAUNCHED();
+      k_scatter_flags<<<nb, CB, 0, st>>>(flags, n_slots, blockcnt, out_idx);
+      NCG_LAUNCHED();
+      return NCGPU_OK;
+}
+
 int compact_existing_dev(const int *ex, int largest_id, cudaStream_t st)
 {
       Ctx &c = ctx();
-      int n = largest_id + 1;
-      if (n <= 0) {
-            NCG_CK(cudaMemsetAsync(c.n_dev, 0, sizeof(int), st));
-            return NCGPU_OK;
-      }
-      int nb = (n + CB - 1) / CB;
-      k_count_flags<<<nb, CB, 0, st>>>(ex, n, c.cnt);
-      NCG_LAUNCHED();
-      k_scan_single<<<1, 1024, 0, st>>>(c.cnt, nb, c.n_dev);
-      NCG_LAUNCHED();
-      k_scatter_flags<<<nb, CB, 0, st>>>(ex, n, c.cnt, c.cidx);
-      NCG_LAUNCHED();
-      return NCGPU_OK;
+      return compact_flags_dev(ex, largest_id + 1, c.cnt, c.n_dev, c.cidx, st);
 }
 
 int compact_existing(const int *ex, int largest_id, int *n_host, cudaStream_t st)
 {
       Ctx &c = ctx();
-      int n = largest_id + 1;
-      if (n <= 0) {
+      if (largest_id < 0) {
             *n_host = 0;
             return NCGPU_OK;
       }
-      int nb = (n + CB - 1) / CB;
-      k_count_flags<<<nb, CB, 0, st>>>(ex, n, c.cnt);
-      NCG_LAUNCHED();
-      k_scan_single<<<1, 1024, 0, st>>>(c.cnt, nb, c.n_dev);
-      NCG_LAUNCHED();
-      k_scatter_flags<<<nb, CB, 0, st>>>(ex, n, c.cnt, c.cidx);
-      NCG_LAUNCHED();
+      NCG_TRY(compact_existing_dev(ex, largest_id, st));
       NCG_CK(cudaMemcpyAsync(n_host, c.n_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
       return NCGPU_OK;
@@ -361,32 +360,6 @@ int radix_sort_pairs(uint32_t *keys, int *vals, int n, int bits, cudaStream_t st
             NCG_CK(cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, st));
             NCG_CK(cudaMemcpyAsync(vals, va, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st));
       }
-      return NCGPU_OK;
-}
-
-}  // namespace ncg
-
-namespace ncg {
-
-// Order-preserving compaction of the flagged slots 0..n_slots-1 into out_idx
-// with caller-provided scratch (blockcnt: ceil(n_slots/1024) + 1 ints, n_dev:
-// 1 int); the count is copied to *n_host (synchronises the stream).
-int compact_flags_into(const int *flags, int n_slots, int *blockcnt, int *n_dev, int *out_idx, int *n_host,
-                       cudaStream_t st)
-{
-      if (n_slots <= 0) {
-            *n_host = 0;
-            return NCGPU_OK;
-      }
-      int nb = (n_slots + CB - 1) / CB;
-      k_count_flags<<<nb, CB, 0, st>>>(flags, n_slots, blockcnt);
-      NCG_LAUNCHED();
-      k_scan_single<<<1, 1024, 0, st>>>(blockcnt, nb, n_dev);
-      NCG_LAUNCHED();
-      k_scatter_flags<<<nb, CB, 0, st>>>(flags, n_slots, blockcnt, out_idx);
-      NCG_LAUNCHED();
-      NCG_CK(cudaMemcpyAsync(n_host, n_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-      NCG_CK(cudaStreamSynchronize(st));
       return NCGPU_OK;
 }
 

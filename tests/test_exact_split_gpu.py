@@ -1,0 +1,49 @@
+"""GPU: the exact force kernel at the edges of its split (8 targets a CTA, rounds
+of 64 sources, 256 bodies a round of CM_acc, one preparation CTA up to 8,192 slots,
+512 threads a CTA up to 2,048): bit-identical to the oracle, with empty slots, with
+softening and J2 on and off, with bodies whose offsets are signed zeros, and in parts."""
+import numpy as np
+import pytest
+
+from conftest import make_params
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("soft,j2", [(0.0, 0), (0.5, 1)])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 63, 64, 65, 255, 257, 513, 2047, 2049, 2600])
+def test_bits(lib, port, n, soft, j2):
+    from ncorpion_b200 import api, disks
+    rng = np.random.default_rng(n)
+    b = disks.gravity_disk(n, seed=n)
+    if n >= 63:  # planes of equal coordinates, of either sign of zero
+        b[: n // 3, 2] = 0.0
+        b[n // 4: n // 3, 2] = -0.0
+        b[5:20, 0] = b[5, 0]
+    ex = np.ones(n, np.int32)
+    if n > 8:
+        ex[rng.random(n) < 0.1] = 0
+    cm = np.array([1e-6, -2e-6, 0.0, 0, 0, 0, 1.0, 1.0])
+    p = make_params(softening_parameter=soft, J2_bool=j2, J2=1e-3 if j2 else 0.0)
+    api.init(n, p)
+    ref, cref = port.vector_field(b, ex, cm, p)
+    acc, cma = api.vector_field(b, ex, cm, mode="exact")
+    assert np.array_equal(acc.view(np.int64)[ex == 1], np.ascontiguousarray(ref).view(np.int64)[ex == 1])
+    assert np.array_equal(cma, cref)
+    api.finalize()
+
+
+def test_past_the_preparation_cta(lib, port):
+    """8,192 and 8,193 slots with most of them empty: the two compactions give the same field."""
+    from ncorpion_b200 import api, disks
+    p = make_params(softening_parameter=0.5)
+    cm = np.array([0.0, 0, 0, 0, 0, 0, 1.0, 1.0])
+    b = disks.gravity_disk(8193, seed=1)
+    ex = (np.random.default_rng(0).random(8193) < 0.1).astype(np.int32)
+    ex[8192] = 0
+    api.init(8193, p)
+    ref, cref = port.vector_field(b, ex, cm, p)
+    for k in (8192, 8193):
+        acc, cma = api.vector_field(b[:k], ex[:k], cm, mode="exact")
+        assert np.array_equal(acc, ref[:k] * (ex[:k] != 0)[:, None]) and np.array_equal(cma, cref)
+    api.finalize()
