@@ -18,7 +18,7 @@
 // rsqrt per pair); the JVP is summed body by body, tiled through shared memory
 // with (target block, source chunk) work units reduced in a fixed order.  In the
 // MIXED gravity mode the bodies are taken in the Morton order of their initial
-// positions (a permutation done on the host at the call's boundary), every
+// positions (a permutation at the call's boundary), every
 // evaluation computes the 128-body tiles' boxes, and only the tile pairs whose
 // boxes are near (near_theta x the larger diagonal, and each tile with itself)
 // are summed in FP64; the others in FP32 on coordinates relative to a tile's
@@ -30,8 +30,8 @@
 // more.  N = 16,384, mixed: a force's pair sums take 128 us and a VJP's 269 (208
 // and 396 when each body's were made by themselves, bound by the FP32 pipe and the
 // near tiles' FP64), a forward call and a forward + adjoint call of 32 steps
-// 28.7 ms (42.9 with those and with six to nine launches a step).  N = 5,003, FP64:
-// 32 us and 62 (50 and 86), 24 steps 6.35 ms (9.46).
+// 24.5 ms (42.3 with those, with six to nine launches a step and strided copies of the
+// caller's arrays).  N = 5,003, FP64: 32 us and 62 (50 and 86), 24 steps 5.73 ms (9.47).
 #include <algorithm>
 #include <vector>
 #include "common.cuh"
@@ -510,6 +510,8 @@ struct LF {
       int C, ncp;
       bool mixed;                  // MIXED gravity mode
       double theta, *box;
+      double *stage;               // the caller's arrays, 3 n
+      const int *perm;             // the caller's body at each position (null: the same)
       cudaStream_t st;
 };
 
@@ -581,18 +583,44 @@ int lf_step_jvp(LF &L, double dt)
       return NCGPU_OK;
 }
 
-void split3(double *dst, const double *src, int n, cudaStream_t st, cudaError_t *e)
+// The caller's arrays cross in one contiguous copy each and are put in the pair
+// sums' order (perm: the body at each position; null: the caller's order) and into
+// three blocks of n on the device.  (Three strided copies of 8-byte rows an array,
+// and the permutation on the host, took 1.0-1.3 ms a call at 16,384 bodies before
+// any step.)
+__global__ void k_gather_rows(const double *__restrict__ in, const int *__restrict__ perm, int n, int width,
+                              double *__restrict__ out)
 {
-      for (int d = 0; d < 3 && *e == cudaSuccess; d++)
-            *e = cudaMemcpy2DAsync(dst + (size_t)d * n, sizeof(double), src + d, 3 * sizeof(double), sizeof(double), n,
-                                   cudaMemcpyHostToDevice, st);
+      const int k = blockIdx.x * blockDim.x + threadIdx.x;
+      if (k >= n) return;
+      const size_t b = perm ? perm[k] : k;
+      for (int d = 0; d < width; d++) out[(size_t)d * n + k] = in[width * b + d];
 }
 
-void join3(double *dst, const double *src, int n, cudaStream_t st, cudaError_t *e)
+__global__ void k_scatter_rows(const double *__restrict__ in, const int *__restrict__ perm, int n, int width,
+                               double *__restrict__ out)
 {
-      for (int d = 0; d < 3 && *e == cudaSuccess; d++)
-            *e = cudaMemcpy2DAsync(dst + d, 3 * sizeof(double), src + (size_t)d * n, sizeof(double), sizeof(double), n,
-                                   cudaMemcpyDeviceToHost, st);
+      const int k = blockIdx.x * blockDim.x + threadIdx.x;
+      if (k >= n) return;
+      const size_t b = perm ? perm[k] : k;
+      for (int d = 0; d < width; d++) out[width * b + d] = in[(size_t)d * n + k];
+}
+
+// src (host, n rows of `width` doubles) into dst (device, `width` blocks of n)
+int rows_in(LF &L, double *dst, const double *src, int width)
+{
+      NCG_CK(cudaMemcpyAsync(L.stage, src, sizeof(double) * width * (size_t)L.n, cudaMemcpyHostToDevice, L.st));
+      k_gather_rows<<<(L.n + 255) / 256, 256, 0, L.st>>>(L.stage, L.perm, L.n, width, dst);
+      NCG_LAUNCHED();
+      return NCGPU_OK;
+}
+
+int rows_out(LF &L, double *dst, const double *src, int width)
+{
+      k_scatter_rows<<<(L.n + 255) / 256, 256, 0, L.st>>>(src, L.perm, L.n, width, L.stage);
+      NCG_LAUNCHED();
+      NCG_CK(cudaMemcpyAsync(dst, L.stage, sizeof(double) * width * (size_t)L.n, cudaMemcpyDeviceToHost, L.st));
+      return NCGPU_OK;
 }
 
 // sR = sp * R, element by element (in place when sR == R), and its FP32 copy with
@@ -614,7 +642,8 @@ __global__ void k_xf(const double *__restrict__ X, const double *__restrict__ V,
             for (int d = 0; d < 3; d++) out[(size_t)d * n + k] = X[(size_t)d * n + k] - h * V[(size_t)d * n + k];
 }
 
-int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
+// perm (host, may be null): the caller's body at each position of the sums' order.
+int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed, const int *perm)
 {
       const bool vjp = mode == 1, jvp = mode == 2;
       Ctx &c = ctx();
@@ -668,7 +697,8 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
                      + 3 * N * 2 + 6 + N                                         // lx lv LX LV gm
                      + (vjp ? st * L.ncp + (size_t)L.C * (3 * N + 3) : 0)        // checkpoints, segment
                      + (jvp ? 3 * N * 3 + N + 6 + 3 + 3 * N * L.nch : 0)         // tx tv tm tX da dA, partials
-                     + 6 * (size_t)L.ntiles;                                     // tile boxes
+                     + 6 * (size_t)L.ntiles                                      // tile boxes
+                     + 3 * N + (N + 1) / 2;                                      // stage, perm
       if (total > c.lf_cap) {  // grown when needed, kept for the next call
             if (c.lf_buf) cudaFree(c.lf_buf);
             c.lf_buf = nullptr;
@@ -695,17 +725,20 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
             L.jpart = take(3 * N * L.nch);
       }
       L.box = take(6 * (size_t)L.ntiles);
+      L.stage = take(3 * N);
+      int *perm_dev = (int *)take((N + 1) / 2);
+      L.perm = perm ? perm_dev : nullptr;
       int status = NCGPU_OK;
       cudaError_t e = cudaSuccess;
       const double h = a->dt / 2.0, dt = a->dt;
       const int nb = (n + 255) / 256;
-      split3(L.X, a->x0, n, L.st, &e);
-      split3(L.V, a->v0, n, L.st, &e);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(L.m, a->m, sizeof(double) * N, cudaMemcpyHostToDevice, L.st);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(L.sR, a->R, sizeof(double) * N, cudaMemcpyHostToDevice, L.st);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(L.cm, a->cm, 6 * sizeof(double), cudaMemcpyHostToDevice, L.st);
-      if (e == cudaSuccess) e = cudaMemsetAsync(L.count, 0, sizeof(unsigned), L.st);
-      if (e != cudaSuccess) return cuda_fail(e, "leapfrog upload", __FILE__, __LINE__);
+      if (perm) NCG_CK(cudaMemcpyAsync(perm_dev, perm, sizeof(int) * N, cudaMemcpyHostToDevice, L.st));
+      NCG_TRY(rows_in(L, L.X, a->x0, 3));
+      NCG_TRY(rows_in(L, L.V, a->v0, 3));
+      NCG_TRY(rows_in(L, L.m, a->m, 1));
+      NCG_TRY(rows_in(L, L.sR, a->R, 1));
+      NCG_CK(cudaMemcpyAsync(L.cm, a->cm, 6 * sizeof(double), cudaMemcpyHostToDevice, L.st));
+      NCG_CK(cudaMemsetAsync(L.count, 0, sizeof(unsigned), L.st));
 #define LF_TRY(call)                         \
       do {                                   \
             if ((status = (call)) != NCGPU_OK) goto done; \
@@ -719,10 +752,10 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
       k_scale_R<<<(int)((NP + 255) / 256), 256, 0, L.st>>>(L.sR, sp, L.sR, n, L.sR32, (int)NP);
       LF_LAUNCHED();
       if (jvp) {
-            split3(L.tx, a->tan_x0, n, L.st, &e);
-            split3(L.tv, a->tan_v0, n, L.st, &e);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(L.tm, a->tan_m, sizeof(double) * N, cudaMemcpyHostToDevice, L.st);
-            if (e == cudaSuccess) e = cudaMemsetAsync(L.tX, 0, 6 * sizeof(double), L.st);
+            LF_TRY(rows_in(L, L.tx, a->tan_x0, 3));
+            LF_TRY(rows_in(L, L.tv, a->tan_v0, 3));
+            LF_TRY(rows_in(L, L.tm, a->tan_m, 1));
+            e = cudaMemsetAsync(L.tX, 0, 6 * sizeof(double), L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "tangent upload", __FILE__, __LINE__); goto done; }
             k_axpy3<<<nb, 256, 0, L.st>>>(h, L.tv, L.tx, n, n, nullptr, nullptr);
             LF_LAUNCHED();
@@ -743,22 +776,22 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
       if (jvp) {
             k_xf<<<nb, 256, 0, L.st>>>(L.tx, L.tv, h, L.da, n);
             LF_LAUNCHED();
-            join3(a->tan_x_final, L.da, n, L.st, &e);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(L.st);
+            LF_TRY(rows_out(L, a->tan_x_final, L.da, 3));
+            e = cudaStreamSynchronize(L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "tangent download", __FILE__, __LINE__); goto done; }
       }
       if (a->x_final || a->v_final) {
             k_xf<<<nb, 256, 0, L.st>>>(L.X, L.V, h, L.out, n);  // half back-drift of the output (src/rk4.c:929-936)
             LF_LAUNCHED();
-            if (a->x_final) join3(a->x_final, L.out, n, L.st, &e);
-            if (a->v_final) join3(a->v_final, L.V, n, L.st, &e);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(L.st);
+            if (a->x_final) LF_TRY(rows_out(L, a->x_final, L.out, 3));
+            if (a->v_final) LF_TRY(rows_out(L, a->v_final, L.V, 3));
+            e = cudaStreamSynchronize(L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "leapfrog download", __FILE__, __LINE__); goto done; }
       }
       if (vjp) {
             // x_F = x_n - h v_n
-            split3(L.lx, a->adj_x_final, n, L.st, &e);
-            if (e == cudaSuccess) e = cudaMemsetAsync(L.lv, 0, sizeof(double) * 3 * N, L.st);
+            LF_TRY(rows_in(L, L.lx, a->adj_x_final, 3));
+            e = cudaMemsetAsync(L.lv, 0, sizeof(double) * 3 * N, L.st);
             if (e == cudaSuccess) e = cudaMemsetAsync(L.LX, 0, 6 * sizeof(double), L.st);  // LX, LV
             if (e == cudaSuccess) e = cudaMemsetAsync(L.gm, 0, sizeof(double) * N, L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "adjoint init", __FILE__, __LINE__); goto done; }
@@ -782,10 +815,10 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed)
             // initial half drift x = x0 + h v0
             k_axpy3<<<nb, 256, 0, L.st>>>(h, L.lx, L.lv, n, n, nullptr, nullptr);
             LF_LAUNCHED();
-            join3(a->grad_x0, L.lx, n, L.st, &e);
-            join3(a->grad_v0, L.lv, n, L.st, &e);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(a->grad_m, L.gm, sizeof(double) * N, cudaMemcpyDeviceToHost, L.st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(L.st);
+            LF_TRY(rows_out(L, a->grad_x0, L.lx, 3));
+            LF_TRY(rows_out(L, a->grad_v0, L.lv, 3));
+            LF_TRY(rows_out(L, a->grad_m, L.gm, 1));
+            e = cudaStreamSynchronize(L.st);
             if (e != cudaSuccess) { status = cuda_fail(e, "adjoint download", __FILE__, __LINE__); goto done; }
       }
 #undef LF_TRY
@@ -806,72 +839,53 @@ void morton_order(const double *x, int n, std::vector<int> &perm)
                   hi[d] = std::max(hi[d], x[3 * k + d]);
             }
       const double ext = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
-      std::vector<uint32_t> key(n);
+      auto spread = [](uint32_t v) {  // bits 0..9 to 0, 3, ..., 27
+            v = (v | (v << 16)) & 0x030000ffu;
+            v = (v | (v << 8)) & 0x0300f00fu;
+            v = (v | (v << 4)) & 0x030c30c3u;
+            return (v | (v << 2)) & 0x09249249u;
+      };
+      // a stable radix sort, three digits of 10 bits (16,384 bodies: 0.2 ms; 1.6 ms
+      // with the keys bit by bit and a comparison sort)
+      constexpr int D = 1024;
+      std::vector<uint32_t> key(n), kb(n);
+      std::vector<int> pb(n), at(3 * D, 0);
       for (int k = 0; k < n; k++) {
-            uint32_t q[3];
+            uint32_t m = 0;
             for (int d = 0; d < 3; d++) {
                   const double f = ext > 0. ? (x[3 * k + d] - lo[d]) / ext : 0.;
-                  q[d] = (uint32_t)std::min(std::max((int)(f * 1023.999), 0), 1023);
+                  m |= spread((uint32_t)std::min(std::max((int)(f * 1023.999), 0), 1023)) << d;
             }
-            uint32_t m = 0;
-            for (int b = 9; b >= 0; b--)
-                  for (int d = 2; d >= 0; d--) m = (m << 1) | ((q[d] >> b) & 1u);
             key[k] = m;
+            for (int q = 0; q < 3; q++) at[q * D + ((m >> (10 * q)) & (D - 1))]++;
       }
       perm.resize(n);
       for (int k = 0; k < n; k++) perm[k] = k;
-      std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return key[a] < key[b]; });
+      for (int q = 0; q < 3; q++) {
+            int *c = &at[q * D], run = 0;
+            for (int v = 0; v < D; v++) {
+                  const int w = c[v];
+                  c[v] = run;
+                  run += w;
+            }
+            for (int k = 0; k < n; k++) {
+                  const int to = c[(key[k] >> (10 * q)) & (D - 1)]++;
+                  kb[to] = key[k];
+                  pb[to] = perm[k];
+            }
+            key.swap(kb);
+            perm.swap(pb);
+      }
 }
 
-// The MIXED mode runs on the bodies in Morton order of their initial
-// positions: the inputs are permuted here, the outputs restored to the
-// caller's order.
+// The MIXED mode runs on the bodies in Morton order of their initial positions.
 int lf_run(const struct ncgpu_leapfrog_args *a, int mode)
 {
-      Ctx &c = ctx();
-      if (c.P.par_gravity_mode != NCGPU_GRAVITY_MIXED) return lf_core(a, mode, false);
-      const int n = a->n;
-      if (n <= 0 || !a->x0 || !a->v0 || !a->m || !a->R || !a->cm || a->nsteps < 0) return NCGPU_E_ARG;
+      if (ctx().P.par_gravity_mode != NCGPU_GRAVITY_MIXED) return lf_core(a, mode, false, nullptr);
+      if (a->n <= 0 || !a->x0 || !a->v0 || !a->m || !a->R || !a->cm || a->nsteps < 0) return NCGPU_E_ARG;
       std::vector<int> perm;
-      morton_order(a->x0, n, perm);
-      const size_t N = (size_t)n;
-      auto gather3 = [&](const double *src, std::vector<double> &dst) {
-            dst.resize(3 * N);
-            for (size_t i = 0; i < N; i++)
-                  for (int d = 0; d < 3; d++) dst[3 * i + d] = src[3 * (size_t)perm[i] + d];
-      };
-      auto gather1 = [&](const double *src, std::vector<double> &dst) {
-            dst.resize(N);
-            for (size_t i = 0; i < N; i++) dst[i] = src[perm[i]];
-      };
-      std::vector<double> x0, v0, m, R, adj, tx0, tv0, tm, xf, vf, gx, gv, gm, txf;
-      gather3(a->x0, x0); gather3(a->v0, v0); gather1(a->m, m); gather1(a->R, R);
-      struct ncgpu_leapfrog_args b = *a;
-      b.x0 = x0.data(); b.v0 = v0.data(); b.m = m.data(); b.R = R.data();
-      if (a->adj_x_final) { gather3(a->adj_x_final, adj); b.adj_x_final = adj.data(); }
-      if (a->tan_x0) { gather3(a->tan_x0, tx0); b.tan_x0 = tx0.data(); }
-      if (a->tan_v0) { gather3(a->tan_v0, tv0); b.tan_v0 = tv0.data(); }
-      if (a->tan_m) { gather1(a->tan_m, tm); b.tan_m = tm.data(); }
-      if (a->x_final) { xf.resize(3 * N); b.x_final = xf.data(); }
-      if (a->v_final) { vf.resize(3 * N); b.v_final = vf.data(); }
-      if (a->grad_x0) { gx.resize(3 * N); b.grad_x0 = gx.data(); }
-      if (a->grad_v0) { gv.resize(3 * N); b.grad_v0 = gv.data(); }
-      if (a->grad_m) { gm.resize(N); b.grad_m = gm.data(); }
-      if (a->tan_x_final) { txf.resize(3 * N); b.tan_x_final = txf.data(); }
-      const int st = lf_core(&b, mode, true);
-      if (st != NCGPU_OK) return st;
-      auto scatter3 = [&](const std::vector<double> &src, double *dst) {
-            for (size_t i = 0; i < N; i++)
-                  for (int d = 0; d < 3; d++) dst[3 * (size_t)perm[i] + d] = src[3 * i + d];
-      };
-      if (a->x_final) scatter3(xf, a->x_final);
-      if (a->v_final) scatter3(vf, a->v_final);
-      if (a->grad_x0) scatter3(gx, a->grad_x0);
-      if (a->grad_v0) scatter3(gv, a->grad_v0);
-      if (a->grad_m)
-            for (size_t i = 0; i < N; i++) a->grad_m[perm[i]] = gm[i];
-      if (a->tan_x_final) scatter3(txf, a->tan_x_final);
-      return NCGPU_OK;
+      morton_order(a->x0, a->n, perm);
+      return lf_core(a, mode, true, perm.data());
 }
 
 }  // namespace
