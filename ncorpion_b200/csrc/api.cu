@@ -75,7 +75,7 @@ void free_all()
       mesh_free();
       void *ptrs[] = {c.x, c.y, c.z, c.vx, c.vy, c.vz, c.m, c.R, c.ex, c.cm, c.cm_acc, c.acc, c.cmterm,
                       c.partial, c.cidx, c.cnt, c.n_dev, c.src64, c.srcR, c.src32, c.srcR32, c.tilebox,
-                      c.keys, c.keys2, c.vals, c.vals2, c.hist, c.red, c.err, c.aos, c.exs,
+                      c.keys, c.keys2, c.vals, c.vals2, c.hist, c.red, c.aos, c.exs,
                       c.did, c.dirty, c.dlist, c.free_idx, c.scal, c.hi, c.hj, c.ev, c.evrec,
                       c.snap[0], c.snap[1], c.snap[2], c.snap[3], c.snap[4], c.snap[5], c.snap[6], c.snap[7],
                       c.snap_cm, c.fmt_slots, c.fmt_text, c.fmt_len, c.ell, c.ell_code, c.ell_list, c.lf_buf};
@@ -383,9 +383,9 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
       c.hist_cap = 256 * ((NS + 2047) / 2048);
       A(c.hist, c.hist_cap + 1);  // + total of the in-place scan
       A(c.red, 4096);
-      A(c.err, 1);
       A(c.aos, 8 * N);
-      A(c.did, N); A(c.dirty, N); A(c.dlist, 3 * N); A(c.free_idx, N); A(c.scal, S_COUNT);
+      A(c.did, N); A(c.dirty, N); A(c.dlist, 3 * N); A(c.free_idx, N); A(c.scal, S_COUNT + 1);
+      c.err = (unsigned *)(c.scal + S_COUNT);  // (they come back in one copy)
       c.hit_cap = (int)NS;
       A(c.hi, NS); A(c.hj, NS);
       c.ev_cap = (int)(2 * N + 1024);

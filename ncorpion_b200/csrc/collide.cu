@@ -9,7 +9,8 @@
 //                     (exact reference arithmetic) by a tiled sweep; colliding
 //                     pairs are appended through a warp-aggregated atomic
 //                     counter.
-//   2. sort           hits ordered by (i, j) with two stable radix passes.
+//   2. sort           hits ordered by (i, j): by k_bf_events itself for few bodies,
+//                     else with two stable radix passes.
 //   3. k_bf_events    one CTA replays the sweep order: the next event is the
 //                     smallest (i, j) after the last one that either is an
 //                     entry-state hit between two untouched bodies, or involves
@@ -17,6 +18,7 @@
 //                     current state (those pairs are re-tested in parallel by
 //                     the CTA).  Events are resolved one by one with the
 //                     reference's arithmetic, so state and event order match.
+#include <algorithm>
 #include "common.cuh"
 #include "physics.cuh"
 
@@ -48,24 +50,25 @@ __device__ __forceinline__ void append_hit(bool hit, int i, int j, int *hi, int 
       }
 }
 
-// One CTA per (i tile, j tile) with j tile >= i tile; thread = body i.
-__global__ void __launch_bounds__(BT) k_bf_hits(DevState S, int lid, double dt, int *hi, int *hj, int cap,
+// One CTA per (BT bodies i, jn bodies j), thread = body i, the bodies j staged in
+// shared memory (closest_approach's test on the same values); a CTA whose bodies j
+// all precede its bodies i leaves.  jn = 32 up to 8,192 slots: the sweep is then a few
+// waves of short CTAs (2,000 bodies, 128 at a time: 136 CTAs with work, one an SM,
+// 128 tests in a row, 29 us; 32 at a time 11).
+__global__ void __launch_bounds__(BT) k_bf_hits(DevState S, int lid, int jper, double dt, int *hi, int *hj, int cap,
                                                 unsigned *err)
 {
-      // tile (ti, tj), tj >= ti: body i of the thread against the tile's bodies j
-      // staged in shared memory (closest_approach's test on the same values)
       __shared__ double sj[7][BT];
       __shared__ int sv[BT];
-      const int ti = blockIdx.y, tj = blockIdx.x;
-      if (tj < ti) return;
-      const int i = ti * BT + threadIdx.x;
+      const int i0 = blockIdx.y * BT, j0 = blockIdx.x * jper;
+      if (j0 + jper - 1 <= i0) return;
+      const int i = i0 + threadIdx.x;
       const bool vi = i <= lid && S.ex[i] && !S.did[i];
       double xi = 0., yi = 0., zi = 0., vxi = 0., vyi = 0., vzi = 0., Ri = 0.;
       if (vi) {
             xi = S.x[i]; yi = S.y[i]; zi = S.z[i]; vxi = S.vx[i]; vyi = S.vy[i]; vzi = S.vz[i]; Ri = S.R[i];
       }
-      const int j0 = tj * BT;
-      const int jn = min(BT, lid + 1 - j0);
+      const int jn = min(jper, lid + 1 - j0);
       if ((int)threadIdx.x < jn) {
             const int j = j0 + threadIdx.x;
             sj[0][threadIdx.x] = S.x[j]; sj[1][threadIdx.x] = S.y[j]; sj[2][threadIdx.x] = S.z[j];
@@ -74,6 +77,7 @@ __global__ void __launch_bounds__(BT) k_bf_hits(DevState S, int lid, double dt, 
             sv[threadIdx.x] = S.ex[j] && !S.did[j];
       }
       __syncthreads();
+#pragma unroll 4
       for (int jj = 0; jj < jn; ++jj) {
             const int j = j0 + jj;
             bool hit = false;
@@ -164,15 +168,53 @@ __device__ void d_treat(const DevState &S, int a, int b, const EvArgs &E, int *e
       S.scal[S_NDIRTY] = nd;
 }
 
+// The hits' keys (i, j) into ascending order: a bitonic network of the CTA over the
+// next power of two, padded with the largest key; in shared memory up to EVS hits,
+// in `k` otherwise.
+constexpr int EVS = 2048;
+
+__device__ void sort_keys(unsigned long long *k, int n)
+{
+      int m = 1;
+      while (m < n) m <<= 1;
+      for (int q = n + threadIdx.x; q < m; q += EVT) k[q] = ~0ull;
+      __syncthreads();
+      for (int size = 2; size <= m; size <<= 1)
+            for (int gap = size >> 1; gap > 0; gap >>= 1) {
+                  for (int q = threadIdx.x; q < m / 2; q += EVT) {
+                        const int a = 2 * q - (q & (gap - 1)), b = a + gap;
+                        const unsigned long long x = k[a], y = k[b];
+                        if ((x > y) == ((a & size) == 0)) {
+                              k[a] = y;
+                              k[b] = x;
+                        }
+                  }
+                  __syncthreads();
+            }
+}
+
+// sorted: hi, hj are in order (the host sorted them); else this kernel orders the
+// S_NHITS hits itself (gk: room for kcap keys, a power of two), so that the host need
+// not learn their number.  Clears the dirty marks it set.
 __global__ void __launch_bounds__(EVT) k_bf_events(DevState S, const int *__restrict__ hi, const int *__restrict__ hj,
                                                    EvArgs E, int *ev, double *evrec, unsigned char *dirty, int *dlist,
-                                                   unsigned *err)
+                                                   unsigned *err, int sorted, unsigned long long *gk, int kcap)
 {
       __shared__ unsigned long long best;
       __shared__ unsigned long long candA;
       __shared__ int hp_s;
+      __shared__ unsigned long long sk[EVS];
       const unsigned long long INF = ~0ull;
-      const int nh = min(S.scal[S_NHITS], (int)0x7fffffff);
+      const int nh = S.scal[S_NHITS];
+      unsigned long long *keys = nh <= EVS ? sk : gk;
+      if (!sorted) {
+            if (nh > kcap) {
+                  if (threadIdx.x == 0) atomicOr(err, ERR_CAPACITY);
+                  return;
+            }
+            for (int q = threadIdx.x; q < nh; q += EVT) keys[q] = pkey(hi[q], hj[q]);
+            if (nh > 1) sort_keys(keys, nh);
+      }
       unsigned long long cur = 0;  // key of the last event; (0, 0) is never a pair
       if (threadIdx.x == 0) hp_s = 0;
       __syncthreads();
@@ -185,9 +227,14 @@ __global__ void __launch_bounds__(EVT) k_bf_events(DevState S, const int *__rest
             }
             if (threadIdx.x == 0) {
                   int hp = hp_s;
-                  while (hp < nh && (pkey(hi[hp], hj[hp]) <= cur || dirty[hi[hp]] || dirty[hj[hp]])) hp++;
+                  unsigned long long key = INF;
+                  for (; hp < nh; hp++) {
+                        key = sorted ? pkey(hi[hp], hj[hp]) : keys[hp];
+                        if (key > cur && !dirty[key >> 32] && !dirty[key & 0xffffffffu]) break;
+                        key = INF;
+                  }
                   hp_s = hp;
-                  candA = hp < nh ? pkey(hi[hp], hj[hp]) : INF;
+                  candA = key;
                   best = candA;
             }
             __syncthreads();
@@ -215,12 +262,9 @@ __global__ void __launch_bounds__(EVT) k_bf_events(DevState S, const int *__rest
             cur = nxt;
             __syncthreads();
       }
-}
-
-__global__ void k_clear_dirty(unsigned char *dirty, const int *dlist, const int *scal)
-{
-      int n = scal[S_NDIRTY];
-      for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dirty[dlist[k]] = 0;
+      __syncthreads();
+      const int nd = S.scal[S_NDIRTY];
+      for (int k = threadIdx.x; k < nd; k += EVT) dirty[dlist[k]] = 0;
 }
 
 }  // namespace
@@ -266,10 +310,11 @@ int sync_scalars() { int h[S_COUNT]; return sync_scalars_h(h); }
 int sync_scalars_h(int *h)
 {
       Ctx &c = ctx();
-      unsigned e = 0;  // the device scalars and the error word behind one synchronisation
-      NCG_CK(cudaMemcpyAsync(h, c.scal, sizeof(int) * S_COUNT, cudaMemcpyDeviceToHost, c.s));
-      NCG_CK(cudaMemcpyAsync(&e, c.err, sizeof e, cudaMemcpyDeviceToHost, c.s));
+      int b[S_COUNT + 1];  // the device scalars and the error word behind them: one copy
+      NCG_CK(cudaMemcpyAsync(b, c.scal, sizeof b, cudaMemcpyDeviceToHost, c.s));
       NCG_CK(cudaStreamSynchronize(c.s));
+      std::copy(b, b + S_COUNT, h);
+      const unsigned e = (unsigned)b[S_COUNT];
       c.largest_id = h[S_LID];
       c.n_events = h[S_NEV];
       c.collision_count = h[S_CCOUNT];
@@ -289,27 +334,33 @@ int collide_brute_state(bool defer)
             NCG_CK(cudaMemsetAsync(c.scal + S_NEV, 0, sizeof(int), st));
             return sync_scalars();
       }
-      // S_NHITS, S_NEV, S_NDIRTY = 0
-      NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, 2 * sizeof(int), st));
-      NCG_CK(cudaMemsetAsync(c.scal + S_NDIRTY, 0, sizeof(int), st));
+      static_assert(S_NEV == S_NHITS + 1 && S_NDIRTY == S_NHITS + 2, "one clear for the three");
+      NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, 3 * sizeof(int), st));
       DevState S = dev_state();
-      const int nt = (lid + BT) / BT;
-      dim3 grid(nt, nt);
-      k_bf_hits<<<grid, BT, 0, st>>>(S, lid, c.dt, c.hi, c.hj, c.hit_cap, c.err);
+      const int jper = lid < 8192 ? 32 : BT;
+      k_bf_hits<<<dim3(lid / jper + 1, lid / BT + 1), BT, 0, st>>>(S, lid, jper, c.dt, c.hi, c.hj, c.hit_cap, c.err);
       NCG_LAUNCHED();
+      // Up to 4,096 slots the event kernel orders the hits itself (a step has tens of
+      // them, thousands in a dense cluster): the host's wait for their number and the
+      // radix passes cost 25 us of a 2,000-body step.  The scratch keys hold 2^19 then,
+      // as many hits as half the hit list.
+      const bool self = lid < 4096 && c.hit_cap == 1 << 20;
       int nh = 0;
-      NCG_CK(cudaMemcpyAsync(&nh, c.scal + S_NHITS, sizeof(int), cudaMemcpyDeviceToHost, st));
-      NCG_CK(cudaStreamSynchronize(st));
-      if (nh > c.hit_cap) return NCGPU_E_CAPACITY;
-      int *si = c.hi + c.hit_cap / 2, *sj = c.hj + c.hit_cap / 2;  // sorted hits (upper halves)
-      if (nh > c.hit_cap / 2) return NCGPU_E_CAPACITY;
-      NCG_TRY(sort_hits(nh, si, sj, lid, st));
+      int *si = c.hi, *sj = c.hj;
+      if (!self) {
+            NCG_CK(cudaMemcpyAsync(&nh, c.scal + S_NHITS, sizeof(int), cudaMemcpyDeviceToHost, st));
+            NCG_CK(cudaStreamSynchronize(st));
+            if (nh > c.hit_cap) return NCGPU_E_CAPACITY;
+            si = c.hi + c.hit_cap / 2;  // sorted hits (upper halves)
+            sj = c.hj + c.hit_cap / 2;
+            if (nh > c.hit_cap / 2) return NCGPU_E_CAPACITY;
+            NCG_TRY(sort_hits(nh, si, sj, lid, st));
+      }
       EvArgs E{lid, c.dt, c.P.par_collision_type, c.P.par_collision_parameter, c.P.par_one_collision_only_bool,
                c.P.par_mesh_bool, c.ev_cap, c.n_max, FragArgs{}};
       if (E.type == NCGPU_COLLISION_FRAGMENTATION && !make_frag_args(c, E.frag)) return NCGPU_E_ARG;
-      k_bf_events<<<1, EVT, 0, st>>>(S, si, sj, E, c.ev, c.evrec, c.dirty, c.dlist, c.err);
-      NCG_LAUNCHED();
-      k_clear_dirty<<<32, 256, 0, st>>>(c.dirty, c.dlist, c.scal);
+      k_bf_events<<<1, EVT, 0, st>>>(S, si, sj, E, c.ev, c.evrec, c.dirty, c.dlist, c.err, !self,
+                                     (unsigned long long *)c.keys2, c.hit_cap / 2);
       NCG_LAUNCHED();
       if (defer && E.type != NCGPU_COLLISION_FRAGMENTATION) return NCGPU_OK;
       return sync_scalars();

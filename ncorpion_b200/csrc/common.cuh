@@ -569,7 +569,7 @@ struct Ctx {
       int *hist = nullptr;         // radix histogram scratch
       size_t hist_cap = 0;
       double *red = nullptr;       // reduction scratch (bbox etc.)
-      unsigned *err = nullptr;     // device error word
+      unsigned *err = nullptr;     // device error word (behind scal)
       double *aos = nullptr;       // 8 * n_max staging for host AoS copies
       double *pinned = nullptr;    // pinned host staging (8 * n_max doubles)
       cudaEvent_t kev0 = nullptr, kev1 = nullptr;  // bracket the dominant kernel

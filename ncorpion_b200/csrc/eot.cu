@@ -257,12 +257,10 @@ int eot_state(int *hm_out)
       k_eot_flag<<<nb, 256, 0, st>>>(S, lid, c.cm, P.par_central_mass_bool, P.par_disruption_threshold,
                                      P.par_high_dumping_threshold, flag);
       NCG_LAUNCHED();
-      int h[S_COUNT];
-      unsigned e = 0;  // the step's device errors come back with the counts
+      int h[S_COUNT + 1];  // the step's device errors come back with the counts
       NCG_CK(cudaMemcpyAsync(h, c.scal, sizeof h, cudaMemcpyDeviceToHost, st));
-      NCG_CK(cudaMemcpyAsync(&e, c.err, sizeof e, cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
-      if (e) NCG_TRY(check_err_word());
+      if (h[S_COUNT]) NCG_TRY(check_err_word());
       c.n_events = h[S_NEV];  // (a collision pass of this step may have left these to us)
       c.collision_count = h[S_CCOUNT];
       mesh_counts_finish(h);
