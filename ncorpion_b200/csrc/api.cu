@@ -206,6 +206,7 @@ int refresh_j2()
       NCG_TRY(state_cm_host(cm9));
       c.j2_prev = c.j2;
       c.j2 = j2_value(c.P, cm9[6], cm9[8]);
+      c.j2_M = cm9[6];
       return NCGPU_OK;
 }
 
@@ -217,12 +218,13 @@ int kick_state()
       c.com_reduced = 0;
       const int nslots = c.largest_id + 1;
       const bool mesh_grav = c.P.par_mesh_bool && !c.force_naive && !c.P.par_mesh_brute_gravity;
-      // the central mass's state on the host: for the tiled gravity's arguments and
-      // the J2 term; mesh gravity and the exact brute force read it from device memory
+      // the central mass's state on the host: for the tiled gravity's arguments; mesh
+      // gravity and the exact brute force read it from device memory, and the J2 term
+      // needs the mass alone, known since the last upload or end of step
       const bool exact = c.P.par_gravity_mode == NCGPU_GRAVITY_EXACT;
       double cm9[9] = {0.};
-      if ((!mesh_grav && !exact) || c.P.par_J2_bool) NCG_TRY(state_cm_host(cm9));
-      const J2Arg j2 = j2_arg(c.P, cm9[6], c.j2);
+      if (!mesh_grav && !exact) NCG_TRY(state_cm_host(cm9));
+      const J2Arg j2 = j2_arg(c.P, c.j2_M, c.j2);
       if (mesh_grav)
             NCG_TRY(mesh_gravity_state(j2));
       else

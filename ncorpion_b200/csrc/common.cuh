@@ -527,6 +527,7 @@ struct Ctx {
       double *cm = nullptr;        // 16 doubles: central mass record (8), SideralOmega at [8]
       double j2 = 0.;              // the J2 in force for the state's kicks (set at upload and end of step)
       double j2_prev = 0.;         // the J2 in force before the last end of step's update
+      double j2_M = 1.;            // the central mass of that upload or end of step (its mass changes there only)
       int com_reduced = 0;         // the last end of step reduced the barycentre
       int eot_lid = -1;            // largest_id at the start of the last end of step
       // output staging (output.cu): snapshot body fields and central body, the
@@ -652,24 +653,29 @@ struct Ctx {
 enum Scal : int {
       S_LID = 0,        // largest_id
       S_NFREE = 1,      // how_many_free
-      S_NHITS = 2,      // hits appended by a sweep
-      S_NEV = 3,        // events of the current sweep
-      S_NDIRTY = 4,     // entries in dlist
-      S_CCOUNT = 5,     // collision_count
-      S_NPAIRS = 6,     // pairs appended (mesh)
-      S_HM = 7,         // how_many_moonlets
-      S_NFLAG = 8,      // bodies flagged for dumping
-      S_NEEDCOM = 9,    // need_to_reduce_COM_bool
-      S_NBIG = 10,      // bodies larger than the mesh size
-      S_NDROP = 11,     // candidates dropped by removals
-      S_NINS = 12,      // bodies inserted in the cell table
-      S_FMERGE = 13,    // merger_count (fragmentation model outcomes, src/structure.h:148-151)
-      S_FSUPER = 14,    // super_catastrophic_count
-      S_FHALF = 15,     // half_fragmentation_count
-      S_FFULL = 16,     // full_fragmentation_count
-      S_NXPAIRS = 17,   // fragment pairs appended by a mesh pass (extra pairs)
-      S_NSKIP = 18,     // mesh event candidates that append no pair of their own
-      S_NFEV = 19,      // full fragmentations of a mesh pass
+      S_CCOUNT = 2,     // collision_count
+      S_HM = 3,         // how_many_moonlets
+      S_NFLAG = 4,      // bodies flagged for dumping
+      S_NEEDCOM = 5,    // need_to_reduce_COM_bool
+      S_FMERGE = 6,     // merger_count (fragmentation model outcomes, src/structure.h:148-151)
+      S_FSUPER = 7,     // super_catastrophic_count
+      S_FHALF = 8,      // half_fragmentation_count
+      S_FFULL = 9,      // full_fragmentation_count
+      // counters of a sweep or pass, cleared together at its start (a brute-force
+      // sweep clears the first three)
+      S_PASS = 10,
+      S_NHITS = 10,     // hits appended by a sweep
+      S_NEV = 11,       // events of the current sweep
+      S_NDIRTY = 12,    // entries in dlist
+      S_NBIG = 13,      // bodies larger than the mesh size
+      S_NDROP = 14,     // candidates dropped by removals
+      S_NINS = 15,      // bodies inserted in the cell table
+      S_NXPAIRS = 16,   // fragment pairs appended by a mesh pass (extra pairs)
+      S_NSKIP = 17,     // mesh event candidates that append no pair of their own
+      S_NFEV = 18,      // full fragmentations of a mesh pass
+      S_V2MAX = 19,     // a mesh pass's largest squared speed (k_mesh_records)
+      S_NCAND = 20,     // a mesh segment's candidates' end
+      S_PASS_END = 21,
       S_COUNT = 24
 };
 
@@ -701,12 +707,13 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cm_host8, con
                  long acc_stride_block, double *d_cm_acc, int mode, cudaStream_t st, int part = 0, int nparts = 1,
                  const double *cm_dev = nullptr);
 
-// Sequential FP64 sums, in index order, of the 3 arrays terms[c*n .. c*n + n),
-// starting from init[c] (0 when init is null); out may alias init.
-int seq_sum3(const double *terms, int n, const double *init, double *out, cudaStream_t st);
+// Sequential FP64 sums, in index order, of the first *n_dev terms (n_dev null: N)
+// of the 3 arrays terms[c*N .. c*N + N), starting from init[c] (0 when init is null);
+// out may alias init.
+int seq_sum3(const double *terms, int N, const int *n_dev, const double *init, double *out, cudaStream_t st);
 // The same sums as a deterministic two-level parallel reduction (non-exact
 // gravity modes), added to init[c] at the end.
-int par_sum3(const double *terms, int n, const double *init, double *out, cudaStream_t st);
+int par_sum3(const double *terms, int N, const int *n_dev, const double *init, double *out, cudaStream_t st);
 
 // tides (src/physics.c:496-542) on the device state after the vector field
 // (tides.cu): acc blocks of n_max and the device CM_acc receive the tidal

@@ -258,7 +258,10 @@ int eot_state(int *hm_out)
                                      P.par_high_dumping_threshold, flag);
       NCG_LAUNCHED();
       int h[S_COUNT + 1];  // the step's device errors come back with the counts
+      double cm9[9];       // and with the fluid-body J2 the central body
+      const bool fluid = P.par_J2_bool && P.par_J2 == 0.;
       NCG_CK(cudaMemcpyAsync(h, c.scal, sizeof h, cudaMemcpyDeviceToHost, st));
+      if (fluid) NCG_CK(cudaMemcpyAsync(cm9, c.cm, sizeof cm9, cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
       if (h[S_COUNT]) NCG_TRY(check_err_word());
       c.n_events = h[S_NEV];  // (a collision pass of this step may have left these to us)
@@ -297,7 +300,15 @@ int eot_state(int *hm_out)
             NCG_LAUNCHED();
       }
       if (changed) NCG_TRY(sync_scalars());
-      if (P.par_J2_bool && P.par_J2 == 0.) NCG_TRY(refresh_j2());  // src/rk4.c:459-463
+      if (fluid) {  // src/rk4.c:459-463
+            if (h[S_NFLAG] > 0) NCG_TRY(state_cm_host(cm9));  // (dumped bodies changed its mass)
+            c.j2_prev = c.j2;
+            c.j2 = j2_value(P, cm9[6], cm9[8]);
+            c.j2_M = cm9[6];
+      } else if (P.par_J2_bool && h[S_NFLAG] > 0) {
+            NCG_TRY(state_cm_host(cm9));
+            c.j2_M = cm9[6];
+      }
       if (hm_out) *hm_out = hm;
       return NCGPU_OK;
 }

@@ -362,15 +362,16 @@ __global__ void __launch_bounds__(1024) k_prep_exact(BodyView bv, int nslots, do
 }
 
 // CM_acc += G*mk*DX/r3 in slot order (src/physics.c:137-139): sequential FP64
-// sums of the 3 arrays cterm[c*n .. c*n + n), in index order, from init[c] (0
+// sums of the 3 arrays cterm[c*N .. c*N + n), in index order, from init[c] (0
 // without init), one CTA (one warp) per component, so the result matches the
 // reference bit for bit.  out may alias init.
-__global__ void __launch_bounds__(32) k_seq_sum3(const double *__restrict__ cterm, int n, const double *init,
-                                                 double *out)
+__global__ void __launch_bounds__(32) k_seq_sum3(const double *__restrict__ cterm, int N,
+                                                 const int *__restrict__ n_dev, const double *init, double *out)
 {
+      const int n = n_dev ? *n_dev : N;
       __shared__ __align__(16) double stage[CHN];
       const int w = blockIdx.x;
-      const double s = warp_chain_sum(cterm + (size_t)w * n, n, init ? init[w] : 0., stage);
+      const double s = warp_chain_sum(cterm + (size_t)w * N, n, init ? init[w] : 0., stage);
       if (threadIdx.x == 0) out[w] = s;
 }
 
@@ -840,12 +841,14 @@ __global__ void __launch_bounds__(256) k_pair_final(PairRun pr, const D4 *__rest
 }
 
 // Deterministic two-level sum of 3 component arrays of length n.
-__global__ void k_sum3_part(const double *__restrict__ v, int n, double *__restrict__ part)
+__global__ void k_sum3_part(const double *__restrict__ v, int N, const int *__restrict__ n_dev,
+                            double *__restrict__ part)
 {
+      const int n = n_dev ? *n_dev : N;
       __shared__ double sh[3][RB];
       double s[3] = {0., 0., 0.};
       for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB)
-            for (int d = 0; d < 3; d++) s[d] += v[(size_t)d * n + i];
+            for (int d = 0; d < 3; d++) s[d] += v[(size_t)d * N + i];
       for (int d = 0; d < 3; d++) sh[d][threadIdx.x] = s[d];
       __syncthreads();
       for (int o = RB / 2; o > 0; o >>= 1) {
@@ -887,20 +890,20 @@ __global__ void k_set3(double *__restrict__ out, double a, double b, double c)
 
 }  // namespace
 
-int par_sum3(const double *terms, int n, const double *init, double *out, cudaStream_t st)
+int par_sum3(const double *terms, int N, const int *n_dev, const double *init, double *out, cudaStream_t st)
 {
       Ctx &c = ctx();
-      const int np = min(128, max(1, (n + RB - 1) / RB));
-      k_sum3_part<<<np, RB, 0, st>>>(terms, n, c.red + 2048);
+      const int np = min(128, max(1, (N + RB - 1) / RB));
+      k_sum3_part<<<np, RB, 0, st>>>(terms, N, n_dev, c.red + 2048);
       NCG_LAUNCHED();
       k_sum3_final<<<1, 96, 0, st>>>(c.red + 2048, np, init, out);
       NCG_LAUNCHED();
       return NCGPU_OK;
 }
 
-int seq_sum3(const double *terms, int n, const double *init, double *out, cudaStream_t st)
+int seq_sum3(const double *terms, int N, const int *n_dev, const double *init, double *out, cudaStream_t st)
 {
-      k_seq_sum3<<<3, 32, 0, st>>>(terms, n, init, out);
+      k_seq_sum3<<<3, 32, 0, st>>>(terms, N, n_dev, init, out);
       NCG_LAUNCHED();
       return NCGPU_OK;
 }
@@ -953,7 +956,7 @@ int exact_field(const BodyView &bv, int nslots, const CmArg &cm, double G, doubl
 int finish_cm(int central, int n, double *d_cm_acc, cudaStream_t st)
 {
       Ctx &c = ctx();
-      if (central) return par_sum3(c.cmterm, n, nullptr, d_cm_acc, st);
+      if (central) return par_sum3(c.cmterm, n, nullptr, nullptr, d_cm_acc, st);
       k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
       NCG_LAUNCHED();
       return NCGPU_OK;

@@ -61,6 +61,7 @@ __global__ void k_mesh_keys(DevState S, int lid, double gam, double half, int d,
       ckey[k] = (int)L;
       keys[k] = L >= 0 ? (uint32_t)L : NOKEY;
       vals[k] = k;
+      if (k == lid) keys[lid + 1] = NOKEY;  // the sentinel behind the sorted keys
 }
 
 __global__ void k_cell_heads(const uint32_t *__restrict__ keys, int n, int2 *__restrict__ crange,
@@ -91,19 +92,26 @@ __global__ void k_cell_clear(const uint32_t *__restrict__ keys, int n, int2 *__r
 // Cell-ordered copy of the fields the pass reads: record q is body vals[q];
 // pv[q] is vals[q] for an existing body, INT_MAX otherwise, so that "p < k and
 // p exists" is one compact load (pv[q] < k).
+// *v2max: the largest high word of the existing bodies' squared speeds (at least
+// infinity's when one is not finite).
 __global__ void k_mesh_records(const DevState S, const int *__restrict__ vals, int n, MRec *__restrict__ rec,
-                               int *__restrict__ pv)
+                               int *__restrict__ pv, unsigned *__restrict__ v2max)
 {
       int q = blockIdx.x * blockDim.x + threadIdx.x;
-      if (q >= n) return;
-      const int b = vals[q];
-      MRec r;
-      r.x = S.x[b]; r.y = S.y[b]; r.z = S.z[b]; r.R = S.R[b];
-      r.vx = S.vx[b]; r.vy = S.vy[b]; r.vz = S.vz[b];
-      r.ex = S.ex[b];
-      r.did = S.did[b];
-      rec[q] = r;
-      pv[q] = r.ex ? b : 0x7fffffff;
+      unsigned h = 0;
+      if (q < n) {
+            const int b = vals[q];
+            MRec r;
+            r.x = S.x[b]; r.y = S.y[b]; r.z = S.z[b]; r.R = S.R[b];
+            r.vx = S.vx[b]; r.vy = S.vy[b]; r.vz = S.vz[b];
+            r.ex = S.ex[b];
+            r.did = S.did[b];
+            rec[q] = r;
+            pv[q] = r.ex ? b : 0x7fffffff;
+            if (r.ex) h = (unsigned)__double2hiint(r.vx * r.vx + r.vy * r.vy + r.vz * r.vz) & 0x7fffffffu;
+      }
+      h = __reduce_max_sync(0xffffffffu, h);
+      if ((threadIdx.x & 31) == 0 && h > *v2max) atomicMax(v2max, h);
 }
 
 // The 27 neighbour cells as 9 rows of three consecutive linear indices
@@ -139,36 +147,47 @@ __global__ void k_mesh_count(const int *__restrict__ pv, const int *__restrict__
 
 // Candidates of body k in pop order; hit flag from the entry-state predicate.
 //
-// The warp's 32 bodies (consecutive in cell order) share the work: each lane
-// queues the positions of every body in its 27 cells, in pop order (rows 8..0,
-// cells x + 1 .. x - 1, each cell's bodies in ascending index), into shared
-// memory; then the warp takes the queued entries 32 at a time, each lane one
-// entry whatever list it belongs to.  An entry is a candidate when its body p
-// has a lower index than the list's owner k and exists; its position is the
-// owner's offset plus the number of the owner's candidates before it (a ballot
-// over the round, plus a running count per owner), so the lists come out in
-// the reference's order.  The candidates of one list are written by adjacent
-// lanes (coalesced stores) and the FP64 predicates run with every lane busy.
-// A lane whose queue is full walks again in the next round, queueing the
-// entries after those already taken.
-constexpr int MWW = 4;   // warps per block
-constexpr int MWQ = 32;  // queued entries per lane and round
+// Each lane walks its body's 27 cells in pop order (rows 8..0, cells x + 1 ..
+// x - 1, each cell's bodies in ascending index) and queues the positions of the
+// candidates -- existing bodies of lower index -- in shared memory.  Then the warp
+// takes the queued candidates 32 at a time, each lane one whatever list it belongs
+// to: its place is the owner's offset plus its number in the owner's queue, so the
+// lists come out in the reference's order, written by adjacent lanes (coalesced
+// stores), and the FP64 predicates run with every lane busy.  A lane whose queue is
+// full walks again in the next round, queueing the candidates after those taken.
+// The predicate's full records are read only for pairs that can touch within dt: the
+// distance, from the records' first 32 bytes, is compared with the radii plus the way
+// that any two bodies can close (twice the largest speed; the margin of 1e-6 is far
+// above the predicate's rounding, about 1e-8 of the same lengths).
+// Bound by latency: of 400 us for 13 million candidates the walk takes 190, the
+// partners' positions 100 and the lists' scattered stores 110.  Queueing every body of
+// the cells and telling the candidates apart in the balanced loop took twice its
+// rounds, with a ballot and running counts in each, and whole records for every pair:
+// a step of the 1,048,576-body disk 358 us, now 264 (more CTAs an SM, of fewer
+// registers, spill; two rounds at once are 25 % slower).
+constexpr int MWW = 4;        // warps per block
+constexpr int MWQ = 32;       // queued candidates per lane and round
+constexpr int MWS = MWQ + 1;  // a lane's row (the pad keeps the lanes off each other's banks)
 
-__global__ void __launch_bounds__(MWW * 32) k_mesh_write(const MRec *__restrict__ rec, const int *__restrict__ ckey,
+__global__ void __launch_bounds__(MWW * 32, 8) k_mesh_write(const MRec *__restrict__ rec, const int *__restrict__ ckey,
                                                         const int *__restrict__ vals, const int *__restrict__ pv,
                                                         const int2 *__restrict__ crange,
                                                         const int *__restrict__ off, int lid, int lo, int hi, int d,
-                                                        long long cap, double dt, int test, int *__restrict__ ck,
+                                                        long long cap, const unsigned *__restrict__ v2max, double dt,
+                                                        int test, int *__restrict__ ck,
                                                         int *__restrict__ cp, unsigned char *__restrict__ cflag,
                                                         int *__restrict__ hitpos, int hit_cap, int *__restrict__ nhits,
-                                                        long pair_cap, unsigned *err)
+                                                        long pair_cap, unsigned *err, int *__restrict__ n_end)
 {
-      __shared__ int qb[MWW][32 * MWQ];
+      __shared__ int qb[MWW][32 * MWS];
       __shared__ unsigned char owner[MWW][32 * MWQ];
-      __shared__ int pre[MWW][32], run[MWW][32], okk[MWW][32], opos[MWW][32];
-      __shared__ MRec orec[MWW][32];  // the lists' owners' records
+      __shared__ int pre[MWW][32], okk[MWW][32], opos[MWW][32];
       const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
       const int t = blockIdx.x * blockDim.x + threadIdx.x;  // cell order, as k_mesh_count
+      const int t0 = t - lane;                               // the warp's first record
+      if (t == 0) *n_end = off[lid + 1];
+      // no two bodies close in by more than this within dt (inf or NaN: no bound)
+      const double reach = 2. * sqrt(__hiloint2double((int)*v2max + 1, 0)) * fmax(dt, 0.);
       int k = -1, L = -1;
       if (t <= lid) {
             k = vals[t];
@@ -176,33 +195,34 @@ __global__ void __launch_bounds__(MWW * 32) k_mesh_write(const MRec *__restrict_
       }
       bool dk = false;
       if (L >= 0) {
-            const MRec rk = load_mrec(rec, t);
-            orec[w][lane] = rk;
-            dk = test && rk.did;
+            dk = test && rec[t].did;
             opos[w][lane] = off[k];
       }
       okk[w][lane] = (L >= 0 ? k : -1) | (dk ? 0x80000000 : 0);
-      run[w][lane] = 0;
       const long long dd = (long long)d * d;
       int skip = 0;
       bool more = L >= 0;
       while (__any_sync(0xffffffffu, more)) {
             int cnt = 0;
             if (more) {
-                  int idx = 0;
+                  int idx = -skip;
 #pragma unroll 1
                   for (int r = 8; r >= 0; --r) {
                         int2 cr[3];
                         row_cells(crange, d_row(L, r, d, dd), cap, cr);
-#pragma unroll
-                        for (int x = 2; x >= 0; --x) {  // cells mid + 1, mid, mid - 1
-                              const int a = max(cr[x].x, cr[x].x + skip - idx), b = min(cr[x].y, cr[x].x + skip + MWQ - idx);
-                              for (int q = a; q < b; ++q) qb[w][lane * MWQ + idx + (q - cr[x].x) - skip] = q;
-                              if (cr[x].x >= 0) idx += cr[x].y - cr[x].x;
+                        // cells mid + 1, mid, mid - 1 in one loop
+                        const int n2 = cr[2].y - cr[2].x, n1 = n2 + cr[1].y - cr[1].x, n0 = n1 + cr[0].y - cr[0].x;
+#pragma unroll 1
+                        for (int i = 0; i < n0; ++i) {
+                              const int q = i + (i < n2 ? cr[2].x : i < n1 ? cr[1].x - n2 : cr[0].x - n1);
+                              if (pv[q] < k) {  // (a body removed earlier in the pass is not pushed)
+                                    if (idx >= 0 && idx < MWQ) qb[w][lane * MWS + idx] = q;
+                                    ++idx;
+                              }
                         }
                   }
-                  cnt = min(max(idx - skip, 0), MWQ);
-                  more = idx > skip + MWQ;
+                  cnt = min(max(idx, 0), MWQ);
+                  more = idx > MWQ;
             }
             int incl = cnt;
             for (int o = 1; o < 32; o <<= 1) {
@@ -214,47 +234,38 @@ __global__ void __launch_bounds__(MWW * 32) k_mesh_write(const MRec *__restrict_
             pre[w][lane] = mine;
             for (int j = 0; j < cnt; ++j) owner[w][mine + j] = (unsigned char)lane;
             __syncwarp();
-            for (int f0 = 0; f0 < total; f0 += 32) {
-                  const int fi = f0 + lane;
-                  int o = -1, q = 0, p = 0, kk = -1;
-                  bool cand = false;
-                  if (fi < total) {
-                        o = owner[w][fi];
-                        q = qb[w][o * MWQ + fi - pre[w][o]];
-                        kk = okk[w][o] & 0x7fffffff;
-                        p = pv[q];
-                        cand = p < kk;  // (a body removed earlier in the pass is not pushed)
+            for (int fi = lane; fi < total; fi += 32) {
+                  const int o = owner[w][fi], i = fi - pre[w][o];
+                  const int q = qb[w][o * MWS + i];
+                  const long pos = (long)opos[w][o] + skip + i;
+                  if (pos >= pair_cap) {
+                        atomicOr(err, ERR_CAPACITY);
+                        continue;
                   }
-                  const unsigned m = __ballot_sync(0xffffffffu, cand);
-                  // this entry's list starts at lane a of the round (the lists are contiguous, in lane order)
-                  const int a = o >= 0 ? max(pre[w][o] - f0, 0) : 0;
-                  const unsigned below = (1u << lane) - 1u, from_a = ~((1u << a) - 1u);
-                  const int nb = o >= 0 ? run[w][o] + __popc(m & below & from_a) : 0;
-                  const int on = __shfl_down_sync(0xffffffffu, o, 1);
-                  __syncwarp();
-                  if (o >= 0 && (lane == 31 || on != o))  // the list's last entry in this round: its running count
-                        run[w][o] += __popc(m & from_a & (lane == 31 ? 0xffffffffu : ((2u << lane) - 1u)));
-                  if (cand) {
-                        const long pos = (long)opos[w][o] + nb;
-                        if (pos >= pair_cap) {
-                              atomicOr(err, ERR_CAPACITY);
-                        } else {
-                              ck[pos] = kk;
-                              cp[pos] = p;
-                              unsigned char f = 0;
+                  const int kk = okk[w][o];
+                  ck[pos] = kk & 0x7fffffff;
+                  cp[pos] = pv[q];
+                  unsigned char f = 0;
+                  if (test && kk >= 0) {
+                        // the positions and radii first: one 32-byte sector of each record
+                        const double2 *hp = reinterpret_cast<const double2 *>(rec + q);
+                        const double2 *hk = reinterpret_cast<const double2 *>(rec + t0 + o);
+                        const double2 pxy = hp[0], pz = hp[1], kxy = hk[0], kz = hk[1];
+                        const double dx = pxy.x - kxy.x, dy = pxy.y - kxy.y, dz = pz.x - kz.x;
+                        const double far = (fabs(pz.y + kz.y) + reach) * (1. + 1e-6);
+                        if (!(dx * dx + dy * dy + dz * dz > far * far)) {  // (true for NaN)
                               const MRec rp = load_mrec(rec, q);
-                              if (test && !(okk[w][o] & 0x80000000) && !rp.did &&
-                                  d_contact_rec(rp, orec[w][o], dt)) {  // closest_approach(p, k)
+                              if (!rp.did && d_contact_rec(rp, load_mrec(rec, t0 + o), dt)) {  // closest_approach(p, k)
                                     f = 1;
-                                    int h = atomicAdd(nhits, 1);
+                                    const int h = atomicAdd(nhits, 1);
                                     if (h < hit_cap) hitpos[h] = (int)pos;
                                     else atomicOr(err, ERR_CAPACITY);
                               }
-                              cflag[pos] = f;
                         }
                   }
-                  __syncwarp();
+                  cflag[pos] = f;
             }
+            __syncwarp();
             skip += MWQ;
       }
 }
@@ -770,7 +781,8 @@ static int mesh_segment_launch(const DevState &S, int lid, int lo, int hi, long 
       const int nb = (n + 255) / 256;
       const int d = c.P.par_collision_cube_cells;
       MRec *rec = (MRec *)c.mrec;
-      k_mesh_records<<<nb, 256, 0, st>>>(S, c.mvals, n, rec, c.mpv);
+      unsigned *v2max = (unsigned *)(c.scal + S_V2MAX);  // (the pass's maximum: it bounds every segment's)
+      k_mesh_records<<<nb, 256, 0, st>>>(S, c.mvals, n, rec, c.mpv, v2max);
       NCG_LAUNCHED();
       k_mesh_count<<<nb, 256, 0, st>>>(c.mpv, c.ckey, c.mvals, c.crange, lid, lo, hi, d,
                                        (long long)c.cell_cap, c.mcnt);
@@ -780,12 +792,12 @@ static int mesh_segment_launch(const DevState &S, int lid, int lo, int hi, long 
             k_add_base<<<(n + 256) / 256, 256, 0, st>>>(c.moff, n, (int)base);
             NCG_LAUNCHED();
       }
-      NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, sizeof(int), st));
+      if (base > 0) NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, sizeof(int), st));
       // (positions at or past pair_cap are not written: the kernel records the
       // overflow and the host returns NCGPU_E_CAPACITY)
-      k_mesh_write<<<(n + MWW * 32 - 1) / (MWW * 32), MWW * 32, 0, st>>>(rec, c.ckey, c.mvals, c.mpv, c.crange, c.moff, lid, lo, hi, d,
-                                       (long long)c.cell_cap, c.dt, test, c.cand_k, c.cand_p, c.cflag, c.hi, c.hit_cap,
-                                       c.scal + S_NHITS, c.pair_cap, c.err);
+      k_mesh_write<<<(n + MWW * 32 - 1) / (MWW * 32), MWW * 32, 0, st>>>(
+          rec, c.ckey, c.mvals, c.mpv, c.crange, c.moff, lid, lo, hi, d, (long long)c.cell_cap, v2max, c.dt, test,
+          c.cand_k, c.cand_p, c.cflag, c.hi, c.hit_cap, c.scal + S_NHITS, c.pair_cap, c.err, c.scal + S_NCAND);
       NCG_LAUNCHED();
       return NCGPU_OK;
 }
@@ -826,11 +838,10 @@ static int mesh_segment(const DevState &S, int lid, int lo, int hi, long base, i
 {
       Ctx &c = ctx();
       NCG_TRY(mesh_segment_launch(S, lid, lo, hi, base, test));
-      int h2[2] = {0, 0};  // candidates' end, hits
-      NCG_CK(cudaMemcpyAsync(&h2[0], c.moff + lid + 1, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-      NCG_CK(cudaMemcpyAsync(&h2[1], c.scal + S_NHITS, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+      int h[S_COUNT];
+      NCG_CK(cudaMemcpyAsync(h, c.scal, sizeof h, cudaMemcpyDeviceToHost, c.s));
       NCG_CK(cudaStreamSynchronize(c.s));
-      return mesh_segment_finish(S, lid, hi, base, h2[0], h2[1], E0, tot);
+      return mesh_segment_finish(S, lid, hi, base, h[S_NCAND], h[S_NHITS], E0, tot);
 }
 
 // Cell table of the bodies' insertion cells (ckey -> sorted keys, heads).
@@ -839,7 +850,6 @@ static int mesh_table(int n)
       Ctx &c = ctx();
       cudaStream_t st = c.s;
       NCG_TRY(radix_sort_pairs(c.mkeys, c.mvals, n, 32, st));
-      NCG_CK(cudaMemsetAsync(c.mkeys + n, 0xff, sizeof(uint32_t), st));
       k_cell_heads<<<(n + 255) / 256, 256, 0, st>>>(c.mkeys, n, c.crange, c.scal + S_NINS);
       NCG_LAUNCHED();
       return NCGPU_OK;
@@ -872,9 +882,7 @@ int mesh_pass(double gam, int test, bool defer)
       const int lid = c.largest_id;
       const int n = lid + 1;
       // counters of the pass cleared on the device (no host copy on the step's path)
-      NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, 2 * sizeof(int), st));    // NHITS, NEV
-      NCG_CK(cudaMemsetAsync(c.scal + S_NBIG, 0, 3 * sizeof(int), st));     // NBIG, NDROP, NINS
-      NCG_CK(cudaMemsetAsync(c.scal + S_NXPAIRS, 0, 3 * sizeof(int), st));  // NXPAIRS, NSKIP, NFEV
+      NCG_CK(cudaMemsetAsync(c.scal + S_PASS, 0, (S_PASS_END - S_PASS) * sizeof(int), st));
       c.n_cand = c.n_pairs = 0;
       c.total_neighbours = 0;
       c.how_many_small = c.how_many_big = 0;
@@ -893,12 +901,10 @@ int mesh_pass(double gam, int test, bool defer)
       // candidates' end and the hits, one synchronisation); with such bodies
       // the segmented pass below starts over
       NCG_TRY(mesh_segment_launch(S, lid, 0, lid + 1, 0, test));
-      int h3[3] = {0, 0, 0};  // bodies larger than the mesh size, candidates' end, hits
-      NCG_CK(cudaMemcpyAsync(&h3[0], c.scal + S_NBIG, sizeof(int), cudaMemcpyDeviceToHost, st));
-      NCG_CK(cudaMemcpyAsync(&h3[1], c.moff + n, sizeof(int), cudaMemcpyDeviceToHost, st));
-      NCG_CK(cudaMemcpyAsync(&h3[2], c.scal + S_NHITS, sizeof(int), cudaMemcpyDeviceToHost, st));
+      int hp[S_COUNT];  // bodies larger than the mesh size, candidates' end, hits
+      NCG_CK(cudaMemcpyAsync(hp, c.scal, sizeof hp, cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
-      const int nbig = h3[0];
+      const int nbig = hp[S_NBIG];
       MeshEvArgs E{lid, d, c.P.par_collision_type, c.P.par_one_collision_only_bool, c.P.par_mesh_bool, c.ev_cap,
                    c.n_max, c.occ_cap, n, (long long)c.cell_cap, c.dt, c.P.par_collision_parameter,
                    c.P.par_mutual_bool, c.xpair_cap, FragArgs{}, lid + 1};
@@ -917,7 +923,7 @@ int mesh_pass(double gam, int test, bool defer)
       };
       if (!test || nbig == 0) {
             int tot = 0;
-            NCG_TRY(mesh_segment_finish(S, lid, lid + 1, 0, h3[1], h3[2], E, &tot));
+            NCG_TRY(mesh_segment_finish(S, lid, lid + 1, 0, hp[S_NCAND], hp[S_NHITS], E, &tot));
             base = small_total = tot;
       } else {
             int s = 0;

@@ -538,15 +538,16 @@ __global__ void k_mesh_grav(DevState S, MGArgs A, const int *__restrict__ ckey, 
 // (the cell relation is symmetric, the reference's index aliasing included),
 // and the sum over them is taken in any fixed order.  The three cells of a row
 // (x - 1, x, x + 1) are consecutive linear indices, hence one contiguous range
-// of the cell-sorted bodies: a body walks 9 ranges.  The warp's bodies queue
-// their partners (record positions, per lane in shared memory) during the
-// walk; then the warp evaluates the queued pair terms 32 at a time, every lane
-// busy whatever the lengths of the bodies' lists.  A round's terms of one body
-// sit in adjacent lanes: a segmented scan over the warp (five shuffle steps)
-// leaves each list's sum in its last lane, which the body adds to its own sums
-// (a fixed order: deterministic).  The pair term is FP64 with one
-// reciprocal square root (G m dx / D^3 = G m dx (1/D)^3); against the exact
-// mode, only its rounding and the order of the sum differ.
+// of the cell-sorted bodies: a body walks 9 ranges.  Each lane queues its body's
+// partners (record positions) in shared memory during the walk, then sums its own
+// queue: the walk's ragged rows (0 to 6 bodies each) are flattened into one loop whose
+// length is the longest of the warp's lists, and the sums need no exchange (a fixed
+// order: deterministic).  The pair term is FP64 with one reciprocal square root
+// (G m dx / D^3 = G m dx (1/D)^3); against the exact mode, only its rounding and the
+// order of the sum differ.  Bound by the FP64 pipe and the gathers' latency.  Sharing
+// a warp's queued terms out 32 at a time keeps every lane busy, but the owners' sums
+// then take 36 shuffles a round, more than the idle lanes cost: 294 us at 1,048,576
+// bodies, now 191 (with the 12 chain sums' 120 shuffles a warp brought to 26).
 constexpr int FGW = 4;   // warps per block
 constexpr int FGQ = 32;  // queued partners per lane and round
 
@@ -572,6 +573,27 @@ __device__ __forceinline__ void term_fast(double xb, double yb, double zb, doubl
       tz = w * dz;
 }
 
+// The sums over the warp of 12 values a lane, each in one lane: halves of the values
+// change sides with halves of the warp (6 + 3 + 2 + 1 + 1 exchanges, where one value
+// at a time takes 5 each).  Lane l returns the sum of value idx(l) (-1: none).
+__device__ __forceinline__ double warp_sum12(const double (&v)[12], int lane, int &idx)
+{
+      double a[6], b[3], c[2];
+      const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+#pragma unroll
+      for (int q = 0; q < 6; q++)
+            a[q] = (h16 ? v[q + 6] : v[q]) + __shfl_xor_sync(0xffffffffu, h16 ? v[q] : v[q + 6], 16);
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+            b[q] = (h8 ? a[q + 3] : a[q]) + __shfl_xor_sync(0xffffffffu, h8 ? a[q] : a[q + 3], 8);
+      c[0] = (h4 ? b[2] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[2], 4);
+      c[1] = (h4 ? 0. : b[1]) + __shfl_xor_sync(0xffffffffu, h4 ? b[1] : 0., 4);
+      double s = (h2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, h2 ? c[0] : c[1], 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      idx = (h4 && h2) || (lane & 1) ? -1 : (h16 ? 6 : 0) + (h8 ? 3 : 0) + (h4 ? 2 : h2 ? 1 : 0);
+      return s;
+}
+
 __global__ void __launch_bounds__(FGW * 32, 8) k_mesh_grav_fast(DevState S, MGArgs A, const uint32_t *__restrict__ keys,
                                                                const int *__restrict__ vals,
                                                                const int2 *__restrict__ crange,
@@ -582,12 +604,9 @@ __global__ void __launch_bounds__(FGW * 32, 8) k_mesh_grav_fast(DevState S, MGAr
                                                                double *__restrict__ cpart)
 {
       __shared__ int qb[FGW][32 * FGQ];
-      __shared__ unsigned char owner[FGW][32 * FGQ];
-      __shared__ int pre[FGW][32];
       __shared__ double csum[12][FGW];
       const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
       const int t = blockIdx.x * blockDim.x + threadIdx.x;  // cell order
-      const int t0 = t - lane;                               // the warp's first record
       const bool act = t <= A.lid;
       const int b = act ? vals[t] : 0;
       GRec me;
@@ -605,11 +624,9 @@ __global__ void __launch_bounds__(FGW * 32, 8) k_mesh_grav_fast(DevState S, MGAr
             } else {
                   for (int c = 0; c < 12; c++) tv[c] = 0.;
             }
-            for (int c = 0; c < 12; c++) {
-                  double v = tv[c];
-                  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                  if (lane == 0) csum[c][w] = v;
-            }
+            int ci;
+            const double cs = warp_sum12(tv, lane, ci);
+            if (ci >= 0) csum[ci][w] = cs;
             __syncthreads();
             if (threadIdx.x < 12) {
                   double v = 0.;
@@ -620,73 +637,31 @@ __global__ void __launch_bounds__(FGW * 32, 8) k_mesh_grav_fast(DevState S, MGAr
       const uint32_t L = act ? keys[t] : 0xffffffffu;
       walk = walk && L != 0xffffffffu;  // outside the collision cube: no pairs
       const long long dd = (long long)A.d * A.d;
+      int *list = qb[w] + lane;  // entry i at list[32 i]: no bank conflicts
       int skip = 0;
       bool more = walk;
-      while (__any_sync(0xffffffffu, more)) {
-            int cnt = 0;
-            if (more) {
-                  int idx = 0;
+      while (more) {
+            int idx = -skip;
 #pragma unroll 1
-                  for (int r = 0; r < 9; ++r) {
-                        int s0, e0;
-                        if (!row_range(crange, d_row(L, r, A.d, dd), A.cell_cap, &s0, &e0)) continue;
-                        for (int q = s0; q < e0; ++q) {
-                              if (q == t) continue;  // (bodies 0..2 and removed ones add zero terms)
-                              if (idx >= skip && idx < skip + FGQ) qb[w][lane * FGQ + idx - skip] = q;
-                              ++idx;
-                        }
-                  }
-                  cnt = min(idx - skip, FGQ);
-                  more = idx > skip + FGQ;
-            }
-            int incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                  const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                  if (lane >= o) incl += u;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            const int mine = incl - cnt;
-            pre[w][lane] = mine;
-            for (int j = 0; j < cnt; ++j) owner[w][mine + j] = (unsigned char)lane;
-            __syncwarp();
-            for (int f0 = 0; f0 < total; f0 += 32) {
-                  const int fi = f0 + lane;
-                  double tx = 0., ty = 0., tz = 0.;
-                  int a = lane;  // the lane where this entry's list starts in the round
-                  if (fi < total) {
-                        const int o = owner[w][fi];
-                        const int q = qb[w][o * FGQ + fi - pre[w][o]];
-                        const double2 *ow = reinterpret_cast<const double2 *>(grec + t0 + o);
-                        const double2 oxy = ow[0], oz = ow[1];
-                        term_fast(oxy.x, oxy.y, oz.x, A.soft ? grec[t0 + o].R : 0., gp, grec, q, A, tx, ty, tz);
-                        a = max(pre[w][o] - f0, 0);
-                  }
-                  // segmented inclusive scan over the round (the lists are contiguous in
-                  // lane order): the last lane of a list then holds the list's sum
-#pragma unroll
-                  for (int dl = 1; dl < 32; dl <<= 1) {
-                        const double ux = __shfl_up_sync(0xffffffffu, tx, dl);
-                        const double uy = __shfl_up_sync(0xffffffffu, ty, dl);
-                        const double uz = __shfl_up_sync(0xffffffffu, tz, dl);
-                        if (lane - dl >= a) {
-                              tx += ux;
-                              ty += uy;
-                              tz += uz;
-                        }
-                  }
-                  // each body takes its list's sum of this round from the list's last lane
-                  const int i0 = max(mine, f0), i1 = min(mine + cnt, f0 + 32);
-                  const int src = i1 > i0 ? i1 - 1 - f0 : lane;
-                  const double sx = __shfl_sync(0xffffffffu, tx, src);
-                  const double sy = __shfl_sync(0xffffffffu, ty, src);
-                  const double sz = __shfl_sync(0xffffffffu, tz, src);
-                  if (i1 > i0) {
-                        a_x += sx;
-                        a_y += sy;
-                        a_z += sz;
+            for (int r = 0; r < 9; ++r) {
+                  int s0, e0;
+                  if (!row_range(crange, d_row(L, r, A.d, dd), A.cell_cap, &s0, &e0)) continue;
+                  for (int q = s0; q < e0; ++q) {
+                        if (q == t) continue;  // (bodies 0..2 and removed ones add zero terms)
+                        if (idx >= 0 && idx < FGQ) list[32 * idx] = q;
+                        ++idx;
                   }
             }
-            __syncwarp();
+            const int cnt = min(idx, FGQ);
+            more = idx > FGQ;
+#pragma unroll 2
+            for (int i = 0; i < cnt; ++i) {
+                  double tx, ty, tz;
+                  term_fast(me.x, me.y, me.z, me.R, gp, grec, list[32 * i], A, tx, ty, tz);
+                  a_x += tx;
+                  a_y += ty;
+                  a_z += tz;
+            }
             skip += FGQ;
       }
       if (walk || (act && me.ex && b > 2)) {

@@ -51,14 +51,15 @@ __device__ __forceinline__ double tide_step(const double *r, double W, double Dt
       return DADD(W, div_by_recip(DMUL(r[RCQ], DSUB(DMUL(r[RX], aY), DMUL(r[RY], aX))), r[RS], r[RYS]));
 }
 
-__global__ void k_tides_prep(DevState S, const int *__restrict__ cidx, int n, const double *__restrict__ cm,
+__global__ void k_tides_prep(DevState S, const int *__restrict__ cidx, int N, const int *__restrict__ n_dev,
+                             const double *__restrict__ cm,
                              const double *__restrict__ cm_acc, const double *__restrict__ ax,
                              const double *__restrict__ ay, double *__restrict__ az, double dt, double A, double Dt,
                              double moi, double R, double *__restrict__ rec, double *__restrict__ terms,
                              double *__restrict__ aout, int *__restrict__ first)
 {
       const int q = blockIdx.x * blockDim.x + threadIdx.x;
-      if (q >= n) return;
+      if (q >= *n_dev) return;
       const int k = cidx[q];
       const double M = cm[6];
       const double X = DSUB(S.x[k], cm[0]), Y = DSUB(S.y[k], cm[1]), Z = DSUB(S.z[k], cm[2]);
@@ -77,7 +78,7 @@ __global__ void k_tides_prep(DevState S, const int *__restrict__ cidx, int n, co
       // aZ = S*K*(r2*Z + Delta_t*(2.*rv*Z + r2*vZ)): no SideralOmega in it
       const double aZ = DMUL(SK, DADD(DMUL(r2, Z), DMUL(Dt, DADD(DMUL(tr, Z), DMUL(r2, vZ)))));
       az[k] = DSUB(az[k], aZ);
-      terms[2 * (size_t)n + q] = DDIV(DMUL(aZ, m), M);
+      terms[2 * (size_t)N + q] = DDIV(DMUL(aZ, m), M);
       double *r = rec + (size_t)TREC * q;
       r[RX] = X;
       r[RY] = Y;
@@ -107,9 +108,11 @@ constexpr int TPER = TBK * TREC / 32;   // doubles each lane stages per block
 // The SideralOmega recurrence in slot order (one warp) from the first body
 // whose step changes the rotation (none: nothing to do); writes (a_x, a_y) of
 // those bodies to aout and the final SideralOmega to cm[8].
-__global__ void __launch_bounds__(32) k_tides_chain(const double *__restrict__ rec, int n, double Dt, double *cm,
-                                                    double *__restrict__ aout, const int *__restrict__ first)
+__global__ void __launch_bounds__(32) k_tides_chain(const double *__restrict__ rec, const int *__restrict__ n_dev,
+                                                    double Dt, double *cm, double *__restrict__ aout,
+                                                    const int *__restrict__ first)
 {
+      const int n = *n_dev;
       __shared__ __align__(16) double st[TBK * TREC];
       __shared__ double ob[2 * TBK];
       const int lane = threadIdx.x;
@@ -148,19 +151,20 @@ __global__ void __launch_bounds__(32) k_tides_chain(const double *__restrict__ r
       if (lane == 0) cm[8] = W;
 }
 
-__global__ void k_tides_apply(DevState S, const int *__restrict__ cidx, int n, const double *__restrict__ cm,
+__global__ void k_tides_apply(DevState S, const int *__restrict__ cidx, int N, const int *__restrict__ n_dev,
+                              const double *__restrict__ cm,
                               const double *__restrict__ aout, double *__restrict__ ax, double *__restrict__ ay,
                               double *__restrict__ terms)
 {
       const int q = blockIdx.x * blockDim.x + threadIdx.x;
-      if (q >= n) return;
+      if (q >= *n_dev) return;
       const int k = cidx[q];
       const double aX = aout[2 * (size_t)q], aY = aout[2 * (size_t)q + 1];
       const double m = S.m[k], M = cm[6];
       ax[k] = DSUB(ax[k], aX);
       ay[k] = DSUB(ay[k], aY);
       terms[q] = DDIV(DMUL(aX, m), M);
-      terms[(size_t)n + q] = DDIV(DMUL(aY, m), M);
+      terms[(size_t)N + q] = DDIV(DMUL(aY, m), M);
 }
 
 }  // namespace
@@ -170,29 +174,29 @@ int tides_state(double *d_acc, long bs, double *d_cm_acc)
       Ctx &c = ctx();
       const ncgpu_params &P = c.P;
       cudaStream_t st = c.s;
-      int n = 0;
-      NCG_TRY(compact_existing(c.ex, c.largest_id, &n, st));
-      if (n == 0) return NCGPU_OK;
-      NCG_TRY(ensure_partial((size_t)(TREC + 2 + 3) * n + 1));
-      double *rec = c.partial, *aout = rec + (size_t)TREC * n, *terms = aout + 2 * (size_t)n;
-      int *first = (int *)(terms + 3 * (size_t)n);  // first body whose step changes the rotation
+      const int N = c.largest_id + 1;  // (the existing bodies' count stays on the device)
+      if (N <= 0) return NCGPU_OK;
+      NCG_TRY(compact_existing_dev(c.ex, c.largest_id, st));
+      NCG_TRY(ensure_partial((size_t)(TREC + 2 + 3) * N + 1));
+      double *rec = c.partial, *aout = rec + (size_t)TREC * N, *terms = aout + 2 * (size_t)N;
+      int *first = (int *)(terms + 3 * (size_t)N);  // first body whose step changes the rotation
       NCG_CK(cudaMemsetAsync(first, 0x7f, sizeof(int), st));
       const double R = P.par_R_unit;
       const double R5 = R * R * R * R * R;
       const double A = 3. * P.par_k2 * P.par_G * R5;  // src/physics.c:505-506
       double *ax = d_acc, *ay = d_acc + bs, *az = d_acc + 2 * bs;
       DevState S = dev_state();
-      const int nb = (n + 255) / 256;
-      k_tides_prep<<<nb, 256, 0, st>>>(S, c.cidx, n, c.cm, d_cm_acc, ax, ay, az, c.dt, A, P.par_Delta_t,
+      const int nb = (N + 255) / 256;
+      k_tides_prep<<<nb, 256, 0, st>>>(S, c.cidx, N, c.n_dev, c.cm, d_cm_acc, ax, ay, az, c.dt, A, P.par_Delta_t,
                                        P.par_dimensionless_moi, R, rec, terms, aout, first);
       NCG_LAUNCHED();
-      k_tides_chain<<<1, 32, 0, st>>>(rec, n, P.par_Delta_t, c.cm, aout, first);
+      k_tides_chain<<<1, 32, 0, st>>>(rec, c.n_dev, P.par_Delta_t, c.cm, aout, first);
       NCG_LAUNCHED();
-      k_tides_apply<<<nb, 256, 0, st>>>(S, c.cidx, n, c.cm, aout, ax, ay, terms);
+      k_tides_apply<<<nb, 256, 0, st>>>(S, c.cidx, N, c.n_dev, c.cm, aout, ax, ay, terms);
       NCG_LAUNCHED();
       // CM_acc += a m / M: in slot order (exact mode), or a parallel sum
-      if (P.par_gravity_mode == NCGPU_GRAVITY_EXACT) return seq_sum3(terms, n, d_cm_acc, d_cm_acc, st);
-      return par_sum3(terms, n, d_cm_acc, d_cm_acc, st);
+      if (P.par_gravity_mode == NCGPU_GRAVITY_EXACT) return seq_sum3(terms, N, c.n_dev, d_cm_acc, d_cm_acc, st);
+      return par_sum3(terms, N, c.n_dev, d_cm_acc, d_cm_acc, st);
 }
 
 }  // namespace ncg
