@@ -87,7 +87,8 @@ void free_all()
       if (c.sev0) cudaEventDestroy(c.sev0);
       if (c.sev1) cudaEventDestroy(c.sev1);
       if (c.s2) cudaStreamDestroy(c.s2);
-      if (c.cev) cudaEventDestroy(c.cev);
+      for (cudaEvent_t e : c.fev_done)
+            if (e) cudaEventDestroy(e);
       if (c.s3) cudaStreamDestroy(c.s3);
       if (c.s) cudaStreamDestroy(c.s);
       c = Ctx{};
@@ -394,7 +395,7 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
       A(c.ev, 3 * (size_t)c.ev_cap);
       A(c.evrec, EVREC * (size_t)c.ev_cap);
 #undef A
-      if (cudaMallocHost((void **)&c.pinned, 8 * N * sizeof(double)) != cudaSuccess) {
+      if (cudaMallocHost((void **)&c.pinned, (8 * N + 128) * sizeof(double)) != cudaSuccess) {
             free_all();
             return NCGPU_E_CUDA;
       }
@@ -402,10 +403,14 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
             free_all();
             return NCGPU_E_CUDA;
       }
+      for (cudaEvent_t &e : c.fev_done)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                  free_all();
+                  return NCGPU_E_CUDA;
+            }
       if (cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking) != cudaSuccess ||
           cudaStreamCreateWithFlags(&c.s2, cudaStreamNonBlocking) != cudaSuccess ||
           cudaStreamCreateWithFlags(&c.s3, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&c.cev, cudaEventDisableTiming) != cudaSuccess ||
           cudaEventCreateWithFlags(&c.sev0, cudaEventDisableTiming) != cudaSuccess ||
           cudaEventCreateWithFlags(&c.sev1, cudaEventDisableTiming) != cudaSuccess) {
             free_all();

@@ -572,7 +572,7 @@ struct Ctx {
       double *red = nullptr;       // reduction scratch (bbox etc.)
       unsigned *err = nullptr;     // device error word (behind scal)
       double *aos = nullptr;       // 8 * n_max staging for host AoS copies
-      double *pinned = nullptr;    // pinned host staging (8 * n_max doubles)
+      double *pinned = nullptr;    // pinned host staging (8 * n_max doubles, and 128 for the device's small answers)
       cudaEvent_t kev0 = nullptr, kev1 = nullptr;  // bracket the dominant kernel
       int kev_valid = 0;
       // display()'s statistics, started by ncgpu_format_cartesian on a second
@@ -583,7 +583,7 @@ struct Ctx {
       cudaEvent_t sev0 = nullptr, sev1 = nullptr;
       // the output text's copies to the host, chunk by chunk behind the formatting
       cudaStream_t s3 = nullptr;
-      cudaEvent_t cev = nullptr;
+      cudaEvent_t fev_done[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
       int stats_pre = 0;
 
       // collision state (device)
