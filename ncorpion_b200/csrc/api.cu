@@ -421,6 +421,7 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
             return st;
       }
       cudaMemsetAsync(c.err, 0, sizeof(unsigned), c.s);
+      cudaMemsetAsync(c.n_dev, 0, 8 * sizeof(int), c.s);
       cudaMemsetAsync(c.ex, 0, N * sizeof(int), c.s);
       cudaMemsetAsync(c.did, 0, N * sizeof(int), c.s);
       cudaMemsetAsync(c.dirty, 0, N, c.s);
@@ -545,8 +546,10 @@ int ncgpu_vector_field(struct ncgpu_body *bodies, const int *exists, int largest
       }
       double *h = c.pinned;
       NCG_CK(cudaMemcpyAsync(h, c.cm_acc, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+      unsigned *e = (unsigned *)(c.pinned + 3);
+      NCG_CK(cudaMemcpyAsync(e, c.err, sizeof *e, cudaMemcpyDeviceToHost, st));
       NCG_CK(cudaStreamSynchronize(st));
-      NCG_TRY(check_err_word());
+      if (*e) NCG_TRY(check_err_word());
       cm_acc[0] = h[0];
       cm_acc[1] = h[1];
       cm_acc[2] = h[2];

@@ -160,6 +160,49 @@ __device__ __forceinline__ f2 f2_rsqrt(f2 q)
       return f2_pack(rsqrt_ftz(lo), rsqrt_ftz(hi));
 }
 
+constexpr int GS = 256;  // threads of a block in grid_sum3
+
+// The sum over the grid of one value per lane of each block's warp 0 (three
+// components), by the last block to arrive: every block leaves its warp's sums in
+// red, the last one adds them in block order (deterministic).  True for the
+// threads of the last block, with the sums in tot[3] (shared).  count returns to 0.
+__device__ __forceinline__ bool grid_sum3(double v0, double v1, double v2, double *__restrict__ red,
+                                          unsigned *__restrict__ count, double *tot)
+{
+      __shared__ double sh[3][GS];
+      __shared__ int last;
+      if (threadIdx.x < 32) {
+            for (int o = 16; o > 0; o >>= 1) {
+                  v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+                  v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+                  v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+            }
+            if (threadIdx.x == 0) {
+                  red[3 * blockIdx.x] = v0;
+                  red[3 * blockIdx.x + 1] = v1;
+                  red[3 * blockIdx.x + 2] = v2;
+                  __threadfence();
+                  last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+            }
+      }
+      __syncthreads();
+      if (!last) return false;
+      __threadfence();
+      double s[3] = {0., 0., 0.};
+      for (int b = threadIdx.x; b < (int)gridDim.x; b += GS)
+            for (int d = 0; d < 3; d++) s[d] += __ldcg(red + 3 * b + d);
+      for (int d = 0; d < 3; d++) sh[d][threadIdx.x] = s[d];
+      __syncthreads();
+      for (int o = GS / 2; o > 0; o >>= 1) {
+            if (threadIdx.x < o)
+                  for (int d = 0; d < 3; d++) sh[d][threadIdx.x] += sh[d][threadIdx.x + o];
+            __syncthreads();
+      }
+      if (threadIdx.x < 3) tot[threadIdx.x] = sh[threadIdx.x][0];
+      __syncthreads();
+      return true;
+}
+
 // Two tiles' boxes (centre xyz, half extents xyz) are near when the gap
 // between them is below theta times the larger full diagonal.
 __device__ __forceinline__ bool tiles_near(const double *__restrict__ bi, const double *__restrict__ bj, double theta)
