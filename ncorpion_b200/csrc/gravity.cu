@@ -583,10 +583,12 @@ __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, do
 // half extents of its box, and with `mixed` the FP32 tile-relative copy.
 __global__ void k_tile_prep(BodyView bv, const int *__restrict__ slots, const int *__restrict__ n_dev, int ntiles,
                             double sp, int mixed, D4 *__restrict__ s64, double *__restrict__ sR,
-                            double *__restrict__ box, float *__restrict__ s32, float *__restrict__ sR32)
+                            double *__restrict__ box, float *__restrict__ s32, float *__restrict__ sR32,
+                            unsigned *__restrict__ count)
 {
       const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
       if (warp >= ntiles) return;
+      if (warp == 0 && lane == 0) *count = 0u;  // the final pass's arrivals
       const int n = *n_dev, base = warp * T;
       D4 d[T / 32];
       double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
@@ -1122,7 +1124,8 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
             NCG_TRY(radix_sort_pairs(c.keys, c.vals, nslots, 30, st));
             k_tile_prep<<<(ntub * 32 + 255) / 256, 256, 0, st>>>(bv, c.vals, c.n_dev, ntub, P.par_softening_parameter,
                                                                  mode == NCGPU_GRAVITY_MIXED, (D4 *)c.src64, c.srcR,
-                                                                 c.tilebox, (float *)c.src32, c.srcR32);
+                                                                 c.tilebox, (float *)c.src32, c.srcR32,
+                                                                 (unsigned *)(c.n_dev + 1));
             NCG_LAUNCHED();
             double h3[3];  // radius range and count: one copy
             NCG_CK(cudaMemcpyAsync(h3, c.red + 6, sizeof h3, cudaMemcpyDeviceToHost, st));
