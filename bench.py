@@ -39,10 +39,10 @@ sys.path.insert(0, ROOT)
 N_BODIES = 65536
 SOFTENING = 0.5
 FLOP_PER_INTERACTION = 20  # 3 sub, 3 FMA (r^2+eps^2), rsqrt (2), 3 mul, 3 FMA accumulate
-# DRAM bytes (read + write) of one k_grav_tiled<mixed> launch at N=65,536, from one ncu capture of
-# this script's gravity workload (profiles/k_grav_tiled_mixed_n65536.txt): 3.77 MB read + 105.56 MB written
-# (the written bytes are the per-chunk partial sums: 103 source chunks x 3 x 65,536 doubles).
-MIXED_DRAM_BYTES = 109.33e6
+# DRAM bytes (read + write) of one k_pair_sym<mixed> launch at N=65,536, from one ncu capture
+# (profiles/k_pair_sym_mixed_n65536.txt): 3.32 MB read + 142.57 MB written (the written bytes are the
+# partial rows: 128 blocks of bodies, 129 rows x 3 x 65,536 doubles, less what stays in L2).
+MIXED_DRAM_BYTES = 145.89e6
 # DRAM bytes of one mesh step's two main kernels (k_mesh_write + k_mesh_grav_fast) captured at N=262,144
 # (profiles/mesh_step_kernels_n262144.txt, current version: 40.3 MB + 36.0 MB), scaled by the bodies to
 # N=1,048,576.
@@ -944,8 +944,8 @@ def main(argv=None):
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved / fp32_peak, "traffic": MIXED_DRAM_BYTES,
                          "traffic_note": "bytes per launch from ncu (dram__bytes_read.sum + dram__bytes_write.sum); "
-                                         "algorithmic input 2.6 MB, the rest is the per-chunk partial sums",
-                         "kernel": "k_grav_tiled<mixed>", "kernel_ms": kms_mixed,
+                                         "algorithmic input 2.6 MB, the rest is the partial rows",
+                         "kernel": "k_pair_sym<mixed>", "kernel_ms": kms_mixed,
                          "flop_per_interaction": FLOP_PER_INTERACTION,
                          "peak_source": "measured in this run: best of the scalar FFMA and packed f32x2 FMA "
                                         "dependency-chain probes (ncgpu_probe_fp32_rates)",
