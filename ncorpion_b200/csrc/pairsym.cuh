@@ -350,8 +350,8 @@ constexpr size_t pair_smem()
 
 // One CTA of W warps = one unit.  MODE 0: mixed (FP32 far tile pairs, FP64 near
 // ones), 1: all FP64.  SOFT 0: none, 1: uniform eps^2, 2: eps = sum of the two
-// softening * radius.  With fewer row tiles than warps (B < W), two warps share a
-// row tile and take a column tile's two groups.
+// softening * radius.  With fewer row tiles than warps (B < W), two or four warps
+// share a row tile and the groups of a column tile.
 // part: rows of PAIR_OUT * npad doubles, row 2 (k - k0) the row sums of offset k,
 // row 2 (k - k0) + 1 its column sums.
 template <int MODE, int SOFT, int OP, int B, int W>
@@ -359,8 +359,9 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
                                                              double *__restrict__ part, long npad)
 {
       constexpr int NO = PAIR_OUT<OP>, RU = PAIR_ROWS<OP>;
-      constexpr int H = W / B;    // warps a row tile: 1 or 2
-      constexpr int NG = 2 / H;   // 64-column groups a warp takes of each column tile
+      constexpr int H = W / B;              // warps a row tile: 1, 2 or 4
+      constexpr int NG = H == 1 ? 2 : 1;    // 64-column groups a warp takes of each far column tile
+      constexpr int NN = PU / H;            // 32-column groups of each near one
       constexpr int NB = B * PT, TH = 32 * W;
       extern __shared__ __align__(16) unsigned char pair_sm[];
       double *col = reinterpret_cast<double *>(pair_sm), *rows = col + NO * NB;
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
 #pragma unroll
                                     for (int d = 0; d < NO; d++) acc[u][d] = 0.;
 #pragma unroll 1
-                              for (int g = 2 * h * NG; g < 2 * (h + 1) * NG; g++) {
+                              for (int g = h * NN; g < (h + 1) * NN; g++) {
                                     if (what == 1)
                                           near_group<SOFT, OP, true>(P, J * PT + 32 * g, i, lane, T, eps2, acc,
                                                                      cl + 32 * g, NB);
@@ -426,7 +427,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
                               for (int u = 0; u < RU; u++)
 #pragma unroll
                                     for (int d = 0; d < NO; d++) rs[(NO * u + d) * TH] += acc[u][d];
-                        } else {
+                        } else if (h * NG < 2) {
                               // coordinates relative to the column tile's centre
                               PairRows<OP, RU> F;
 #pragma unroll
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
             const int at = (q % 32) + 32 * (q / PT), u = (q % PT) / 32;
             for (int d = 0; d < NO; d++) {
                   double v = rows[(NO * u + d) * TH + at];
-                  if (H == 2) v += rows[(NO * u + d) * TH + at + 32 * B];
+                  for (int e = 1; e < H; e++) v += rows[(NO * u + d) * TH + at + 32 * B * e];
                   prow[d * npad + (long)b * NB + q] = v;
                   pcol[d * npad + (long)c * NB + q] = col[d * NB + q];
             }
@@ -519,6 +520,7 @@ __global__ void __launch_bounds__(256) k_pair_accum(const double *__restrict__ p
 // and, with several, the sums of the earlier ones behind them).
 struct PairPlan {
       int B, nb, nk, per;
+      bool few;  // few enough tiles for four warps a unit in the mixed kernel too
       long npad;
       size_t doubles;
 };
@@ -536,7 +538,16 @@ PairPlan pair_plan(int n)
       // 520 / 498 / 576 at 30,011, 1,730 / 1,669 / 1,657 at 65,536; FP64 276 / 297 / 352
       // at 12,345, 972 / 958 / 966 at 30,011, 3,935 / 3,882 / 3,808 at 65,536.  (The
       // VJP's larger sums leave room for four CTAs of two tiles.)
+      // With one row tile a CTA, four warps share it in the all-FP64 kernel and, up to
+      // 96 tiles, in the mixed one, whose near tile pairs are what a unit waits for; two
+      // beyond that, where the far ones are and only two of four warps would have a
+      // group of them.  Two / four warps, kernel microseconds: mixed 28 / 19 at 2,000
+      // bodies, 37 / 31 at 5,000, 54 / 51 at 8,192, 90 / 89 at 12,345, 134 / 139 at
+      // 16,384; FP64 28 / 18 at 2,000, 77 / 73 at 8,192, 156 / 148 at 12,345, 267 / 262
+      // at 16,384; 24 leapfrog steps and their VJPs, ms: FP64 4.1 / 3.0 at 1,000 bodies,
+      // 4.6 / 3.7 at 3,000; mixed 4.3 / 3.0 and 4.75 / 3.75.
       pl.B = ntiles <= 128 ? 1 : ntiles < 384 || OP == 1 ? 2 : 4;
+      pl.few = ntiles <= 96;
       pl.nb = (ntiles + pl.B - 1) / pl.B;
       pl.npad = (long)pl.nb * pl.B * PT;
       pl.nk = pair_offsets(pl.nb);
@@ -567,13 +578,15 @@ int pair_launch(const PairData &pd, int k0, int nk, double theta, double eps2, d
 }
 
 template <int MODE, int SOFT, int OP>
-int pair_launch_b(int B, const PairData &pd, int k0, int nk, double theta, double eps2, double *part, long npad,
-                  cudaStream_t st)
+int pair_launch_b(const PairPlan &pl, const PairData &pd, int k0, int nk, double theta, double eps2, double *part,
+                  long npad, cudaStream_t st)
 {
       if constexpr (OP == 0)
-            if (B == 4) return pair_launch<MODE, SOFT, OP, 4, 4>(pd, k0, nk, theta, eps2, part, npad, st);
-      if (B == 2) return pair_launch<MODE, SOFT, OP, 2, 4>(pd, k0, nk, theta, eps2, part, npad, st);
-      return pair_launch<MODE, SOFT, OP, 1, 2>(pd, k0, nk, theta, eps2, part, npad, st);
+            if (pl.B == 4) return pair_launch<MODE, SOFT, OP, 4, 4>(pd, k0, nk, theta, eps2, part, npad, st);
+      if (pl.B == 2) return pair_launch<MODE, SOFT, OP, 2, 4>(pd, k0, nk, theta, eps2, part, npad, st);
+      if constexpr (MODE == 0)
+            if (!pl.few) return pair_launch<MODE, SOFT, OP, 1, 2>(pd, k0, nk, theta, eps2, part, npad, st);
+      return pair_launch<MODE, SOFT, OP, 1, 4>(pd, k0, nk, theta, eps2, part, npad, st);
 }
 
 // Every unordered pair of pd's bodies once, into part (pl.doubles doubles).
@@ -588,13 +601,13 @@ int pair_sums(PairData pd, const PairPlan &pl, int mode, int soft, double theta,
             const int m = pl.nk - k0 < pl.per ? pl.nk - k0 : pl.per;
             int s;
             if (mode == 0)
-                  s = soft == 0   ? pair_launch_b<0, 0, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st)
-                      : soft == 1 ? pair_launch_b<0, 1, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st)
-                                  : pair_launch_b<0, 2, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st);
+                  s = soft == 0   ? pair_launch_b<0, 0, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st)
+                      : soft == 1 ? pair_launch_b<0, 1, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st)
+                                  : pair_launch_b<0, 2, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st);
             else
-                  s = soft == 0   ? pair_launch_b<1, 0, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st)
-                      : soft == 1 ? pair_launch_b<1, 1, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st)
-                                  : pair_launch_b<1, 2, OP>(pl.B, pd, k0, m, theta, eps2, part, pl.npad, st);
+                  s = soft == 0   ? pair_launch_b<1, 0, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st)
+                      : soft == 1 ? pair_launch_b<1, 1, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st)
+                                  : pair_launch_b<1, 2, OP>(pl, pd, k0, m, theta, eps2, part, pl.npad, st);
             NCG_TRY(s);
             if (k0 + m < pl.nk) {
                   k_pair_accum<PAIR_OUT<OP>><<<(pd.n + 31) / 32, 256, 0, st>>>(part, pl.npad, pl.nb, k0, m, pl.B * PT,
