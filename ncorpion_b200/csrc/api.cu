@@ -84,6 +84,7 @@ void free_all()
       if (c.pinned) cudaFreeHost(c.pinned);
       if (c.kev0) cudaEventDestroy(c.kev0);
       if (c.kev1) cudaEventDestroy(c.kev1);
+      if (c.prep_done) cudaEventDestroy(c.prep_done);
       if (c.sev0) cudaEventDestroy(c.sev0);
       if (c.sev1) cudaEventDestroy(c.sev1);
       if (c.s2) cudaStreamDestroy(c.s2);
@@ -400,6 +401,10 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
             return NCGPU_E_CUDA;
       }
       if (cudaEventCreate(&c.kev0) != cudaSuccess || cudaEventCreate(&c.kev1) != cudaSuccess) {
+            free_all();
+            return NCGPU_E_CUDA;
+      }
+      if (cudaEventCreateWithFlags(&c.prep_done, cudaEventDisableTiming) != cudaSuccess) {
             free_all();
             return NCGPU_E_CUDA;
       }

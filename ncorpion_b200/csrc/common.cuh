@@ -618,6 +618,7 @@ struct Ctx {
       double *pinned = nullptr;    // pinned host staging (8 * n_max doubles, and 128 for the device's small answers)
       cudaEvent_t kev0 = nullptr, kev1 = nullptr;  // bracket the dominant kernel
       int kev_valid = 0;
+      cudaEvent_t prep_done = nullptr;  // a tiled field's body count and radius range are in `pinned`
       // display()'s statistics, started by ncgpu_format_cartesian on a second
       // stream while its text crosses to the host; ncgpu_output_stats takes
       // them when no other entry point ran in between (any other one first
@@ -772,6 +773,9 @@ int refresh_j2();
 // LSD radix sort of (key, value) pairs, stable; keys use `bits` low bits.
 // Result ends in (keys, vals) buffers passed in (ping-pong through ctx scratch).
 int radix_sort_pairs(uint32_t *keys, int *vals, int n, int bits, cudaStream_t st);
+
+// The values in the stable order of their 32-bit keys, to `out` (not in place).
+int rank_sort(const uint32_t *keys, const int *vals, int n, int *out, cudaStream_t st);
 
 // Exclusive prefix sum; out has n + 1 entries (out[n] = total).
 int scan_exclusive(const int *in, int *out, int n, int *sums, cudaStream_t st);

@@ -414,9 +414,9 @@ __global__ void k_bbox_part(BodyView bv, const int *__restrict__ cidx, const int
 }
 
 // Folds the (at most 256) block partials: lo xyz, hi xyz, R min, R max in part[0..7],
-// the count of existing bodies in part[8].
+// the count of existing bodies in part[8]; the last three in page-locked host memory too.
 __global__ void __launch_bounds__(256) k_bbox_final(double *__restrict__ part, int nparts,
-                                                    const int *__restrict__ n_dev)
+                                                    const int *__restrict__ n_dev, double *__restrict__ answer)
 {
       __shared__ double sh[8][256];
       const int t = threadIdx.x;
@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(256) k_bbox_final(double *__restrict__ part, i
             __syncthreads();
       }
       if (t < 8) part[t] = sh[t][0];
-      if (t == 8) part[8] = (double)*n_dev;  // beside the radius range, so that one copy brings back both
+      if (t == 8) part[8] = (double)*n_dev;
+      if (t >= 6 && t < 9) answer[t - 6] = t == 8 ? (double)*n_dev : sh[t][0];
 }
 
 __device__ __forceinline__ uint32_t spread3(uint32_t v)
@@ -482,13 +483,17 @@ __global__ void k_morton(BodyView bv, const int *__restrict__ cidx, const int *_
 }
 
 // Up to 1024 U slots in one CTA: the compaction of the existing ones, `fill` in the
-// empty slots' rows, the bounding box, radius range and count (box[0..8]) and the
-// Morton keys, instead of seven launches (with CM_acc added up by the final pass: a 1,000-body
-// call 124 -> 102 us, a 12,345-body one 234 -> 209).
-template <int U>
+// empty slots' rows, the bounding box, radius range and count (box[0..8], the last three
+// in `answer` too, page-locked host memory) and, with KEYS, the Morton keys, instead of
+// seven launches (with CM_acc added up by the final pass: a 1,000-body call 124 -> 102 us,
+// a 12,345-body one 234 -> 209).  The host waits for the answer only, while the sort and
+// the tile preparation run: with the rank sort 93 -> 54 us at 1,000 bodies.  Beyond
+// 4,096 slots k_morton makes the keys, on all SMs (12,345: 31 us with them here, 23 and
+// 2.5 without).
+template <int U, bool KEYS>
 __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, double fill, int *__restrict__ cidx,
                                                      int *__restrict__ n_dev, double *__restrict__ box,
-                                                     uint32_t *__restrict__ keys, int *__restrict__ vals,
+                                                     double *__restrict__ answer, uint32_t *__restrict__ keys, int *__restrict__ vals,
                                                      double *__restrict__ ax, double *__restrict__ ay,
                                                      double *__restrict__ az)
 {
@@ -507,17 +512,37 @@ __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, do
             const unsigned m = __ballot_sync(0xffffffffu, e);
             below[u] = (unsigned char)__popc(m & ((1u << lane) - 1u));
             if (lane == 0) cnt[u * 32 + w] = __popc(m);
-            if (e) {
-                  in |= 1u << u;
-                  const long s = (long)i * bv.stride;
-                  const double b[4] = {bv.x[s], bv.y[s], bv.z[s], bv.R[s]};
-                  for (int d = 0; d < 3; d++) {
-                        v[d] = fmin(v[d], b[d]);
-                        v[3 + d] = fmax(v[3 + d], b[d]);
+            if (e) in |= 1u << u;
+      }
+      // the fields V slots at a time, their loads in flight together
+      constexpr int V = KEYS ? 2 : 4;  // (the keys take registers)
+#pragma unroll
+      for (int u0 = 0; u0 < U; u0 += V) {
+            double b[V][4];
+#pragma unroll
+            for (int u = 0; u < V; u++)
+                  if ((in >> (u0 + u)) & 1u) {
+                        const long s = (long)((u0 + u) * 1024 + tid) * bv.stride;
+                        b[u][0] = bv.x[s];
+                        b[u][1] = bv.y[s];
+                        b[u][2] = bv.z[s];
+                        b[u][3] = bv.R[s];
                   }
-                  v[6] = fmin(v[6], b[3]);
-                  v[7] = fmax(v[7], b[3]);
-            } else if (i < nslots) {
+#pragma unroll
+            for (int u = 0; u < V; u++)
+                  if ((in >> (u0 + u)) & 1u) {
+                        for (int d = 0; d < 3; d++) {
+                              v[d] = fmin(v[d], b[u][d]);
+                              v[3 + d] = fmax(v[3 + d], b[u][d]);
+                        }
+                        v[6] = fmin(v[6], b[u][3]);
+                        v[7] = fmax(v[7], b[u][3]);
+                  }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+            const int i = u * 1024 + tid;
+            if (i < nslots && !((in >> u) & 1u)) {
                   ax[i] = fill;
                   ay[i] = fill;
                   az[i] = fill;
@@ -536,6 +561,7 @@ __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, do
             if (lane == 0) {
                   bx[w] = a;
                   box[w] = a;
+                  if (w >= 6) answer[w - 6] = a;
             }
       } else if (w == 8) {  // exclusive prefix of the 32 U warp counts, U a lane
             int s = 0;
@@ -555,6 +581,7 @@ __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, do
                   n_s = incl;
                   *n_dev = incl;
                   box[8] = (double)incl;
+                  answer[2] = (double)incl;
             }
       }
       __syncthreads();
@@ -563,15 +590,18 @@ __global__ void __launch_bounds__(1024) k_prep_tiled(BodyView bv, int nslots, do
             const int i = u * 1024 + tid;
             if (!((in >> u) & 1u)) continue;
             const int p = cnt[u * 32 + w] + below[u];
-            const long s = (long)i * bv.stride;
             cidx[p] = i;
-            keys[p] = morton_key(bv.x[s], bv.y[s], bv.z[s], bx);
-            vals[p] = i;
+            if constexpr (KEYS) {
+                  const long s = (long)i * bv.stride;
+                  keys[p] = morton_key(bv.x[s], bv.y[s], bv.z[s], bx);
+                  vals[p] = i;
+            }
       }
-      for (int p = n_s + tid; p < nslots; p += 1024) {  // sorted after every body
-            keys[p] = 0xffffffffu;
-            vals[p] = -1;
-      }
+      if constexpr (KEYS)
+            for (int p = n_s + tid; p < nslots; p += 1024) {  // sorted after every body
+                  keys[p] = 0xffffffffu;
+                  vals[p] = -1;
+            }
 }
 
 // FP32 tile-relative sources, one SoA block per tile of T bodies:
@@ -1060,6 +1090,12 @@ int exact_field(const BodyView &bv, int nslots, const CmArg &cm, double G, doubl
       return NCGPU_OK;
 }
 
+// Slots up to which the Morton order is a rank sort (n^2 compares in one launch), beyond
+// it a radix sort (eight launches).  Whole mixed calls, rank / radix, us: 49 / 69 at 250
+// bodies, 55 / 79 at 1,000, 73 / 99 at 4,096, 117 / 143 at 8,192, 175 / 188 at 12,345,
+// 241 / 238 at 16,384, 394 / 356 at 24,000.
+constexpr int RANK_MAX = 14336;
+
 // CM_acc of the tiled modes: the two-level sum of its terms, or zero.
 int finish_cm(int central, int n, double *d_cm_acc, cudaStream_t st)
 {
@@ -1103,11 +1139,16 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
             // count and the radius range come back to the host (for the pair
             // kernel's grid and instance) while the GPU sorts and packs
             const int ntub = (nslots + T - 1) / T;
+            volatile double *answer = c.pinned + 8 * (size_t)c.n_max + 96;  // (behind the output text's answers)
+            double *ans = const_cast<double *>(answer);
+            int *vals = nslots <= RANK_MAX ? c.vals2 : c.vals;  // (the rank sort is not in place)
             if (nslots <= 4096) {
-                  k_prep_tiled<4><<<1, 1024, 0, st>>>(bv, nslots, fill, c.cidx, c.n_dev, c.red, c.keys, c.vals, ax, ay, az);
+                  k_prep_tiled<4, true><<<1, 1024, 0, st>>>(bv, nslots, fill, c.cidx, c.n_dev, c.red, ans, c.keys, vals, ax,
+                                                            ay, az);
                   NCG_LAUNCHED();
             } else if (nslots <= 16384) {
-                  k_prep_tiled<16><<<1, 1024, 0, st>>>(bv, nslots, fill, c.cidx, c.n_dev, c.red, c.keys, c.vals, ax, ay, az);
+                  k_prep_tiled<16, false><<<1, 1024, 0, st>>>(bv, nslots, fill, c.cidx, c.n_dev, c.red, ans, nullptr, nullptr,
+                                                              ax, ay, az);
                   NCG_LAUNCHED();
             } else {
                   k_fill3<<<(nslots + 255) / 256, 256, 0, st>>>(ax, ay, az, nslots, fill);
@@ -1116,23 +1157,25 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
                   const int nbb = min(256, (nslots + RB - 1) / RB);
                   k_bbox_part<<<nbb, RB, 0, st>>>(bv, c.cidx, c.n_dev, c.red);
                   NCG_LAUNCHED();
-                  k_bbox_final<<<1, 256, 0, st>>>(c.red, nbb, c.n_dev);
-                  NCG_LAUNCHED();
-                  k_morton<<<(nslots + 255) / 256, 256, 0, st>>>(bv, c.cidx, c.n_dev, nslots, c.red, c.keys, c.vals);
+                  k_bbox_final<<<1, 256, 0, st>>>(c.red, nbb, c.n_dev, ans);
                   NCG_LAUNCHED();
             }
-            NCG_TRY(radix_sort_pairs(c.keys, c.vals, nslots, 30, st));
+            NCG_CK(cudaEventRecord(c.prep_done, st));
+            if (nslots > 4096) {
+                  k_morton<<<(nslots + 255) / 256, 256, 0, st>>>(bv, c.cidx, c.n_dev, nslots, c.red, c.keys, vals);
+                  NCG_LAUNCHED();
+            }
+            if (nslots <= RANK_MAX) NCG_TRY(rank_sort(c.keys, vals, nslots, c.vals, st));
+            else NCG_TRY(radix_sort_pairs(c.keys, c.vals, nslots, 30, st));
             k_tile_prep<<<(ntub * 32 + 255) / 256, 256, 0, st>>>(bv, c.vals, c.n_dev, ntub, P.par_softening_parameter,
                                                                  mode == NCGPU_GRAVITY_MIXED, (D4 *)c.src64, c.srcR,
                                                                  c.tilebox, (float *)c.src32, c.srcR32,
                                                                  (unsigned *)(c.n_dev + 1));
             NCG_LAUNCHED();
-            double h3[3];  // radius range and count: one copy
-            NCG_CK(cudaMemcpyAsync(h3, c.red + 6, sizeof h3, cudaMemcpyDeviceToHost, st));
-            NCG_CK(cudaStreamSynchronize(st));
-            rr[0] = h3[0];
-            rr[1] = h3[1];
-            n = (int)h3[2];
+            NCG_CK(cudaEventSynchronize(c.prep_done));
+            rr[0] = answer[0];
+            rr[1] = answer[1];
+            n = (int)answer[2];
       }
       const double G = P.par_G;
       const double mu = G * cmh[6];

@@ -314,6 +314,71 @@ int compact_existing(const int *ex, int largest_id, int *n_host, cudaStream_t st
       return NCGPU_OK;
 }
 
+// The values in the stable order of their keys, in one launch: a key's place is the
+// number of smaller keys and of equal ones before it.  The lanes of each of a CTA's
+// warps hold the same 32 targets; the warps share out the sources, 32 at a time from
+// shared memory, all lanes reading the same four.  n^2 compares, bound by their issue
+// (2.7 us at 1,000 keys, 8.8 at 5,000, 27 at 12,345), against about 40 us of eight
+// dependent launches for the radix sort at any of these.
+constexpr int RKC = 4096;  // keys staged at once
+
+__global__ void __launch_bounds__(256) k_rank_sort(const uint32_t *__restrict__ keys, const int *__restrict__ vals,
+                                                   int n, int *__restrict__ out)
+{
+      __shared__ __align__(16) uint32_t ks[RKC];
+      __shared__ int part[8][32];
+      const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+      const int b = blockIdx.x * 32, i = b + lane;
+      const uint32_t key = i < n ? keys[i] : 0xffffffffu;
+      const int val = w == 0 && i < n ? vals[i] : 0;
+      int c = 0;
+      for (int base = 0; base < n; base += RKC) {
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < RKC / 256; r++) {
+                  const int j = base + r * 256 + tid;
+                  ks[r * 256 + tid] = j < n ? keys[j] : 0xffffffffu;  // never before a target
+            }
+            __syncthreads();
+            const int m = min(RKC, n - base);
+            for (int g = 32 * w; g < m; g += 256) {
+                  const uint4 *k4 = reinterpret_cast<const uint4 *>(ks + g);
+                  if (base + g < b) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                              const uint4 k = k4[q];
+                              c += (k.x <= key) + (k.y <= key) + (k.z <= key) + (k.w <= key);
+                        }
+                  } else if (base + g > b) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                              const uint4 k = k4[q];
+                              c += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+                        }
+                  } else {
+                        for (int q = 0; q < 32; q++) {
+                              const uint32_t k = ks[g + q];
+                              c += k < key || (k == key && q < lane);
+                        }
+                  }
+            }
+      }
+      part[w][lane] = c;
+      __syncthreads();
+      if (w == 0 && i < n) {
+            for (int q = 1; q < 8; q++) c += part[q][lane];
+            out[c] = val;
+      }
+}
+
+int rank_sort(const uint32_t *keys, const int *vals, int n, int *out, cudaStream_t st)
+{
+      if (n <= 0) return NCGPU_OK;
+      k_rank_sort<<<(n + 31) / 32, 256, 0, st>>>(keys, vals, n, out);
+      NCG_LAUNCHED();
+      return NCGPU_OK;
+}
+
 int radix_sort_pairs(uint32_t *keys, int *vals, int n, int bits, cudaStream_t st)
 {
       Ctx &c = ctx();

@@ -64,3 +64,26 @@ def test_pair_sums(lib, n, radii):
         again, _ = api.vector_field(b, ex, mode=mode)
         assert np.array_equal(acc, again)  # the sums' order is fixed
     api.finalize()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 4095, 4097, 14336, 14337])
+def test_equal_keys(lib, n):
+    """Bodies at 64 places, so that nearly all Morton keys have equals (a stable
+    order places each once), with holes; the same bounds as above."""
+    from ncorpion_b200 import api, disks
+    b = disks.gravity_disk(n, seed=n)
+    rng = np.random.default_rng(n)
+    b[:, :3] = b[rng.integers(0, min(n, 64), n), :3]
+    ex = np.ones(n, np.int32)
+    ex[rng.random(n) < 0.1] = 0
+    ex[n - 1] = 1
+    api.init(n, make_params(softening_parameter=0.5, central_mass_bool=0))
+    live = np.flatnonzero(ex)
+    rows = live if len(live) <= 48 else np.sort(rng.choice(live, 48, replace=False))
+    ref, mag = reference(b, ex, 0.5, rows)
+    scale = mag.max(axis=1, keepdims=True) + 1e-300
+    for mode, tol in (("fp64", 1e-13), ("mixed", 4e-6)):
+        acc, _ = api.vector_field(b, ex, mode=mode)
+        assert np.all(np.isfinite(acc)) and not acc[ex == 0].any()
+        assert (np.abs(acc[rows] - ref) / scale).max() <= tol
+    api.finalize()
