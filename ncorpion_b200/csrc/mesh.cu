@@ -772,7 +772,8 @@ __global__ void k_clear_dirty_events_dev(unsigned char *dirty, const int *ev, co
 }
 
 // Candidates of the bodies k in [lo, hi) (pop order, positions from base) and
-// their hits against the current state: the kernels, without waiting.
+// their hits against the current state, counted on in S_NHITS: the kernels, without
+// waiting.
 static int mesh_segment_launch(const DevState &S, int lid, int lo, int hi, long base, int test)
 {
       Ctx &c = ctx();
@@ -792,7 +793,6 @@ static int mesh_segment_launch(const DevState &S, int lid, int lo, int hi, long 
             k_add_base<<<(n + 256) / 256, 256, 0, st>>>(c.moff, n, (int)base);
             NCG_LAUNCHED();
       }
-      if (base > 0) NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, sizeof(int), st));
       // (positions at or past pair_cap are not written: the kernel records the
       // overflow and the host returns NCGPU_E_CAPACITY)
       k_mesh_write<<<(n + MWW * 32 - 1) / (MWW * 32), MWW * 32, 0, st>>>(
@@ -832,11 +832,14 @@ static int mesh_segment_finish(const DevState &S, int lid, int hi, long base, in
       return NCGPU_OK;
 }
 
-// Both halves with one synchronisation between them.
+// Both halves with one synchronisation between them.  (The hits' counter holds the
+// launch before, the whole pass's first one also where no candidate came before this
+// segment.)
 static int mesh_segment(const DevState &S, int lid, int lo, int hi, long base, int test, const MeshEvArgs &E0,
                         int *tot)
 {
       Ctx &c = ctx();
+      NCG_CK(cudaMemsetAsync(c.scal + S_NHITS, 0, sizeof(int), c.s));
       NCG_TRY(mesh_segment_launch(S, lid, lo, hi, base, test));
       int h[S_COUNT];
       NCG_CK(cudaMemcpyAsync(h, c.scal, sizeof h, cudaMemcpyDeviceToHost, c.s));

@@ -289,3 +289,37 @@ def test_mesh_steps_fast_mode_match_exact(gpu, case):
                 assert np.array_equal(bf[live][:, :3], br[live][:, :3])
             np.testing.assert_allclose(bf[live], br[live], rtol=1e-12, atol=0)
             np.testing.assert_allclose(cmf, cmr, rtol=1e-12, atol=1e-18)
+
+
+@pytest.mark.parametrize("ctype", [1, 2])
+@pytest.mark.parametrize("slots", [(1000,), (0, 1500), (1, 2, 2990)])
+def test_mesh_pass_big_bodies_in_any_slot(gpu, ctype, slots):
+    """mesh() on bodies as they are, without the three largest in front: the first
+    segment of small bodies is one of colliding pairs, with more behind the big body."""
+    n, cells, gam = 3000, 32, 0.05
+    rng = np.random.default_rng(11)
+    b = np.zeros((n, 8))
+    b[:, :3] = rng.uniform(-0.6, 0.6, (n, 3))
+    b[:, 3:6] = rng.normal(0, 0.05, (n, 3))
+    b[:, 6] = 10.0 ** rng.uniform(-9, -7, n)
+    b[:, 7] = rng.uniform(2e-3, 2.4e-2, n)
+    b[list(slots), 7] = 0.06
+    ex = np.ones(n, np.int32)
+    ex[5::29] = 0
+    cm = np.array([0, 0, 0, 0, 0, 0, 1.0, 1.0])
+    p = mesh_params(ctype, cells=cells, collision_cube_min=gam * cells)
+    api = gpu(n, p)
+    api.upload(b, ex, cm)
+    api.set_timestep(1e-2)
+    n_pairs, n_ev, tn = api.mesh(gam, True)
+    w = oracle.PortWorld(n, p)
+    w.set_state(b, ex, cm, dt=1e-2, gam=gam)
+    w.lib.orc_w_mesh()
+    ev = w.events()
+    assert len(ev) > 50 and ev[:, :2].max() > min(slots)
+    assert np.array_equal(api.events(), ev)
+    assert np.array_equal(api.pairs(), w.pairs())
+    assert tn == w.lib.orc_w_total_neighbours()
+    bg, exg, _ = api.download(n)
+    b_ref, ex_ref, _ = w.get_state()
+    assert_state_equal(bg, exg, b_ref, ex_ref)
