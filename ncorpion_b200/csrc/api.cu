@@ -208,7 +208,6 @@ int refresh_j2()
       NCG_TRY(state_cm_host(cm9));
       c.j2_prev = c.j2;
       c.j2 = j2_value(c.P, cm9[6], cm9[8]);
-      c.j2_M = cm9[6];
       return NCGPU_OK;
 }
 
@@ -220,13 +219,13 @@ int kick_state()
       c.com_reduced = 0;
       const int nslots = c.largest_id + 1;
       const bool mesh_grav = c.P.par_mesh_bool && !c.force_naive && !c.P.par_mesh_brute_gravity;
-      // the central mass's state on the host: for the tiled gravity's arguments; mesh
-      // gravity and the exact brute force read it from device memory, and the J2 term
-      // needs the mass alone, known since the last upload or end of step
+      // the central mass's state on the host, for the tiled gravity's arguments; mesh
+      // gravity and the exact brute force read it from device memory (its mass too, which
+      // a collision pass may have changed: super-catastrophic fragmentations add to it)
       const bool exact = c.P.par_gravity_mode == NCGPU_GRAVITY_EXACT;
       double cm9[9] = {0.};
       if (!mesh_grav && !exact) NCG_TRY(state_cm_host(cm9));
-      const J2Arg j2 = j2_arg(c.P, c.j2_M, c.j2);
+      const J2Arg j2 = j2_arg(c.P, c.j2);
       if (mesh_grav)
             NCG_TRY(mesh_gravity_state(j2));
       else
@@ -505,7 +504,7 @@ int ncgpu_vector_field_part(const double *d_bodies, const int *d_exists, int lar
       // d_acc is 3 consecutive blocks of (largest_id + 1) doubles
       long bs = largest_id + 1;
       // gravity_eval writes ax, ay, az blocks; repack to xyz triples
-      const J2Arg j2 = j2_arg(c.P, cm->mass, j2_value(c.P, cm->mass, c.P.par_sideral_omega));
+      const J2Arg j2 = j2_arg(c.P, j2_value(c.P, cm->mass, c.P.par_sideral_omega));
       NCG_TRY(gravity_eval(bv, largest_id, (const double *)cm, j2, c.acc, c.n_max, d_cm_acc, gravity_mode, st, part,
                            nparts));
       if (bs > 0) {  // interleave into d_acc[3*k + d]
@@ -539,7 +538,7 @@ int ncgpu_vector_field(struct ncgpu_body *bodies, const int *exists, int largest
             NCG_CK(cudaMemcpyAsync(c.exs, exists, sizeof(int) * (size_t)ns, cudaMemcpyHostToDevice, st));
       }
       BodyView bv{c.aos, c.aos + 1, c.aos + 2, c.aos + 3, c.aos + 4, c.aos + 5, c.aos + 6, c.aos + 7, 8, c.exs};
-      const J2Arg j2 = j2_arg(c.P, cm->mass, j2_value(c.P, cm->mass, c.P.par_sideral_omega));
+      const J2Arg j2 = j2_arg(c.P, j2_value(c.P, cm->mass, c.P.par_sideral_omega));
       NCG_TRY(gravity_eval(bv, largest_id, (const double *)cm, j2, c.acc, c.n_max, c.cm_acc, gravity_mode, st));
       // the records come back whole: the velocity fields of the existing bodies
       // carry their accelerations, every other byte is the caller's own

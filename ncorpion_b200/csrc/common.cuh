@@ -45,10 +45,11 @@ struct BodyView {
 };
 
 // The J2 term of a force evaluation (src/physics.c:149-160): off, or on with
-// R_unit, the J2 in force and the central mass M.
+// R_unit and the J2 in force.  (The central mass is not here: collisions change it on
+// the device, so the kernels take it from where they take the central body.)
 struct J2Arg {
       int on;
-      double R, J2, M;
+      double R, J2;
 };
 
 // J2_value when it is nonzero, else the fluid-body J2 of central mass M and
@@ -60,18 +61,18 @@ inline double j2_value(const ncgpu_params &P, double M, double omega)
       return 0.5 * omega * omega * P.par_R_unit * P.par_R_unit * P.par_R_unit / (P.par_G * M);
 }
 
-// The J2 term of a force evaluation with the J2 value j2 (central mass M).
-inline J2Arg j2_arg(const ncgpu_params &P, double M, double j2)
+// The J2 term of a force evaluation with the J2 value j2.
+inline J2Arg j2_arg(const ncgpu_params &P, double j2)
 {
-      return J2Arg{P.par_J2_bool && P.par_central_mass_bool, P.par_R_unit, j2, M};
+      return J2Arg{P.par_J2_bool && P.par_central_mass_bool, P.par_R_unit, j2};
 }
 
-// Adds body k's J2 term to its acceleration a[] and returns CM_acc's share in
-// c[], every operation the reference's in its order with IEEE rounding:
+// Adds body k's J2 term (central mass M, mu = G M) to its acceleration a[] and returns
+// CM_acc's share in c[], every operation the reference's in its order with IEEE rounding:
 //   r2 = rk*rk, r5 = r3*r2, K = mu*R*R*J2/r5, q = 7.5/r2*DZ*DZ
 //   a += K*(-1.5*DX + q*DX), K*(-1.5*DY + q*DY), K*(-4.5*DZ + q*DZ)
 //   c  = K*(1.5*DX - q*DX)*mk/M, ... (4.5 for z)
-__device__ __forceinline__ void d_j2(const J2Arg &j, double mu, double DX, double DY, double DZ, double rk,
+__device__ __forceinline__ void d_j2(const J2Arg &j, double M, double mu, double DX, double DY, double DZ, double rk,
                                      double r3, double mk, double &ax, double &ay, double &az, double *c)
 {
       const double r2 = __dmul_rn(rk, rk);
@@ -82,9 +83,9 @@ __device__ __forceinline__ void d_j2(const J2Arg &j, double mu, double DX, doubl
       ax = __dadd_rn(ax, __dmul_rn(K, __dadd_rn(__dmul_rn(-1.5, DX), qx)));
       ay = __dadd_rn(ay, __dmul_rn(K, __dadd_rn(__dmul_rn(-1.5, DY), qy)));
       az = __dadd_rn(az, __dmul_rn(K, __dadd_rn(__dmul_rn(-4.5, DZ), qz)));
-      c[0] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(1.5, DX), qx)), mk), j.M);
-      c[1] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(1.5, DY), qy)), mk), j.M);
-      c[2] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(4.5, DZ), qz)), mk), j.M);
+      c[0] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(1.5, DX), qx)), mk), M);
+      c[1] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(1.5, DY), qy)), mk), M);
+      c[2] = __ddiv_rn(__dmul_rn(__dmul_rn(K, __dsub_rn(__dmul_rn(4.5, DZ), qz)), mk), M);
 }
 
 // x / b correctly rounded (round to nearest even) from y = RN(1/b), with
@@ -570,7 +571,6 @@ struct Ctx {
       double *cm = nullptr;        // 16 doubles: central mass record (8), SideralOmega at [8]
       double j2 = 0.;              // the J2 in force for the state's kicks (set at upload and end of step)
       double j2_prev = 0.;         // the J2 in force before the last end of step's update
-      double j2_M = 1.;            // the central mass of that upload or end of step (its mass changes there only)
       int com_reduced = 0;         // the last end of step reduced the barycentre
       int eot_lid = -1;            // largest_id at the start of the last end of step
       // output staging (output.cu): snapshot body fields and central body, the

@@ -304,10 +304,6 @@ int eot_state(int *hm_out)
             if (h[S_NFLAG] > 0) NCG_TRY(state_cm_host(cm9));  // (dumped bodies changed its mass)
             c.j2_prev = c.j2;
             c.j2 = j2_value(P, cm9[6], cm9[8]);
-            c.j2_M = cm9[6];
-      } else if (P.par_J2_bool && h[S_NFLAG] > 0) {
-            NCG_TRY(state_cm_host(cm9));
-            c.j2_M = cm9[6];
       }
       if (hm_out) *hm_out = hm;
       return NCGPU_OK;

@@ -64,8 +64,9 @@ struct CmArg {
 
 // The central mass's acceleration of a body (with J2, src/physics.c:123-160) and
 // CM_acc's terms from it: c[0..2] the central ones, c[3..5] J2's share.
-__device__ __forceinline__ void central_terms(const D4 &me, double cmx, double cmy, double cmz, double mu,
-                                              const J2Arg &j2, double mk, double (&a)[3], double (&c)[6])
+__device__ __forceinline__ void central_terms(const D4 &me, double cmx, double cmy, double cmz, double M,
+                                              double mu, const J2Arg &j2, double mk, double (&a)[3],
+                                              double (&c)[6])
 {
       // src/physics.c:123-139: DX = X - XX, rk = sqrt(DX*DX + DY*DY + DZ*DZ)
       const double DX = __dsub_rn(me.x, cmx), DY = __dsub_rn(me.y, cmy), DZ = __dsub_rn(me.z, cmz);
@@ -79,7 +80,7 @@ __device__ __forceinline__ void central_terms(const D4 &me, double cmx, double c
       c[1] = div_by_recip(__dmul_rn(me.w, DY), r3, y3);
       c[2] = div_by_recip(__dmul_rn(me.w, DZ), r3, y3);
       c[3] = c[4] = c[5] = 0.;
-      if (j2.on) d_j2(j2, mu, DX, DY, DZ, rk, r3, mk, a[0], a[1], a[2], c + 3);  // src/physics.c:149-160
+      if (j2.on) d_j2(j2, M, mu, DX, DY, DZ, rk, r3, mk, a[0], a[1], a[2], c + 3);  // src/physics.c:149-160
 }
 
 // div_by_recip for x != 0.
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(XP + 32, OCC) k_grav_exact(const D4 *__restric
       __shared__ double tm[2][3 * XROW];
       const int tid = threadIdx.x, n = *n_dev;
       const double cmx = cm.dev ? cm.dev[0] : cm.x, cmy = cm.dev ? cm.dev[1] : cm.y, cmz = cm.dev ? cm.dev[2] : cm.z;
-      const double mu = G * (cm.dev ? cm.dev[6] : cm.m);
+      const double M = cm.dev ? cm.dev[6] : cm.m, mu = G * M;
       const bool adder = tid >= XP;
       const int lane = tid & 31;
       if (central && blockIdx.x == 0) {
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(XP + 32, OCC) k_grav_exact(const D4 *__restric
                         const int p = k * XCM + tid;
                         double a[3], c[6] = {0., 0., 0., 0., 0., 0.};
                         if (tid < XCM && p < n)
-                              central_terms(src[p], cmx, cmy, cmz, mu, j2,
+                              central_terms(src[p], cmx, cmy, cmz, M, mu, j2,
                                             j2.on ? bv.m[(long)cidx[p] * bv.stride] : 0., a, c);
                         if (k >= 2) bar_sync(EMPTY + (k & 1), XTH);
                         for (int d = 0; d < 3 && tid < XCM; d++) {
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(XP + 32, OCC) k_grav_exact(const D4 *__restric
       double acc = 0.;
       if (central && live) {
             double a[3], c[6];
-            central_terms(src[ps], cmx, cmy, cmz, mu, j2, j2.on ? bv.m[(long)cidx[ps] * bv.stride] : 0., a, c);
+            central_terms(src[ps], cmx, cmy, cmz, M, mu, j2, j2.on ? bv.m[(long)cidx[ps] * bv.stride] : 0., a, c);
             acc = d == 0 ? a[0] : d == 1 ? a[1] : a[2];
       }
       for (int k = 0; k < rounds; k++) {
@@ -904,7 +905,7 @@ __global__ void __launch_bounds__(MXB, 12) k_grav_tiled(const D4 *__restrict__ s
 // c: the body's CM_acc terms.
 __device__ __forceinline__ void grav_finish(int q, bool own, const double (&m)[3], const D4 *__restrict__ s64,
                                             const int *__restrict__ slots, double cmx, double cmy, double cmz,
-                                            double mu, double G, int central, const J2Arg &j2,
+                                            double M, double G, int central, const J2Arg &j2,
                                             double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                                             double (&c)[3])
 {
@@ -914,12 +915,13 @@ __device__ __forceinline__ void grav_finish(int q, bool own, const double (&m)[3
             double DX = s.x - cmx, DY = s.y - cmy, DZ = s.z - cmz;
             double rk = sqrt(DX * DX + DY * DY + DZ * DZ);
             double r3 = rk * rk * rk;
+            const double mu = G * M;
             a[0] += -mu * DX / r3;
             a[1] += -mu * DY / r3;
             a[2] += -mu * DZ / r3;
             double gm = G * s.w;
             double cj[3] = {0., 0., 0.};
-            if (j2.on) d_j2(j2, mu, DX, DY, DZ, rk, r3, s.w, a[0], a[1], a[2], cj);
+            if (j2.on) d_j2(j2, M, mu, DX, DY, DZ, rk, r3, s.w, a[0], a[1], a[2], cj);
             c[0] = gm * DX / r3 + cj[0];
             c[1] = gm * DY / r3 + cj[1];
             c[2] = gm * DZ / r3 + cj[2];
@@ -931,7 +933,7 @@ __device__ __forceinline__ void grav_finish(int q, bool own, const double (&m)[3
 }
 
 __global__ void k_grav_final(const double *__restrict__ partial, int nchunks, long npad, const D4 *__restrict__ s64,
-                             const int *__restrict__ slots, int n, double cmx, double cmy, double cmz, double mu,
+                             const int *__restrict__ slots, int n, double cmx, double cmy, double cmz, double M,
                              double G, int central, J2Arg j2, int q_lo, int q_hi, double *__restrict__ ax,
                              double *__restrict__ ay, double *__restrict__ az, double *__restrict__ cterm)
 {
@@ -945,7 +947,7 @@ __global__ void k_grav_final(const double *__restrict__ partial, int nchunks, lo
                   for (int d = 0; d < 3; d++) m[d] += partial[(size_t)c * 3 * npad + d * npad + q];
       }
       double c[3];
-      grav_finish(q, own, m, s64, slots, cmx, cmy, cmz, mu, G, central, j2, ax, ay, az, c);
+      grav_finish(q, own, m, s64, slots, cmx, cmy, cmz, M, G, central, j2, ax, ay, az, c);
       if (central)
             for (int d = 0; d < 3; d++) cterm[(size_t)d * n + q] = c[d];
 }
@@ -955,7 +957,7 @@ __global__ void k_grav_final(const double *__restrict__ partial, int nchunks, lo
 // central mass), red: 3 doubles a block, count: zero before and after.
 __global__ void __launch_bounds__(GS) k_pair_final(PairRun pr, const D4 *__restrict__ s64,
                                                     const int *__restrict__ slots, int n, double cmx, double cmy,
-                                                    double cmz, double mu, double G, int central, J2Arg j2,
+                                                    double cmz, double M, double G, int central, J2Arg j2,
                                                     double *__restrict__ ax, double *__restrict__ ay,
                                                     double *__restrict__ az, double *__restrict__ red,
                                                     unsigned *__restrict__ count, double *__restrict__ cm_acc)
@@ -969,7 +971,7 @@ __global__ void __launch_bounds__(GS) k_pair_final(PairRun pr, const D4 *__restr
       if (threadIdx.x < 32 && q < n) {
             if (pr.base)
                   for (int d = 0; d < 3; d++) v[d] = pr.base[d * pr.npad + q] + v[d];
-            grav_finish((int)q, true, v, s64, slots, cmx, cmy, cmz, mu, G, central, j2, ax, ay, az, c);
+            grav_finish((int)q, true, v, s64, slots, cmx, cmy, cmz, M, G, central, j2, ax, ay, az, c);
       }
       if (!central) {
             if (blockIdx.x == 0 && threadIdx.x < 3) cm_acc[threadIdx.x] = 0.;
@@ -1178,7 +1180,6 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
             n = (int)answer[2];
       }
       const double G = P.par_G;
-      const double mu = G * cmh[6];
       if (n == 0) {
             k_set3<<<1, 1, 0, st>>>(d_cm_acc, 0., 0., 0.);
             NCG_LAUNCHED();
@@ -1210,8 +1211,8 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
             NCG_TRY(pair_sums<0>(pd, pl, mode == NCGPU_GRAVITY_MIXED ? 0 : 1, soft_kind, theta, eps2, c.partial, pr, st));
             NCG_CK(cudaEventRecord(c.kev1, st));
             c.kev_valid = 1;
-            k_pair_final<<<(n + 31) / 32, GS, 0, st>>>(pr, s64, c.vals, n, cmh[0], cmh[1], cmh[2], mu, G, central, j2,
-                                                       ax, ay, az, c.cmterm, (unsigned *)(c.n_dev + 1), d_cm_acc);
+            k_pair_final<<<(n + 31) / 32, GS, 0, st>>>(pr, s64, c.vals, n, cmh[0], cmh[1], cmh[2], cmh[6], G, central,
+                                                       j2, ax, ay, az, c.cmterm, (unsigned *)(c.n_dev + 1), d_cm_acc);
             NCG_LAUNCHED();
             return NCGPU_OK;
       }
@@ -1255,7 +1256,7 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       NCG_CK(cudaEventRecord(c.kev1, st));
       c.kev_valid = 1;
       k_grav_final<<<(n + 255) / 256, 256, 0, st>>>(c.partial, nchunks, npad, s64, c.vals, n, cmh[0], cmh[1], cmh[2],
-                                                    mu, G, central, j2, ib_lo * T, min(n, ib_hi * T), ax, ay, az,
+                                                    cmh[6], G, central, j2, ib_lo * T, min(n, ib_hi * T), ax, ay, az,
                                                     c.cmterm);
       NCG_LAUNCHED();
       return finish_cm(central, n, d_cm_acc, st);

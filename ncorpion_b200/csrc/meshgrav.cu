@@ -366,7 +366,7 @@ __device__ __forceinline__ bool body_prologue(const DevState &S, const MGArgs &A
             const double cc[3] = {div_by_recip(DMUL(g, DX), r3, y3), div_by_recip(DMUL(g, DY), r3, y3),
                                   div_by_recip(DMUL(g, DZ), r3, y3)};
             double cj[3] = {0., 0., 0.};
-            if (A.j2.on) d_j2(A.j2, mu, DX, DY, DZ, rk, r3, me.m, a_x, a_y, a_z, cj);  // src/physics.c:149-160
+            if (A.j2.on) d_j2(A.j2, A.cm[6], mu, DX, DY, DZ, rk, r3, me.m, a_x, a_y, a_z, cj);  // src/physics.c:149-160
             for (int c = 0; c < 3; c++) {
                   if (tv) {
                         tv[9 + c] = A.j2.on ? cc[c] + cj[c] : cc[c];

@@ -137,3 +137,63 @@ def test_j2_needs_central_mass(lib):
         A.init(64, make_params(central_mass_bool=0, J2_bool=1, J2=0.01))
     assert e.value.status == A.E_ARG
     A.finalize()
+
+
+def shattering_pair(n, seed=5):
+    """A light disk and, in slots 5 and 6, two bodies of 0.002 central masses that meet head on:
+    a super-catastrophic collision, whose lost mass goes to the central body."""
+    from ncorpion_b200 import disks
+    b = disks.gravity_disk(n, seed=seed)
+    b[:, 6], b[:, 7] = 1e-7, 1e-4
+    for k, s in ((5, -1.0), (6, 1.0)):
+        b[k] = [1.0 + 0.045 * s, 0, 0.3, -2.0 * s, 0.7, 0, 2e-3, 0.04]
+    return b, np.ones(n, np.int32), np.array([0, 0, 0, 0, 0, 0, 1.0, 1.0])
+
+
+@pytest.mark.parametrize("mode", ["exact", "fp64"])
+@pytest.mark.parametrize("J2", [0.25, 0.0])
+def test_j2_after_central_mass_grew_in_a_collision(gpu, mode, J2):
+    """The brute-force driver: the step after a super-catastrophic collision as from the same state
+    uploaded afresh."""
+    from ncorpion_b200 import api as A
+    b, ex, cm = shattering_pair(300)
+    api = gpu(512, collision_bool=1, collision_type=3, gravity_mode=A.GRAVITY_MODES[mode], J2_bool=1, J2=J2,
+              sideral_omega=0.7, softening_parameter=0.5, reduce_to_COM_bool=0)
+    api.set_timestep(2e-2)
+    api.upload(b, ex, cm)
+    api.step_brute_force()
+    assert api.fragment_counts()[1] == 1
+    mid = api.download(512)
+    assert mid[2][6] > 1.003
+    api.step_brute_force()
+    out = api.download(512)
+    api.upload(*mid)
+    api.step_brute_force()
+    again = api.download(512)
+    for u, v in zip(out, again):
+        assert np.array_equal(u, v)
+
+
+@pytest.mark.parametrize("J2", [0.25, 0.0])
+def test_mesh_step_j2_with_the_central_mass_of_the_kick(gpu, J2):
+    """One mesh step, in which the collision comes before the kick: the central body's velocity as the
+    oracle's (1e-9 of its norm: the model's powers differ by 2 ulp; the mass before the pass
+    would change it by about 1e-3).  The fluid-body J2 is the one from before the step, which the oracle
+    is given as a constant."""
+    b, ex, cm = shattering_pair(300)
+    kw = dict(mesh_bool=1, brute_force_bool=0, collision_bool=1, collision_type=3, collision_cube_cells=64,
+              collision_cube_min=3.2, N_tilde=4, pq_min_max=[0, 1, 0, 1], J2_bool=1, reduce_to_COM_bool=0)
+    api = gpu(1024, J2=J2, sideral_omega=0.7, **kw)
+    api.set_timestep(2e-2)
+    api.upload(b, ex, cm)
+    api.step_mesh(0.05)
+    assert api.fragment_counts()[1] == 1
+    _, ex1, cm1 = api.download(1024)
+    w = oracle.PortWorld(1024, make_params(J2=J2 or 0.5 * 0.7 * 0.7, **kw))
+    w.set_fragmentation(4, (0, 1, 0, 1))
+    w.set_state(b, ex, cm, dt=2e-2, gam=0.05)
+    w.lib.orc_w_step_mesh()
+    _, ex_ref, cm_ref = w.get_state()
+    assert np.array_equal(ex1, ex_ref)
+    assert cm_ref[6] > 1.003 and abs(cm1[6] - cm_ref[6]) <= 1e-12
+    assert np.linalg.norm(cm1[3:6] - cm_ref[3:6]) <= 1e-9 * np.linalg.norm(cm_ref[3:6])
