@@ -620,10 +620,10 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed, const int
       const double sp = c.P.par_softening_parameter;
       L.soft = 0;
       L.eps2 = 0.;
-      if (sp != 0.) {  // all radii equal: one softening length
+      if (sp != 0.) {  // (all radii equal: one softening length)
             const auto mm = std::minmax_element(a->R, a->R + n);
             L.soft = *mm.first == *mm.second ? 1 : 2;
-            const double eu = 2.0 * sp * a->R[0];
+            const double eu = 2.0 * sp * std::max(std::abs(*mm.first), std::abs(*mm.second));  // the largest
             L.eps2 = eu * eu;
       }
       L.ntiles = (n + AT - 1) / AT;

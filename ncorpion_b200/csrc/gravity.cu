@@ -1193,12 +1193,13 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       D4 *s64 = (D4 *)c.src64;
       double eps2 = 0.;
       int soft_kind = soft ? 2 : 0;
-      if (soft && rr[0] == rr[1]) {
-            // all radii equal (the bounding-box pass found R_min == R_max): the
-            // uniform-epsilon instance, with fewer registers
-            const double eu = 2.0 * sp * rr[0];
+      if (soft) {
+            // the largest softening length; with all radii equal (the bounding-box pass
+            // found R_min == R_max) it is every pair's: the uniform-epsilon instance, with
+            // fewer registers
+            const double eu = 2.0 * sp * std::max(std::abs(rr[0]), std::abs(rr[1]));
             eps2 = eu * eu;
-            soft_kind = 1;
+            if (rr[0] == rr[1]) soft_kind = 1;
       }
       const double theta = P.par_near_theta > 0. ? P.par_near_theta : 0.15;
       if (nparts == 1) {

@@ -50,6 +50,44 @@ struct PairData {
       const float *l32;
 };
 
+// 0 for two near tiles (boxes bi, bj; tiles_near's test); for far ones the power of two
+// that brings their distances near 1, so that neither the cubes and fifth powers of their
+// reciprocals nor their squares leave FP32's range, whatever the caller's unit of length;
+// the sums are scaled back as they go to FP64, exact both ways.  1 where the distances
+// are near 1 as they are (2^20 either way; 2^12 for the fifth powers), which they are in
+// most units: that loop's differences are subtractions, with an operand less, and 3 %
+// faster.  Else the exponent is halfway between those of the smallest and the largest
+// distance, softened: 2^42 (2^25) either way of it is in range.  At most 2^64, so that
+// the padding at 1e18 stays finite.  eps2: the squared softening length (SOFT 1) or its
+// largest (SOFT 2).
+template <int SOFT, int OP>
+__device__ __forceinline__ float far_scale(const double *__restrict__ bi, const double *__restrict__ bj, double theta,
+                                           double eps2)
+{
+      double g2 = 0., di = 0., dj = 0.;
+      int lo = 0, hi = 0;  // high words of the largest gap and the largest distance along an axis
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+            const double c = fabs(bi[d] - bj[d]), gap = c - bi[3 + d] - bj[3 + d];
+            if (gap > 0.) g2 += gap * gap;
+            di += bi[3 + d] * bi[3 + d];
+            dj += bj[3 + d] * bj[3 + d];
+            lo = max(lo, __double2hiint(gap));
+            hi = max(hi, __double2hiint(c + (bi[3 + d] + bj[3 + d])));
+      }
+      if (g2 < theta * theta * (4. * fmax(di, dj))) return 0.f;
+      int el = (lo >> 20) - 1023, eh = (hi >> 20) - 1023;
+      if (SOFT != 0) {
+            const int es = ((__double2hiint(eps2) >> 20) - 1023) >> 1;
+            eh = max(eh, es);
+            if (SOFT == 1) el = max(el, es);
+      }
+      constexpr int IN = OP == 0 ? 20 : 12;
+      if (el >= -IN && eh < IN) return 1.f;
+      if (el <= -1023) el = eh;  // no lower bound
+      return __int_as_float((127 - max(-64, min(120, (eh + el) >> 1))) << 23);
+}
+
 // What a pair adds.  OP 0: the force, three sums a body.  OP 1: the force's
 // vector-Jacobian product with the bodies' lambda, four sums a body: with r from
 // row k to column j and w = m_k lambda_j - m_j lambda_k, t = w / D^3 - 3 r (r . w) / D^5
@@ -82,9 +120,9 @@ __device__ __forceinline__ int pair_phase(int B, int k, int r, int p)
       return 2 * p < B || (2 * p == B && r < p) ? 2 : 0;
 }
 
-// The squared distance, softened.
-template <int SM>
-__device__ __forceinline__ f2 pair_dist2(f2 dx, f2 dy, f2 dz, f2 RS, f2 RT, f2 E)
+// The squared distance, softened.  SC: RS in the caller's unit, the rest times S.
+template <int SM, bool SC>
+__device__ __forceinline__ f2 pair_dist2(f2 dx, f2 dy, f2 dz, f2 RS, f2 RT, f2 E, f2 S)
 {
       f2 q;
       if (SM == 0) {
@@ -92,7 +130,7 @@ __device__ __forceinline__ f2 pair_dist2(f2 dx, f2 dy, f2 dz, f2 RS, f2 RT, f2 E
       } else if (SM == 1) {
             q = f2_fma(dx, dx, E);
       } else {
-            const f2 e = f2_add(RS, RT);
+            const f2 e = SC ? f2_fma(RS, S, RT) : f2_add(RS, RT);
             q = f2_fma(dx, dx, f2_mul(e, e));
       }
       q = f2_fma(dy, dy, q);
@@ -116,24 +154,27 @@ struct PairGroup {
       f2 R[SOFT == 2 ? 64 : 2];
 };
 
-// A lane's rows, packed: both halves alike.
+// A lane's rows, packed: both halves alike.  -x, -y, -z and R times the tile pair's scale.
 template <int OP, int RU>
 struct PairRows {
-      f2 x[RU], y[RU], z[RU], m[RU], R[RU];
+      f2 nx[RU], ny[RU], nz[RU], m[RU], R[RU];
       f2 nlx[RU], nly[RU], nlz[RU];  // -lambda (OP 1)
 };
 
 // One row body against two column bodies packed.  OP 0: the row sums get
 // m_c d / D^3, the column sums m_r d / D^3 with d from row to column (the column's
 // force is minus its sum).  OP 1: t to both; row[3] and col[3] the masses' terms
-// (both are subtracted).  FIRST: the column sums start here.
-template <int SM, int OP, bool FIRST, int RU>
+// (both are subtracted).  FIRST: the column sums start here.  SC: lengths are multiplied
+// by the power of two S (far_scale).
+template <int SM, int OP, bool SC, bool FIRST, int RU>
 __device__ __forceinline__ void pair_sym(ulonglong2 xy, ulonglong2 zm, f2 RS, ulonglong2 l, f2 lz,
-                                         const PairRows<OP, RU> &T, int u, f2 E, f2 (&row)[PAIR_OUT<OP>],
-                                         f2 (&col)[PAIR_OUT<OP>])
+                                         const PairRows<OP, RU> &T, int u, f2 E, f2 S,
+                                         f2 (&row)[PAIR_OUT<OP>], f2 (&col)[PAIR_OUT<OP>])
 {
-      const f2 dx = f2_sub(xy.x, T.x[u]), dy = f2_sub(xy.y, T.y[u]), dz = f2_sub(zm.x, T.z[u]);
-      const f2 i = f2_rsqrt(pair_dist2<SM>(dx, dy, dz, RS, T.R[u], E));
+      const f2 dx = SC ? f2_fma(xy.x, S, T.nx[u]) : f2_add(xy.x, T.nx[u]);
+      const f2 dy = SC ? f2_fma(xy.y, S, T.ny[u]) : f2_add(xy.y, T.ny[u]);
+      const f2 dz = SC ? f2_fma(zm.x, S, T.nz[u]) : f2_add(zm.x, T.nz[u]);
+      const f2 i = f2_rsqrt(pair_dist2<SM, SC>(dx, dy, dz, RS, T.R[u], E, S));
       const f2 ii = f2_mul(i, i), i3 = f2_mul(ii, i);
       if constexpr (OP == 0) {
             const f2 wr = f2_mul(zm.y, i3), wc = f2_mul(T.m[u], i3);
@@ -175,9 +216,9 @@ __device__ __forceinline__ void pair_sym(ulonglong2 xy, ulonglong2 zm, f2 RS, ul
 // (the packed arithmetic's floor is 64): 84.9 with the columns packed, 89.5 with
 // the rows packed (a shuffle then moves half as much); without the 12 accumulating
 // FMAs 53, without shuffles 84, without shared loads and rsqrt 86.
-template <int SM, int OP, int RU>
+template <int SM, int OP, bool SC, int RU>
 __device__ __forceinline__ void far_group(const PairGroup<SM, OP> &st, int lane, const PairRows<OP, RU> &T, f2 E,
-                                          double *__restrict__ rs, int rstride, double *__restrict__ col, int cstride)
+                                          f2 S, const double (&back)[2], double *__restrict__ rs, int rstride, double *__restrict__ col, int cstride)
 {
       constexpr int NO = PAIR_OUT<OP>;
       f2 row[RU][NO];
@@ -199,9 +240,9 @@ __device__ __forceinline__ void far_group(const PairGroup<SM, OP> &st, int lane,
                   const f2 lz = OP == 1 ? st.lz[OP == 1 ? p : 0] : 0ull;
                   const f2 R = SM == 2 ? st.R[SM == 2 ? p : 0] : 0ull;
                   f2 v[NO];
-                  pair_sym<SM, OP, true>(xy, zm, R, l, lz, T, 0, E, row[0], v);
+                  pair_sym<SM, OP, SC, true>(xy, zm, R, l, lz, T, 0, E, S, row[0], v);
 #pragma unroll
-                  for (int u = 1; u < RU; u++) pair_sym<SM, OP, false>(xy, zm, R, l, lz, T, u, E, row[u], v);
+                  for (int u = 1; u < RU; u++) pair_sym<SM, OP, SC, false>(xy, zm, R, l, lz, T, u, E, S, row[u], v);
 #pragma unroll
                   for (int d = 0; d < NO; d++) {
                         c[d] = f2_add(c[d], v[d]);
@@ -213,8 +254,8 @@ __device__ __forceinline__ void far_group(const PairGroup<SM, OP> &st, int lane,
             for (int d = 0; d < NO; d++) {
                   float lo, hi;
                   f2_unpack(c[d], lo, hi);
-                  col[d * cstride + j] -= (double)lo;
-                  col[d * cstride + j + 32] -= (double)hi;
+                  col[d * cstride + j] -= SC ? (double)lo * back[d / 3] : (double)lo;
+                  col[d * cstride + j + 32] -= SC ? (double)hi * back[d / 3] : (double)hi;
             }
             __syncwarp();
             if (r0 & 8) {
@@ -224,7 +265,7 @@ __device__ __forceinline__ void far_group(const PairGroup<SM, OP> &st, int lane,
                         for (int d = 0; d < NO; d++) {
                               float lo, hi;
                               f2_unpack(row[u][d], lo, hi);
-                              const double v = (double)lo + (double)hi;
+                              const double v = SC ? ((double)lo + (double)hi) * back[d / 3] : (double)lo + (double)hi;
                               rs[(NO * u + d) * rstride] += d < 3 ? v : -v;
                               row[u][d] = 0ull;
                         }
@@ -376,6 +417,14 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
       const int I = b * B + r;
       for (int q = tid; q < NO * NB; q += TH) col[q] = 0.;
       for (int q = 0; q < NO * PU; q++) rows[q * TH + tid] = 0.;
+      // the unit's tile pairs (row tile, column tile): far_scale of each, by the threads
+      // that stage least
+      __shared__ float far_s[B * B];
+      if (MODE == 0 && tid >= TH - B * B) {
+            const int q = TH - 1 - tid, ti = b * B + q / B, tj = c * B + q % B;
+            if (ti < P.ntiles && tj < P.ntiles)
+                  far_s[q] = far_scale<SOFT, OP>(P.box + 6 * ti, P.box + 6 * tj, PAIR_NEAR * theta, eps2);
+      }
       if (MODE == 0)
             for (int q = tid; q < 2 * B * 32; q += TH) {
                   const int t = q / 64, g = (q / 32) & 1, s = q & 31, J = c * B + t;
@@ -401,9 +450,9 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
             const int t = r + p < B ? r + p : r + p - B, J = c * B + t;
             const int what = I < P.ntiles && J < P.ntiles ? pair_phase(B, k, r, p) : 0;
             if (what != 0) {
-                  const double *bj = P.box + 6 * J;
                   double *cl = col + t * PT;
-                  const bool near = MODE == 1 || what == 1 || tiles_near(P.box + 6 * I, bj, PAIR_NEAR * theta);
+                  const float sf = MODE == 0 ? far_s[r * B + t] : 0.f;
+                  const bool near = MODE == 1 || what == 1 || sf == 0.f;
 #pragma unroll 1
                   for (int u0 = 0; u0 < PU; u0 += RU) {
                         const int i = I * PT + lane + 32 * u0;
@@ -431,16 +480,18 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
                                     for (int d = 0; d < NO; d++) rs[(NO * u + d) * TH] += acc[u][d];
                         } else if (h * NG < 2) {
                               // coordinates relative to the column tile's centre
+                              const double *bj = P.box + 6 * J;
                               PairRows<OP, RU> F;
 #pragma unroll
                               for (int u = 0; u < RU; u++) {
-                                    const float x = (float)(T.me[u].x - bj[0]), y = (float)(T.me[u].y - bj[1]);
-                                    const float z = (float)(T.me[u].z - bj[2]), m = (float)T.me[u].w;
-                                    F.x[u] = f2_pack(x, x);
-                                    F.y[u] = f2_pack(y, y);
-                                    F.z[u] = f2_pack(z, z);
+                                    const float x = -sf * (float)(T.me[u].x - bj[0]);
+                                    const float y = -sf * (float)(T.me[u].y - bj[1]);
+                                    const float z = -sf * (float)(T.me[u].z - bj[2]), m = (float)T.me[u].w;
+                                    F.nx[u] = f2_pack(x, x);
+                                    F.ny[u] = f2_pack(y, y);
+                                    F.nz[u] = f2_pack(z, z);
                                     F.m[u] = f2_pack(m, m);
-                                    const float e = (float)T.R[u];
+                                    const float e = sf * (float)T.R[u];
                                     F.R[u] = SOFT == 2 ? f2_pack(e, e) : 0ull;
                                     if constexpr (OP == 1) {
                                           const float lx = -(float)T.l[u][0], ly = -(float)T.l[u][1];
@@ -450,10 +501,18 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
                                           F.nlz[u] = f2_pack(lz, lz);
                                     }
                               }
-                              const f2 E = f2_pack((float)eps2, (float)eps2);
+                              const double s = sf;
+                              const double back[2] = {OP == 0 ? s * s : s * s * s, s * s};
+                              const float es = (float)(eps2 * s * s);
+                              const f2 E = f2_pack(es, es), S = f2_pack(sf, sf);
 #pragma unroll 1
                               for (int g = h * NG; g < (h + 1) * NG; g++)
-                                    far_group<SOFT, OP, RU>(st[2 * t + g], lane, F, E, rs, TH, cl + 64 * g, NB);
+                                    if (sf == 1.f)
+                                          far_group<SOFT, OP, false, RU>(st[2 * t + g], lane, F, E, S, back, rs, TH,
+                                                                         cl + 64 * g, NB);
+                                    else
+                                          far_group<SOFT, OP, true, RU>(st[2 * t + g], lane, F, E, S, back, rs, TH,
+                                                                        cl + 64 * g, NB);
                         }
                   }
             }

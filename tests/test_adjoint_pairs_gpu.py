@@ -91,3 +91,31 @@ def test_vjp_past_the_block_size(lib, n):
     for g, r in zip(got["mixed"], got["exact"]):
         assert np.linalg.norm(g - r) <= 2e-5 * np.linalg.norm(r)
     api.finalize()
+
+
+@pytest.mark.parametrize("radii", ["none", "equal", "law"])
+@pytest.mark.parametrize("mode", ["exact", "mixed"])
+def test_units(lib, mode, radii):
+    """Lengths times 2^k, masses times 2^j and G times 2^(3k - j): the positions times 2^k, the gradients
+    to positions and velocities as they were, those to masses times 2^(k - j).  The powers of two
+    pass through every operation but the FP64 reciprocal square root unchanged: the fp64 bound above."""
+    from ncorpion_b200 import api
+    n = 3000
+    b, rng = bodies(n, radii, 4)
+    sp = 0.0 if radii == "none" else 0.5
+    adj = rng.normal(size=(n, 3))
+
+    def run(k, j):
+        L, W = 2.0 ** k, 2.0 ** j
+        api.init(n, make_params(softening_parameter=sp, gravity_mode=api.GRAVITY_MODES[mode], G=2.0 ** (3 * k - j)))
+        cm = np.array([0, 0, 0, 0, 0, 0, W, L])
+        args = (b[:, :3] * L, b[:, 3:6] * L, b[:, 6] * W, b[:, 7] * L, cm, DT, STEPS)
+        x, _ = api.leapfrog(*args)
+        gx, gv, gm = api.leapfrog_vjp(*args, adj)
+        api.finalize()
+        return x / L, gx, gv, gm * (W / L)
+
+    base = run(0, 0)
+    for k, j in [(-60, -60), (-45, 40), (20, 60), (30, -30), (42, 0), (50, 60)]:
+        for p, q in zip(run(k, j), base):
+            assert np.linalg.norm(p - q) <= 1e-11 * np.linalg.norm(q), (k, j)

@@ -87,3 +87,31 @@ def test_equal_keys(lib, n):
         assert np.all(np.isfinite(acc)) and not acc[ex == 0].any()
         assert (np.abs(acc[rows] - ref) / scale).max() <= tol
     api.finalize()
+
+
+@pytest.mark.parametrize("radii", ["none", "equal", "law"])
+@pytest.mark.parametrize("n", [3000, 17000])
+def test_units(lib, n, radii):
+    """The caller's units are not bound to FP32's range: lengths times 2^k and masses times 2^j
+    (0.3 astronomical units are 2^42 cm) give the accelerations times 2^(j - 2k).  The powers of two pass
+    through every operation but the FP64 reciprocal square root unchanged: the fp64 bound above."""
+    from ncorpion_b200 import api, disks
+    b = disks.gravity_disk(n, seed=n)
+    rng = np.random.default_rng(n)
+    b[:, 7] = disks.powerlaw_radii(rng, n, 1e-5, 1e-3) if radii == "law" else 1e-3
+    ex = np.ones(n, np.int32)
+    sp = 0.0 if radii == "none" else 0.5
+    api.init(n, make_params(softening_parameter=sp, central_mass_bool=0))
+    rows = np.arange(0, n, n // 40)
+    _, mag = reference(b, ex, sp, rows)
+    scale = mag.max(axis=1, keepdims=True)
+    for mode in ("fp64", "mixed"):
+        base, _ = api.vector_field(b, ex, mode=mode)
+        for k, j in [(-60, -60), (-45, 40), (0, -60), (20, 60), (42, 0), (44, -30), (50, 60)]:
+            u = b.copy()
+            u[:, [0, 1, 2, 7]] *= 2.0 ** k
+            u[:, 6] *= 2.0 ** j
+            acc, _ = api.vector_field(u, ex, mode=mode)
+            err = np.abs(acc * 2.0 ** (2 * k - j) - base)[rows] / scale
+            assert err.max() <= 1e-13, (mode, k, j, err.max())
+    api.finalize()
