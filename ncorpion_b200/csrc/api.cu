@@ -160,11 +160,14 @@ __global__ void k_kick(const int *__restrict__ ex, int n, double dt, const doubl
       }
 }
 
-// drift, src/rk4.c:115-126: x += timestep * v.
+// drift, src/rk4.c:115-126: x += timestep * v.  Nothing moves when *nhits (may be null) is
+// above nhits_max: a sweep of this step refused its hits.
 __global__ void k_drift(const int *__restrict__ ex, int n, double dt, double *x, double *y, double *z,
                         const double *__restrict__ vx, const double *__restrict__ vy,
-                        const double *__restrict__ vz, double *cm, int drift_cm)
+                        const double *__restrict__ vz, double *cm, int drift_cm,
+                        const int *__restrict__ nhits, int nhits_max)
 {
+      if (nhits && *nhits > nhits_max) return;
       int i = blockIdx.x * blockDim.x + threadIdx.x;
       if (i < n && ex[i]) {
             x[i] = __dadd_rn(x[i], __dmul_rn(dt, vx[i]));
@@ -239,14 +242,15 @@ int kick_state()
       return NCGPU_OK;
 }
 
-int drift_state()
+// hits: behind a brute-force sweep of the same step (see k_drift)
+int drift_state(bool hits)
 {
       Ctx &c = ctx();
       c.com_reduced = 0;
       const int nslots = c.largest_id + 1;
       int nb = nslots > 0 ? (nslots + 255) / 256 : 1;
       k_drift<<<nb, 256, 0, c.s>>>(c.ex, nslots, c.dt, c.x, c.y, c.z, c.vx, c.vy, c.vz, c.cm,
-                                   c.P.par_central_mass_bool);
+                                   c.P.par_central_mass_bool, hits ? c.scal + S_NHITS : nullptr, c.hit_cap / 2);
       NCG_LAUNCHED();
       return NCGPU_OK;
 }
@@ -667,7 +671,7 @@ int ncgpu_drift(void)
 {
       reset_launches();
       if (!g_ctx.inited || !g_ctx.uploaded) return NCGPU_E_STATE;
-      NCG_TRY(drift_state());
+      NCG_TRY(drift_state(false));
       return NCGPU_OK;
 }
 

@@ -169,9 +169,8 @@ __device__ void d_treat(const DevState &S, int a, int b, const EvArgs &E, int *e
 }
 
 // The hits' keys (i, j) into ascending order: a bitonic network of the CTA over the
-// next power of two, padded with the largest key; in shared memory up to EVS hits,
-// in `k` otherwise.
-constexpr int EVS = 2048;
+// next power of two, padded with the largest key.
+constexpr int EVS = 2048;  // keys in shared memory
 
 __device__ void sort_keys(unsigned long long *k, int n)
 {
@@ -193,27 +192,82 @@ __device__ void sort_keys(unsigned long long *k, int n)
             }
 }
 
+// More than EVS hits (hi, hj) of bodies i < EVROWS into ascending order (si, sj): counted
+// by row i, scattered to their rows (gj), each one's place in its row the number of
+// smaller j in it.  cnt: EVROWS ints of shared memory.  (The network of sort_keys in
+// global memory took 4 ms for 44,477 hits of 4,000 bodies, 1 % of the events' 0.4 s.)
+constexpr int EVROWS = 2 * EVS;
+
+__device__ void sort_rows(const int *hi, const int *hj, int n, int *cnt, int *gj, int *si, int *sj)
+{
+      constexpr int C = EVROWS / EVT;
+      __shared__ int wsum[32];
+      const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+      for (int q = tid; q < EVROWS; q += EVT) cnt[q] = 0;
+      __syncthreads();
+      for (int q = tid; q < n; q += EVT) atomicAdd(&cnt[hi[q]], 1);
+      __syncthreads();
+      int c[C], s = 0;  // exclusive prefix of the rows' counts
+#pragma unroll
+      for (int u = 0; u < C; u++) s += c[u] = cnt[C * tid + u];
+      int incl = s;
+      for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+      }
+      if (lane == 31) wsum[w] = incl;
+      __syncthreads();
+      int run = incl - s;
+      for (int u = 0; u < w; u++) run += wsum[u];
+#pragma unroll
+      for (int u = 0; u < C; u++) {
+            cnt[C * tid + u] = run;
+            run += c[u];
+      }
+      __syncthreads();
+      for (int q = tid; q < n; q += EVT) {
+            const int i = hi[q], p = atomicAdd(&cnt[i], 1);  // (afterwards cnt[i] is row i's end)
+            si[p] = i;
+            gj[p] = hj[q];
+      }
+      __syncthreads();
+      for (int p = tid; p < n; p += EVT) {
+            const int i = si[p], j = gj[p], lo = i > 0 ? cnt[i - 1] : 0, hi_ = cnt[i];
+            int r = lo;
+            for (int x = lo; x < hi_; x++) r += gj[x] < j;
+            sj[r] = j;
+      }
+      __syncthreads();
+}
+
 // sorted: hi, hj are in order (the host sorted them); else this kernel orders the
-// S_NHITS hits itself (gk: room for kcap keys, a power of two), so that the host need
-// not learn their number.  Clears the dirty marks it set.
-__global__ void __launch_bounds__(EVT) k_bf_events(DevState S, const int *__restrict__ hi, const int *__restrict__ hj,
-                                                   EvArgs E, int *ev, double *evrec, unsigned char *dirty, int *dlist,
-                                                   unsigned *err, int sorted, unsigned long long *gk, int kcap)
+// S_NHITS hits itself (bodies i below EVROWS; si, sj, gj: room for kcap ints each), so
+// that the host need not learn their number; more than kcap it refuses.  Clears the
+// dirty marks it set.
+__global__ void __launch_bounds__(EVT) k_bf_events(DevState S, const int *hi, const int *hj, EvArgs E, int *ev,
+                                                   double *evrec, unsigned char *dirty, int *dlist, unsigned *err,
+                                                   int sorted, int *si, int *sj, int *gj, int kcap)
 {
       __shared__ unsigned long long best;
       __shared__ unsigned long long candA;
       __shared__ int hp_s;
-      __shared__ unsigned long long sk[EVS];
+      __shared__ unsigned long long keys[EVS];
       const unsigned long long INF = ~0ull;
       const int nh = S.scal[S_NHITS];
-      unsigned long long *keys = nh <= EVS ? sk : gk;
       if (!sorted) {
             if (nh > kcap) {
                   if (threadIdx.x == 0) atomicOr(err, ERR_CAPACITY);
                   return;
             }
-            for (int q = threadIdx.x; q < nh; q += EVT) keys[q] = pkey(hi[q], hj[q]);
-            if (nh > 1) sort_keys(keys, nh);
+            if (nh <= EVS) {
+                  for (int q = threadIdx.x; q < nh; q += EVT) keys[q] = pkey(hi[q], hj[q]);
+                  if (nh > 1) sort_keys(keys, nh);
+            } else {
+                  sort_rows(hi, hj, nh, (int *)keys, gj, si, sj);
+                  hi = si;
+                  hj = sj;
+                  sorted = 1;
+            }
       }
       unsigned long long cur = 0;  // key of the last event; (0, 0) is never a pair
       if (threadIdx.x == 0) hp_s = 0;
@@ -342,9 +396,9 @@ int collide_brute_state(bool defer)
       NCG_LAUNCHED();
       // Up to 4,096 slots the event kernel orders the hits itself (a step has tens of
       // them, thousands in a dense cluster): the host's wait for their number and the
-      // radix passes cost 25 us of a 2,000-body step.  The scratch keys hold 2^19 then,
-      // as many hits as half the hit list.
-      const bool self = lid < 4096 && c.hit_cap == 1 << 20;
+      // radix passes cost 25 us of a 2,000-body step, the wait alone 4.5.  More hits than
+      // half the list, which the sorted ones have to fit as well, are refused there.
+      const bool self = lid < EVROWS;
       int nh = 0;
       int *si = c.hi, *sj = c.hj;
       if (!self) {
@@ -359,8 +413,8 @@ int collide_brute_state(bool defer)
       EvArgs E{lid, c.dt, c.P.par_collision_type, c.P.par_collision_parameter, c.P.par_one_collision_only_bool,
                c.P.par_mesh_bool, c.ev_cap, c.n_max, FragArgs{}};
       if (E.type == NCGPU_COLLISION_FRAGMENTATION && !make_frag_args(c, E.frag)) return NCGPU_E_ARG;
-      k_bf_events<<<1, EVT, 0, st>>>(S, si, sj, E, c.ev, c.evrec, c.dirty, c.dlist, c.err, !self,
-                                     (unsigned long long *)c.keys2, c.hit_cap / 2);
+      k_bf_events<<<1, EVT, 0, st>>>(S, si, sj, E, c.ev, c.evrec, c.dirty, c.dlist, c.err, !self, (int *)c.keys,
+                                     (int *)c.keys2, c.vals, c.hit_cap / 2);
       NCG_LAUNCHED();
       if (defer && E.type != NCGPU_COLLISION_FRAGMENTATION) return NCGPU_OK;
       return sync_scalars();

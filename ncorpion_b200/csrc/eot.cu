@@ -14,7 +14,7 @@ namespace ncg {
 DevState dev_state();
 int sync_scalars();
 int kick_state();
-int drift_state();
+int drift_state(bool hits);
 int collide_brute_state(bool defer);
 int mesh_reset_state();
 int mesh_pass(double gam, int test, bool defer);
@@ -357,8 +357,9 @@ extern "C" int ncgpu_step_brute_force(int *how_many_moonlets)
       reset_launches();
       if (!c.inited || !c.uploaded) return NCGPU_E_STATE;
       NCG_TRY(kick_state());
-      if (c.P.par_collision_bool) NCG_TRY(collide_brute_state(true));  // its counts come back with the end of step's
-      NCG_TRY(drift_state());
+      // the sweep's counts come back with the end of step's
+      if (c.P.par_collision_bool) NCG_TRY(collide_brute_state(true));
+      NCG_TRY(drift_state(c.P.par_collision_bool && c.largest_id > 0));
       return eot_state(how_many_moonlets);
 }
 
@@ -379,7 +380,7 @@ extern "C" int ncgpu_step_mesh(double gam, int *how_many_moonlets, long *total_n
                   NCG_TRY(mesh_pass(gam, 1, true));  // its counts come back with the end of step's
             }
       }
-      NCG_TRY(drift_state());
+      NCG_TRY(drift_state(c.P.par_collision_bool && c.force_naive && c.largest_id > 0));
       if (!c.P.par_collision_bool && !c.force_naive) {
             NCG_TRY(three_largest_state(nullptr));
             NCG_TRY(mesh_pass(gam, 0, false));

@@ -1,7 +1,8 @@
 """GPU: the brute-force sweep's hits put in order by the event kernel itself (up to
-4,096 slots: in shared memory to 2,048 hits, in memory past that) and by the host's
+4,096 slots: in shared memory to 2,048 hits, by rows past that) and by the host's
 sort (past it), at the sweep's tile edges: events and states as the oracle's, bit
-for bit (merged radii within 1 ulp, as in test_collide_gpu.py)."""
+for bit (merged radii within 1 ulp, as in test_collide_gpu.py).  More hits than the
+list holds end a step before it drifts."""
 import numpy as np
 import pytest
 
@@ -49,4 +50,23 @@ def test_sweep(lib, n, spread, ctype):
     bg, exg, _ = api.download(max(n, 64))
     b_ref, ex_ref, _ = w.get_state()
     assert_state_equal(bg, exg, b_ref, ex_ref)
+    api.finalize()
+
+
+def test_step_ends_before_the_drift_when_the_hits_do_not_fit(lib):
+    """1,800 bodies inside one another, half of the pairs approaching: 0.8 million hits, more than the 2^19
+    that the list holds.  As with an error of a sweep by itself, nothing is resolved and nothing moves."""
+    from ncorpion_b200 import api
+    b, ex, cm = cluster(1800, 1e-5, 3)
+    ex[:] = 1
+    b[:, 6], b[:, 7] = 1e-20, 2e-3
+    api.init(2048, make_params(collision_bool=1, collision_type=1, collision_parameter=1.5, reduce_to_COM_bool=0))
+    api.upload(b, ex, cm)
+    api.set_timestep(1e-3)
+    with pytest.raises(api.NcgpuError) as e:
+        api.step_brute_force()
+    assert e.value.status == api.E_CAPACITY
+    b1, ex1, _ = api.download(2048)
+    assert np.array_equal(ex1, ex) and np.array_equal(b1[:, :3], b[:, :3])
+    assert not np.array_equal(b1[:, 3:6], b[:, 3:6])
     api.finalize()
