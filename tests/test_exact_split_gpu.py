@@ -47,3 +47,21 @@ def test_past_the_preparation_cta(lib, port):
         acc, cma = api.vector_field(b[:k], ex[:k], cm, mode="exact")
         assert np.array_equal(acc, ref[:k] * (ex[:k] != 0)[:, None]) and np.array_equal(cma, cref)
     api.finalize()
+
+
+def test_no_slots_leave_the_kernel_time(lib):
+    """A field of no slots runs no field kernel: no time before the first one, that one's after it."""
+    from ncorpion_b200 import api, disks
+    none = np.zeros((0, 8))
+    api.init(64, make_params())
+    for mode in ("exact", "fp64", "mixed"):
+        api.vector_field(none, mode=mode)
+        with pytest.raises(api.NcgpuError) as e:
+            api.last_kernel_ms()
+        assert e.value.status == api.E_STATE
+    api.vector_field(disks.gravity_disk(64, seed=1))
+    t = api.last_kernel_ms()
+    for mode in ("exact", "fp64", "mixed"):
+        api.vector_field(none, mode=mode)
+        assert api.last_kernel_ms() == t
+    api.finalize()
