@@ -710,6 +710,8 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed, const int
       } while (0)
       k_scale_R<<<(int)((NP + 255) / 256), 256, 0, L.st>>>(L.sR, sp, L.sR, n, L.sR32, (int)NP);
       LF_LAUNCHED();
+      // (every input crosses before the first output, which may be the same array)
+      if (vjp) LF_TRY(rows_in(L, L.lx, a->adj_x_final, 3));
       if (jvp) {
             LF_TRY(rows_in(L, L.tx, a->tan_x0, 3));
             LF_TRY(rows_in(L, L.tv, a->tan_v0, 3));
@@ -749,7 +751,6 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed, const int
       }
       if (vjp) {
             // x_F = x_n - h v_n
-            LF_TRY(rows_in(L, L.lx, a->adj_x_final, 3));
             e = cudaMemsetAsync(L.lv, 0, sizeof(double) * 3 * N, L.st);
             if (e == cudaSuccess) e = cudaMemsetAsync(L.LX, 0, 6 * sizeof(double), L.st);  // LX, LV
             if (e == cudaSuccess) e = cudaMemsetAsync(L.gm, 0, sizeof(double) * N, L.st);

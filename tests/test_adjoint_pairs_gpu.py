@@ -71,6 +71,28 @@ def test_vjp_against_autograd(lib, n, radii, mode):
     api.finalize()
 
 
+@pytest.mark.parametrize("mode", ["exact", "mixed"])
+def test_vjp_in_place(lib, mode):
+    """x_final may be the array that brings dL/dx_final, the gradients those of the initial state."""
+    import ctypes as C
+    from ncorpion_b200 import api
+    n = 300
+    b, rng = bodies(n, "equal", 8)
+    adj = rng.normal(size=(n, 3))
+    cm = np.array([0, 0, 0, 0, 0, 0, 1.0, 1.0])
+    api.init(n, make_params(softening_parameter=0.5, gravity_mode=api.GRAVITY_MODES[mode]))
+    args = (b[:, :3], b[:, 3:6], b[:, 6], b[:, 7], cm, DT, STEPS)
+    xf, _ = api.leapfrog(*args)
+    ref = api.leapfrog_vjp(*args, adj)
+    x, v, m, R, xa = (np.array(q, order="C") for q in (b[:, :3], b[:, 3:6], b[:, 6], b[:, 7], adj))
+    p = [q.ctypes.data for q in (x, v, m, R, cm, xa)]
+    a = api.LeapfrogArgs(n, *p[:5], DT, STEPS, 32, p[5], None, p[5], p[0], p[1], p[2])
+    api.check(api.load().ncgpu_leapfrog_vjp(C.byref(a)), "ncgpu_leapfrog_vjp")
+    for got, want in zip((xa, x, v, m), (xf, *ref)):
+        assert np.array_equal(got, want)
+    api.finalize()
+
+
 @pytest.mark.parametrize("n", [16384, 16385, 16650])
 def test_vjp_past_the_block_size(lib, n):
     from ncorpion_b200 import api
