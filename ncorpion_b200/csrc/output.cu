@@ -147,18 +147,18 @@ __global__ void k_fmt_values(Values val, long lo, long hi, char *__restrict__ sl
       len[i] = L < 0 ? 0 : L;
 }
 
-// Copies the slots of values lo .. hi-1 to their places in the packed text
-// (offsets: exclusive scan of those values' lengths, from text; the files'
-// texts follow one another, without newlines).
 // What the host needs of a chunk, in page-locked memory that the device writes: the
 // files' boundaries (offsets within their chunk), the chunk's length, the error word.
 // (Copied back, these few bytes would wait behind the previous chunk's text.)
 struct FmtEnds {
       int n;
-      long at[17];   // first value of each file, and the end
+      long at[17];   // first value of each file (at most 16), and the end
 };
-constexpr int FMT_LEN = 16, FMT_ERR = 17;
+constexpr int FMT_LEN = 17, FMT_ERR = 18, FMT_ANSWERS = 19;  // behind the boundaries
 
+// Copies the slots of values lo .. hi-1 to their places in the packed text
+// (offsets: exclusive scan of those values' lengths, from text; the files'
+// texts follow one another, without newlines).  host: FMT_ANSWERS ints.
 __global__ void k_fmt_pack(const char *__restrict__ slots, const int *__restrict__ off, long lo, long hi,
                            char *__restrict__ text, FmtEnds ends, const unsigned *__restrict__ err, int *host)
 {
@@ -557,11 +557,11 @@ int format_files(const Values &val, int nfiles, const long *first, char *text, u
       }
       const size_t vals = c.fmt_cap / SLOT;
       int *len = c.fmt_len, *off = c.fmt_len + vals + 1, *sums = c.fmt_len + 2 * vals + 2;
-      long h[16] = {0};
+      long h[17] = {0};
       FmtEnds ends;
       ends.n = nfiles;
       for (int f = 0; f <= nfiles; f++) ends.at[f] = first[f];
-      volatile int *answers = (int *)(c.pinned + 8 * (size_t)c.n_max);  // FMT_AHEAD x 18, see FmtEnds
+      volatile int *answers = (int *)(c.pinned + 8 * (size_t)c.n_max);  // FMT_AHEAD x FMT_ANSWERS, see FmtEnds
       unsigned herr = 0;
       long base = 0;
       int st_ret = NCGPU_OK;
@@ -575,7 +575,7 @@ int format_files(const Values &val, int nfiles, const long *first, char *text, u
             // chunk-relative offsets; off[hi] is the chunk's length until the next chunk's scan
             NCG_TRY(scan_exclusive(len + lo, off + lo, (int)(hi - lo), sums, st));
             k_fmt_pack<<<nb, 256, 0, st>>>(c.fmt_slots, off, lo, hi, c.fmt_text + lo * SLOT, ends, c.err,
-                                           (int *)answers + 18 * (q % FMT_AHEAD));
+                                           (int *)answers + FMT_ANSWERS * (q % FMT_AHEAD));
             NCG_LAUNCHED();
             NCG_CK(cudaEventRecord(c.fev_done[q % FMT_AHEAD], st));
             return NCGPU_OK;
@@ -583,7 +583,7 @@ int format_files(const Values &val, int nfiles, const long *first, char *text, u
       for (int q = 0; q < std::min(nchunks, FMT_AHEAD); q++) NCG_TRY(launch(q));
       for (int q = 0; q < nchunks; q++) {
             const long lo = q * FMT_CHUNK, hi = std::min(total, lo + FMT_CHUNK);
-            volatile int *rel = answers + 18 * (q % FMT_AHEAD);
+            volatile int *rel = answers + FMT_ANSWERS * (q % FMT_AHEAD);
             NCG_CK(cudaEventSynchronize(c.fev_done[q % FMT_AHEAD]));
             herr = (unsigned)rel[FMT_ERR];
             if (herr) break;
