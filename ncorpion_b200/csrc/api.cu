@@ -359,7 +359,7 @@ int ncgpu_init(int n_max, const struct ncgpu_params *params)
       A(c.ex, N); A(c.exs, N);
       A(c.cm, 16); A(c.cm_acc, 3);
       A(c.acc, 3 * N);
-      A(c.cmterm, 6 * N);
+      A(c.cmterm, 3 * N);
       A(c.cidx, N);
       A(c.cnt, (std::max(N, (size_t)1 << 20) + 1023) / 1024 + 2);
       A(c.n_dev, 8);

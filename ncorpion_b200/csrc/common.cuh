@@ -597,7 +597,7 @@ struct Ctx {
 
       // gravity scratch
       double *acc = nullptr;       // 3 * n_max (x block, y block, z block)
-      double *cmterm = nullptr;    // 6 * n_max (CM_acc terms; two per body with J2)
+      double *cmterm = nullptr;    // 3 * n_max (CM_acc terms of the tiled modes, by body or by block)
       double *partial = nullptr;   // gravity partial sums (chunks x 3 x n_max)
       size_t partial_cap = 0;      // doubles
       int *cidx = nullptr;         // compacted existing slot ids

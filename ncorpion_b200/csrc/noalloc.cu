@@ -37,8 +37,7 @@ constexpr size_t NBLK = (size_t)NOALLOC_MAX_SLOTS / 1024 + 2;
 // layout (doubles first, 256-byte aligned blocks)
 constexpr size_t OFF_SRC = 0;                                   // 4 * NPAD doubles
 constexpr size_t OFF_SRCR = OFF_SRC + 4 * NPAD * 8;             // NPAD doubles
-constexpr size_t OFF_CTERM = OFF_SRCR + NPAD * 8;               // 6 * NPAD doubles (two per body with J2)
-constexpr size_t OFF_ACC = OFF_CTERM + 6 * NPAD * 8;            // 3 * NPAD doubles
+constexpr size_t OFF_ACC = OFF_SRCR + NPAD * 8;                 // 3 * NPAD doubles
 constexpr size_t OFF_CIDX = OFF_ACC + 3 * NPAD * 8;             // NPAD ints
 constexpr size_t OFF_BLK = OFF_CIDX + NPAD * 4;                 // NBLK ints
 constexpr size_t OFF_MISC = (OFF_BLK + NBLK * 4 + 255) / 256 * 256;  // n_dev
