@@ -650,20 +650,29 @@ int lf_core(const struct ncgpu_leapfrog_args *a, int mode, bool mixed, const int
       L.ncp = (a->nsteps + L.C - 1) / L.C + 1;
       const size_t N = (size_t)n, st = 6 * N + 6, NP = (size_t)L.ntiles * AT;
       const size_t nred = (N + 31) / 32;  // blocks of the final passes
-      const size_t npart = vjp ? std::max(L.pf.doubles, L.pv.doubles) : L.pf.doubles;
-      size_t total = 4 * NP + 2 * NP + NP / 2 + 3 * NP / 2 + 2                   // s64 s32 sR32 l32 count
-                     + 3 * N * 2 + 2 * N + 6 + 3 * N + npart + 3 * nred          // X V m sR cm out part red
+      const size_t rest = 4 * NP + 2 * NP + NP / 2 + 3 * NP / 2 + 2                   // s64 s32 sR32 l32 count
+                     + 3 * N * 2 + 2 * N + 6 + 3 * N + 3 * nred                  // X V m sR cm out red
                      + 3 * N * 2 + 6 + N                                         // lx lv LX LV gm
                      + (vjp ? st * L.ncp + (size_t)L.C * (3 * N + 3) : 0)        // checkpoints, segment
                      + (jvp ? 3 * N * 3 + N + 6 + 3 + 3 * N * L.nch : 0)         // tx tv tm tX da dA, partials
                      + 6 * (size_t)L.ntiles                                      // tile boxes
                      + 3 * N + (N + 1) / 2;                                      // stage, perm
-      if (total > c.lf_cap) {  // grown when needed, kept for the next call
+      size_t npart;  // the pair sums' rows, fewer at a time where the memory is short
+      for (;;) {
+            npart = vjp ? std::max(L.pf.doubles, L.pv.doubles) : L.pf.doubles;
+            if (rest + npart <= c.lf_cap) break;  // grown when needed, kept for the next call
             if (c.lf_buf) cudaFree(c.lf_buf);
             c.lf_buf = nullptr;
             c.lf_cap = 0;
-            NCG_CK(cudaMalloc(&c.lf_buf, total * sizeof(double)));
-            c.lf_cap = total;
+            const cudaError_t e = cudaMalloc(&c.lf_buf, (rest + npart) * sizeof(double));
+            if (e == cudaSuccess) {
+                  c.lf_cap = rest + npart;
+                  break;
+            }
+            cudaGetLastError();
+            c.lf_buf = nullptr;
+            const bool less = pair_halve<0>(L.pf);
+            if (!(pair_halve<1>(L.pv) || less)) return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
       }
       double *p = c.lf_buf;
       auto take = [&](size_t k) { double *q = p; p += k; return q; };

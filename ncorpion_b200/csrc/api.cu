@@ -36,7 +36,12 @@ int ensure_partial(size_t doubles)
       if (c.partial) NCG_CK(cudaFree(c.partial));
       c.partial = nullptr;
       c.partial_cap = 0;
-      NCG_CK(cudaMalloc(&c.partial, doubles * sizeof(double)));
+      const cudaError_t e = cudaMalloc(&c.partial, doubles * sizeof(double));
+      if (e != cudaSuccess) {
+            cudaGetLastError();  // (a caller may go on with less)
+            c.partial = nullptr;
+            return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
+      }
       c.partial_cap = doubles;
       return NCGPU_OK;
 }

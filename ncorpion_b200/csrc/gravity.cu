@@ -1207,8 +1207,10 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       if (nparts == 1) {
             // the whole field: every pair once
             PairData pd{s64, c.srcR, (const float *)c.src32, c.srcR32, c.tilebox, n, ntiles, 0, nullptr, nullptr};
-            const PairPlan pl = pair_plan<0>(n);
-            NCG_TRY(ensure_partial(pl.doubles));
+            PairPlan pl = pair_plan<0>(n);
+            int got;
+            while ((got = ensure_partial(pl.doubles)) != NCGPU_OK && pair_halve<0>(pl)) {}
+            NCG_TRY(got);
             PairRun pr;
             NCG_CK(cudaEventRecord(c.kev0, st));
             NCG_TRY(pair_sums<0>(pd, pl, mode == NCGPU_GRAVITY_MIXED ? 0 : 1, soft_kind, theta, eps2, c.partial, pr, st));

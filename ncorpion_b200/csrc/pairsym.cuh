@@ -588,6 +588,24 @@ struct PairPlan {
 
 constexpr size_t PAIR_ROWS_MAX = (size_t)1 << 27;  // doubles of partial rows at once (1 GB)
 
+// At most `most` offsets of pl at once (the shares about equal).
+template <int OP>
+void pair_share(PairPlan &pl, int most)
+{
+      const int shares = (pl.nk + most - 1) / most;
+      pl.per = (pl.nk + shares - 1) / shares;
+      pl.doubles = PAIR_OUT<OP> * (size_t)pl.npad * (2 * pl.per + (pl.per >= pl.nk ? 0 : 1));
+}
+
+// Half the offsets at once, for a device whose memory is short; false when there is one.
+template <int OP>
+bool pair_halve(PairPlan &pl)
+{
+      if (pl.per <= 1) return false;
+      pair_share<OP>(pl, pl.per / 2);
+      return true;
+}
+
 template <int OP>
 PairPlan pair_plan(int n)
 {
@@ -614,9 +632,7 @@ PairPlan pair_plan(int n)
       pl.nk = pair_offsets(pl.nb);
       const size_t row = 2 * PAIR_OUT<OP> * (size_t)pl.npad;  // both sides of an offset
       const int most = (int)(PAIR_ROWS_MAX / row > (size_t)pl.nk ? pl.nk : PAIR_ROWS_MAX / row < 1 ? 1 : PAIR_ROWS_MAX / row);
-      const int shares = (pl.nk + most - 1) / most;
-      pl.per = (pl.nk + shares - 1) / shares;
-      pl.doubles = row * pl.per + (pl.per >= pl.nk ? 0 : PAIR_OUT<OP> * (size_t)pl.npad);
+      pair_share<OP>(pl, most);
       return pl;
 }
 

@@ -115,3 +115,35 @@ def test_units(lib, n, radii):
             err = np.abs(acc * 2.0 ** (2 * k - j) - base)[rows] / scale
             assert err.max() <= 1e-13, (mode, k, j, err.max())
     api.finalize()
+
+
+def test_short_of_memory(lib):
+    """With 160 MB left on the device the partial rows (1 GB here for the field, 0.4 GB for the leapfrog's VJP)
+    are summed in more and smaller shares, grouped differently: the fp64 bound above."""
+    import torch
+    from ncorpion_b200 import api, disks
+    n, m = 160001, 60000
+    b = disks.gravity_disk(n, seed=1)
+    p = make_params(softening_parameter=0.5, central_mass_bool=0, gravity_mode=api.GRAVITY_MIXED)
+    cm = np.array([0, 0, 0, 0, 0, 0, 1.0, 1.0])
+    args = (b[:m, :3], b[:m, 3:6], b[:m, 6], b[:m, 7], cm, 1e-3, 1, np.ones((m, 3)))
+
+    def run():
+        grads = api.leapfrog_vjp(*args)
+        return [*grads, api.vector_field(b, mode="mixed")[0]]
+
+    api.init(n, p)
+    full = run()
+    api.finalize()
+    api.init(n, p)
+    api.vector_field(b[:256], mode="mixed")
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (160 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        short = run()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        api.finalize()
+    for s, f in zip(short, full):
+        assert np.linalg.norm(s - f) <= 1e-13 * np.linalg.norm(f)
