@@ -77,9 +77,10 @@ struct ncgpu_params {
       int par_switch_to_brute_force;     /* switch_to_brute_force                    */
       int par_gravity_mode;              /* NCGPU_GRAVITY_*                          */
       double par_near_theta;             /* MIXED: tile pairs whose boxes are closer
-                                        than near_theta x the larger box diagonal
-                                        (and some beyond) are summed in FP64
-                                        (default 0.15 if <= 0) */
+                                        than 1.45 near_theta x the larger box diagonal
+                                        are summed in FP64 (near_theta x it in a part
+                                        of the field and in the leapfrog's tangents;
+                                        default 0.15 if <= 0) */
       double par_disruption_threshold;   /* disruption_threshold (dump into the CM)  */
       double par_high_dumping_threshold; /* high_dumping_threshold (dump, unbound)   */
       int par_reduce_to_COM_bool;        /* reduce_to_COM_bool                       */
@@ -168,8 +169,9 @@ int ncgpu_vector_field_dev(const double *d_bodies, const int *d_exists, int larg
    part-th slice of the existing bodies in slot order (exact mode), or of the
    Morton-ordered 128-body target blocks (FP64 / mixed) -- and every other row
    of d_acc receives -0.0 (+0.0 for empty slots from part 0), the identity of
-   the sum, so that the element-wise sum of the parts' d_acc is the full field
-   bit for bit.  d_cm_acc receives the full CM_acc in every part.
+   the sum, so that the element-wise sum of the parts' d_acc is the full field,
+   bit for bit in the exact mode (the tiled modes sum a part's targets by
+   themselves: within the modes' errors).  d_cm_acc receives the full CM_acc in every part.
    ncgpu_vector_field_dev is part 0 of 1.  (No reference counterpart: the
    reference is single-threaded; the sum of the parts is vector_field's.) */
 int ncgpu_vector_field_part(const double *d_bodies, const int *d_exists, int largest_id,

@@ -20,8 +20,8 @@
 // MIXED gravity mode the bodies are taken in the Morton order of their initial
 // positions (a permutation at the call's boundary), every
 // evaluation computes the 128-body tiles' boxes, and only the tile pairs whose
-// boxes are near (near_theta x the larger diagonal, and each tile with itself)
-// are summed in FP64; the others in FP32 on coordinates relative to a tile's
+// boxes are near (1.45 near_theta x the larger diagonal, near_theta x it in the JVP,
+// and each tile with itself) are summed in FP64; the others in FP32 on coordinates relative to a tile's
 // centre, short FP32 sums folded into FP64 -- the force kernel's scheme applied
 // to the force, its VJP and its JVP.
 //

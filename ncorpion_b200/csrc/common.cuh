@@ -743,7 +743,7 @@ int sync_scalars_h(int *h);  // device scalars into c.* and h[S_COUNT], error wo
 // compacted order's part-th slice in the exact mode, the part-th slice of the
 // Morton-ordered target blocks in the tiled modes); every other row gets -0.0
 // (+0.0 for empty slots from part 0), so that the sum over the parts is the
-// full field, bit for bit.  CM_acc is the full one in every part.
+// full field, bit for bit in the exact mode.  CM_acc is the full one in every part.
 // cm_dev (may be null): the central body in device memory, which the exact mode
 // then reads there.  An unknown mode is the exact one up to EXACT_SMALL_N slots.
 constexpr int EXACT_SMALL_N = 8192;

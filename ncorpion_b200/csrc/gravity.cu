@@ -23,7 +23,8 @@
 // MIXED  same tiling; pair terms in FP32 on coordinates relative to a tile's
 //        centre (one MUFU rsqrt per pair), short FP32 sums accumulated in FP64;
 //        tile pairs whose bounding boxes are closer than near_theta x the larger
-//        box diagonal (always including the target's own tile) are summed in FP64.
+//        box diagonal (1.45 times as far in the sums over unordered pairs; always
+//        including the target's own tile) are summed in FP64.
 //        The central-mass term and G are applied in FP64.
 #include <algorithm>
 #include "common.cuh"

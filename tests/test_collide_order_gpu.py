@@ -26,14 +26,17 @@ def cluster(n, spread, seed):
     return b, ex, np.array([0, 0, 0, 0, 0, 0, 1.0, 1.0])
 
 
-# (slots, spread): no hit; a few; tile edges; past 2,048 hits; past 4,096 slots (host's sort, 32 bodies j a CTA)
+# (slots, spread): no hit; a few; tile edges; past 2,048 hits; past 4,096 slots
+# (host's sort, 32 bodies j a CTA); thousands of hits, in every row
 @pytest.mark.parametrize("n,spread", [(2, 1.0), (33, 2e-2), (128, 2e-2), (129, 1e-2), (161, 1e-2), (220, 6e-4),
-                                      (4096, 6e-2), (4097, 6e-2)])
+                                      (4096, 6e-2), (4097, 6e-2), (4096, 1e-2)])
 @pytest.mark.parametrize("ctype", [1, 2])
 def test_sweep(lib, n, spread, ctype):
     from ncorpion_b200 import api
     if ctype == 2 and spread < 1e-3:
         pytest.skip("mergers leave few hits to order")
+    if ctype == 1 and (n, spread) == (4096, 1e-2):
+        pytest.skip("thousands of rebounds in a row take seconds; the mergers have the same hits to order")
     b, ex, cm = cluster(n, spread, n)
     kw = dict(collision_bool=1, collision_type=ctype, collision_parameter=1.5, one_collision_only_bool=int(spread < 1e-3))
     api.init(max(n, 64), make_params(**kw))

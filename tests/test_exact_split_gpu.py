@@ -33,6 +33,38 @@ def test_bits(lib, port, n, soft, j2):
     api.finalize()
 
 
+@pytest.mark.parametrize("nparts", [2, 3, 7])
+@pytest.mark.parametrize("n", [7, 9, 65, 2049])
+def test_bits_in_parts(lib, n, nparts):
+    """Parts that end inside a CTA's 8 targets, and parts without a target: each row from one part (-0.0
+    from the others), their sum and every part's CM_acc bit for bit the whole's."""
+    import ctypes as C
+    import torch
+    from ncorpion_b200 import api, disks
+    ex = np.ones(n, np.int32)
+    ex[::5] = 0
+    cm = np.array([1e-6, -2e-6, 0.0, 0, 0, 0, 1.0, 1.0])
+    d_b, d_ex = torch.from_numpy(disks.gravity_disk(n, seed=n)).cuda(), torch.from_numpy(ex).cuda()
+    api.init(n, make_params(softening_parameter=0.5))
+
+    def run(part, parts):
+        acc, cma = (torch.full(s, np.nan, dtype=torch.float64, device="cuda") for s in ((n, 3), (3,)))
+        api.check(lib.ncgpu_vector_field_part(*(C.c_void_p(t.data_ptr()) for t in (d_b, d_ex)), n - 1, api.ptr(cm), part,
+                                              parts, *(C.c_void_p(t.data_ptr()) for t in (acc, cma)), 0, None), "part")
+        torch.cuda.synchronize()
+        return acc.cpu().numpy(), cma.cpu().numpy()
+
+    full, cma = run(0, 1)
+    total, owners = np.full_like(full, -0.0), np.zeros(n, int)
+    for part in range(nparts):
+        acc, c = run(part, nparts)
+        assert np.array_equal(c, cma)
+        owners += ~(acc.view(np.int64) == np.float64(-0.0).view(np.int64)).all(axis=1)
+        total = total + acc
+    assert np.array_equal(total.view(np.int64), full.view(np.int64)) and (owners[ex == 1] == 1).all()
+    api.finalize()
+
+
 def test_past_the_preparation_cta(lib, port):
     """8,192 and 8,193 slots with most of them empty: the two compactions give the same field."""
     from ncorpion_b200 import api, disks

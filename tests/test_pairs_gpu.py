@@ -19,7 +19,8 @@ from conftest import make_params
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 33, 127, 128, 129, 256, 257, 385, 1000, 12288, 12289, 16384, 16385, 16641, 65408, 65537, 160001]
+SIZES = [1, 2, 31, 33, 127, 128, 129, 256, 257, 385, 1000, 12288, 12289, 16384, 16385, 16641, 65408, 65537, 160001,
+         12290, 16386, 49024, 49026]  # (the odd ones have empty slots; blocks of 1, 2, 2 and 4 tiles)
 
 
 def reference(b, ex, sp, rows):
