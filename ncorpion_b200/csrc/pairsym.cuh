@@ -55,11 +55,12 @@ struct PairData {
 // reciprocals nor their squares leave FP32's range, whatever the caller's unit of length;
 // the sums are scaled back as they go to FP64, exact both ways.  1 where the distances
 // are near 1 as they are (2^20 either way; 2^12 for the fifth powers), which they are in
-// most units: that loop's differences are subtractions, with an operand less, and 3 %
-// faster.  Else the exponent is halfway between those of the smallest and the largest
-// distance, softened: 2^42 (2^25) either way of it is in range.  At most 2^64, so that
-// the padding at 1e18 stays finite.  eps2: the squared softening length (SOFT 1) or its
-// largest (SOFT 2).
+// most units: that loop's differences are subtractions, with an operand less (65,536
+// bodies 1,675 us a call against 1,718 with the scale in every pair, 262,144 22.8 ms
+// against 23.8).  Else the exponent is halfway between those of the smallest and the
+// largest distance, softened: 2^42 (2^25) either way of it is in range.  At most 2^64, so
+// that the padding at 1e18 stays finite.  eps2: the squared softening length (SOFT 1) or
+// its largest (SOFT 2).
 template <int SOFT, int OP>
 __device__ __forceinline__ float far_scale(const double *__restrict__ bi, const double *__restrict__ bj, double theta,
                                            double eps2)
@@ -417,10 +418,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
       const int I = b * B + r;
       for (int q = tid; q < NO * NB; q += TH) col[q] = 0.;
       for (int q = 0; q < NO * PU; q++) rows[q * TH + tid] = 0.;
-      // the unit's tile pairs (row tile, column tile): far_scale of each, by the threads
-      // that stage least
+      // a unit of several tile pairs (row tile, column tile): far_scale of each, by the
+      // threads that stage least; one pair's is worked out below, while its rows load
       __shared__ float far_s[B * B];
-      if (MODE == 0 && tid >= TH - B * B) {
+      if (MODE == 0 && B > 1 && tid >= TH - B * B) {
             const int q = TH - 1 - tid, ti = b * B + q / B, tj = c * B + q % B;
             if (ti < P.ntiles && tj < P.ntiles)
                   far_s[q] = far_scale<SOFT, OP>(P.box + 6 * ti, P.box + 6 * tj, PAIR_NEAR * theta, eps2);
@@ -451,7 +452,9 @@ __global__ void __launch_bounds__(32 * W, 16 / W) k_pair_sym(PairData P, int k0,
             const int what = I < P.ntiles && J < P.ntiles ? pair_phase(B, k, r, p) : 0;
             if (what != 0) {
                   double *cl = col + t * PT;
-                  const float sf = MODE == 0 ? far_s[r * B + t] : 0.f;
+                  const float sf = MODE == 1 ? 0.f
+                                   : B > 1   ? far_s[r * B + t]
+                                             : far_scale<SOFT, OP>(P.box + 6 * I, P.box + 6 * J, PAIR_NEAR * theta, eps2);
                   const bool near = MODE == 1 || what == 1 || sf == 0.f;
 #pragma unroll 1
                   for (int u0 = 0; u0 < PU; u0 += RU) {
