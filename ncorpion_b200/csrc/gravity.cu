@@ -1127,7 +1127,11 @@ int gravity_eval(const BodyView &bv, int largest_id, const double *cmh, const J2
       if (!tiled) {
             // (nothing comes back to the host: the kernels read the count of existing
             // bodies from device memory)
-            if (mode != NCGPU_GRAVITY_EXACT && nslots > EXACT_SMALL_N) return NCGPU_E_ARG;
+            if (mode != NCGPU_GRAVITY_EXACT && nslots > EXACT_SMALL_N) {  // an unknown mode: refused with any body
+                  int n = 0;
+                  NCG_TRY(compact_existing(bv.ex, largest_id, &n, st));
+                  if (n > 0) return NCGPU_E_ARG;
+            }
             NCG_TRY(exact_field(bv, nslots, CmArg{cm_dev, cmh[0], cmh[1], cmh[2], cmh[6]}, P.par_G,
                                 P.par_softening_parameter, central, j2, part, nparts, fill, c.cidx, (D4 *)c.src64,
                                 c.srcR, c.cnt, c.n_dev, ax, ay, az, d_cm_acc, st, c.kev0));

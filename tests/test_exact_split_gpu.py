@@ -97,3 +97,21 @@ def test_no_slots_leave_the_kernel_time(lib):
         api.vector_field(none, mode=mode)
         assert api.last_kernel_ms() == t
     api.finalize()
+
+
+@pytest.mark.parametrize("n", [8192, 8193])
+def test_unknown_mode(lib, n):
+    """A mode that is none of the three: the exact field up to 8,192 slots, refused beyond when a slot is filled."""
+    from ncorpion_b200 import api, disks
+    b, ex = disks.gravity_disk(n, seed=2), np.zeros(n, np.int32)
+    api.init(n, make_params())
+    for live in (0, 5):
+        ex[:live] = 1
+        if live and n > 8192:
+            with pytest.raises(api.NcgpuError) as e:
+                api.vector_field(b, ex, mode=7)
+            assert e.value.status == api.E_ARG
+        else:
+            got, ref = api.vector_field(b, ex, mode=7), api.vector_field(b, ex, mode="exact")
+            assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+    api.finalize()
