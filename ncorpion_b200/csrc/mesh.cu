@@ -154,17 +154,19 @@ __global__ void k_mesh_count(const int *__restrict__ pv, const int *__restrict__
 // to: its place is the owner's offset plus its number in the owner's queue, so the
 // lists come out in the reference's order, written by adjacent lanes (coalesced
 // stores), and the FP64 predicates run with every lane busy.  A lane whose queue is
-// full walks again in the next round, queueing the candidates after those taken.
+// full goes on in the next round from where it stopped.
 // The predicate's full records are read only for pairs that can touch within dt: the
 // distance, from the records' first 32 bytes, is compared with the radii plus the way
 // that any two bodies can close (twice the largest speed; the margin of 1e-6 is far
 // above the predicate's rounding, about 1e-8 of the same lengths).
-// Bound by latency: of 400 us for 13 million candidates the walk takes 190, the
-// partners' positions 100 and the lists' scattered stores 110.  Queueing every body of
-// the cells and telling the candidates apart in the balanced loop took twice its
-// rounds, with a ballot and running counts in each, and whole records for every pair:
-// a step of the 1,048,576-body disk 358 us, now 264 (more CTAs an SM, of fewer
-// registers, spill; two rounds at once are 25 % slower).
+// Bound by latency: of 400 us for 13 million candidates the walk took 190, the
+// partners' positions 100 and the lists' scattered stores 110 (now 369 us).  Queueing
+// every body of the cells and telling the candidates apart in the balanced loop took
+// twice its rounds, with a ballot and running counts in each, and whole records for
+// every pair: a step of the 1,048,576-body disk 358 us, now 254 (more CTAs an SM, of fewer
+// registers, spill; two rounds at once are 25 % slower).  Walking from the start again in
+// every round cost 3 % there, and made a step of 50,000 bodies in 20 clumps, lists of
+// 2,500, 49 ms (now 16).
 constexpr int MWW = 4;        // warps per block
 constexpr int MWQ = 32;       // queued candidates per lane and round
 constexpr int MWS = MWQ + 1;  // a lane's row (the pad keeps the lanes off each other's banks)
@@ -200,29 +202,29 @@ __global__ void __launch_bounds__(MWW * 32, 8) k_mesh_write(const MRec *__restri
       }
       okk[w][lane] = (L >= 0 ? k : -1) | (dk ? 0x80000000 : 0);
       const long long dd = (long long)d * d;
-      int skip = 0;
+      int skip = 0, r = 8, i0 = 0;  // candidates taken; where the walk goes on: row, body of it
       bool more = L >= 0;
       while (__any_sync(0xffffffffu, more)) {
             int cnt = 0;
             if (more) {
-                  int idx = -skip;
 #pragma unroll 1
-                  for (int r = 8; r >= 0; --r) {
+                  for (; r >= 0; --r) {
                         int2 cr[3];
                         row_cells(crange, d_row(L, r, d, dd), cap, cr);
                         // cells mid + 1, mid, mid - 1 in one loop
                         const int n2 = cr[2].y - cr[2].x, n1 = n2 + cr[1].y - cr[1].x, n0 = n1 + cr[0].y - cr[0].x;
+                        int i = i0;
 #pragma unroll 1
-                        for (int i = 0; i < n0; ++i) {
+                        for (; i < n0 && cnt < MWQ; ++i) {
                               const int q = i + (i < n2 ? cr[2].x : i < n1 ? cr[1].x - n2 : cr[0].x - n1);
-                              if (pv[q] < k) {  // (a body removed earlier in the pass is not pushed)
-                                    if (idx >= 0 && idx < MWQ) qb[w][lane * MWS + idx] = q;
-                                    ++idx;
-                              }
+                              // (a body removed earlier in the pass is not pushed)
+                              if (pv[q] < k) qb[w][lane * MWS + cnt++] = q;
                         }
+                        i0 = i;
+                        if (cnt == MWQ) break;
+                        i0 = 0;
                   }
-                  cnt = min(max(idx, 0), MWQ);
-                  more = idx > MWQ;
+                  more = cnt == MWQ;
             }
             int incl = cnt;
             for (int o = 1; o < 32; o <<= 1) {
