@@ -40,13 +40,12 @@ N_BODIES = 65536
 SOFTENING = 0.5
 FLOP_PER_INTERACTION = 20  # 3 sub, 3 FMA (r^2+eps^2), rsqrt (2), 3 mul, 3 FMA accumulate
 # DRAM bytes (read + write) of one k_pair_sym<mixed> launch at N=65,536, from one ncu capture
-# (profiles/k_pair_sym_mixed_n65536.txt): 3.32 MB read + 142.57 MB written (the written bytes are the
+# (profiles/k_pair_sym_mixed_n65536.txt): 3.25 MB read + 142.55 MB written (the written bytes are the
 # partial rows: 128 blocks of bodies, 129 rows x 3 x 65,536 doubles, less what stays in L2).
-MIXED_DRAM_BYTES = 145.89e6
+MIXED_DRAM_BYTES = 145.80e6
 # DRAM bytes of one mesh step's two main kernels (k_mesh_write + k_mesh_grav_fast) captured at N=262,144
-# (profiles/mesh_step_kernels_n262144.txt, current version: 40.3 MB + 36.0 MB), scaled by the bodies to
-# N=1,048,576.
-MESH_DRAM_BYTES_262K = 76.3e6
+# (profiles/mesh_step_kernels_n262144.txt: 38.8 MB + 36.0 MB), scaled by the bodies to N=1,048,576.
+MESH_DRAM_BYTES_262K = 74.8e6
 METRIC = "Pair-interactions/s mixed vs FP64 (rel err<1e-6); mesh collision steps/s at N=1M"
 WORKLOAD = ("gravity-only single-step accelerations, N=65,536 disk (a~U[0.8,1.2], e~Rayleigh 0.01, "
             "i~Rayleigh 0.005), masses log-uniform [1e-9,1e-6], R=1e-5, softening 0.5*(R_k+R_p)")

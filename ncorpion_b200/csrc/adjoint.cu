@@ -27,11 +27,11 @@
 //
 // A kick and drift is three launches (tile data, pair sums, final pass with the
 // kick, the drift and the central body's), a step of the reverse sweep three
-// more.  N = 16,384, mixed: a force's pair sums take 128 us and a VJP's 269 (208
+// more.  N = 16,384, mixed: a force's pair sums take 128 us and a VJP's 268 (208
 // and 396 when each body's were made by themselves, bound by the FP32 pipe and the
 // near tiles' FP64), a forward call and a forward + adjoint call of 32 steps
-// 24.5 ms (42.3 with those, with six to nine launches a step and strided copies of the
-// caller's arrays).  N = 5,003, FP64: 32 us and 62 (50 and 86), 24 steps 5.73 ms (9.47).
+// 24.7 ms (42.3 with those, with six to nine launches a step and strided copies of the
+// caller's arrays).  N = 5,003, FP64: 30 us and 57 (50 and 86), 24 steps 5.50 ms (9.47).
 #include <algorithm>
 #include <vector>
 #include "common.cuh"
