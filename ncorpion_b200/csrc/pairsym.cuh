@@ -651,7 +651,7 @@ template <int MODE, int SOFT, int OP, int B, int W>
 int pair_launch(const PairData &pd, int k0, int nk, double theta, double eps2, double *part, long npad, cudaStream_t st)
 {
       constexpr size_t smem = pair_smem<MODE, SOFT, OP, B, W>();
-      static_assert(smem <= 48 * 1024, "no larger carve-out is asked for");
+      static_assert(smem + B * B * sizeof(float) <= 48 * 1024, "no larger carve-out is asked for");
       k_pair_sym<MODE, SOFT, OP, B, W><<<dim3(pd.nb, nk), 32 * W, smem, st>>>(pd, k0, theta, eps2, part, npad);
       NCG_LAUNCHED();
       return NCGPU_OK;
